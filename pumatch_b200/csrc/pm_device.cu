@@ -94,11 +94,11 @@ struct MatchArgs {
                                 // 2 flat strided (leaf_flat)
   int32_t lane_subtree_max;     // lane_subtree when the parent set is at most this long; 0 = never
   int32_t nl1;
-  int32_t pad1;
   int32_t n;
   int32_t nplans;
   int32_t T;
-  int32_t chunk;
+  int32_t chunk;                // root edges per shard unit (shard k takes units k, k + count, ...)
+  int32_t pop;                  // root edges per queue pop, <= chunk
   int32_t shard_rank;
   int32_t shard_count;
   int32_t split_min;            // donate last-but-one-level ranges at least this long
@@ -125,14 +125,16 @@ struct MatchArgs {
   float* root_reads;
   const int32_t* root_order;
   const int32_t* root_split;      // optional per-root donation threshold of the last-but-one level (plan 0)
-  // donation ring: items (plan, root, level, begin, end, path[2..level])
+  // work hand-off (publish_pieces, wait_piece): a warp out of work draws a
+  // ticket and waits on the ring slot of that number; a warp with work fills
+  // the oldest tickets' slots with (plan, root, level, begin, end,
+  // path[2..level])
   int4* don_items;                // 3 int4 per slot
-  unsigned long long* don_head;   // next slot to fill
-  unsigned long long* don_ready;  // per slot: sequence number + 1 when filled
+  unsigned long long* don_ready;  // per slot: 0 empty, ticket + 1 filled, kQuit no more work
+  unsigned long long* sched;      // (tickets drawn << 32) | pieces handed out
+  unsigned int* started;          // warps that have begun
   unsigned int don_mask;
-  unsigned int* active;           // warps holding work (phase 1 or a donation)
   unsigned int total_warps;
-  unsigned long long* don_tail;   // next slot to take
   unsigned long long* heartbeat;  // bumped by busy warps
   unsigned long long timeout_ns;  // hard limit on the launch; idle warps also give
                                   // up after this long without a heartbeat
@@ -169,8 +171,9 @@ struct alignas(16) WarpState {
   int32_t top[9];    // arena offset where level L's slots start
   int32_t off[16];
   int32_t size[16];
-  unsigned long long next_beat;  // setops value at which to bump the heartbeat
-  unsigned long long next_split; // setops value at which to look for idle warps
+  long long next_check;          // SM clock at which to look for waiting warps and at the deadline
+  long long began;               // SM clock at the start of the current root or piece
+  int32_t checks;                // checks made (the heartbeat is bumped on every 16th)
   unsigned long long t_start;    // %globaltimer at kernel entry (ns)
   int32_t* arena;                // slots of the current path: the warp's own arena or a borrowed one
   int32_t* gather;               // gather space for lists copied out of frames or host memory (paged)
@@ -1311,37 +1314,79 @@ struct Donation {
   int path[7];  // path[2..level] used
 };
 
-// Hands the upper half of the shallowest level range that is long enough to
-// the donation ring, when some warps are idle and fewer pieces are queued
-// than idle warps.  A range whose candidates head whole subtrees is long
-// enough from 2 candidates on; one whose candidates only lead to the last
-// level (one set operation each) needs split_min.  Lane 0 decides.
-__device__ __forceinline__ void maybe_donate(const MatchArgs& a, WarpState& S, int n, int L0, int L, int plan_id,
-                                             int root_id) {
+// How often a busy warp looks for waiting warps (SM cycles, about 2 us).  A
+// look costs one L2 read; a piece costs its taker the prefix again, so work
+// that ends sooner than this is not worth handing out.
+#define PM_CHECK_CYCLES 4096
+
+__device__ __forceinline__ unsigned long long ld_vol_u64(const unsigned long long* p) {
+  return *(const volatile unsigned long long*)p;
+}
+
+// Hands parts of the shallowest level range that is long enough to waiting
+// warps.  sched counts tickets drawn by warps out of work and pieces handed
+// out; their difference is the number of warps waiting, and a piece goes into
+// the slot of the oldest unserved ticket, whose holder polls that slot alone
+// -- so handing out is one CAS by the donor and no contention among the
+// waiting (thousands of idle warps competing for one queue head by CAS cost
+// several microseconds a piece and held every query with few roots at 5 us
+// per donation).  With many waiting for each busy warp the range is cut into
+// up to 33 pieces at once, one published per lane, so that a single heavy
+// root reaches all warps in two or three rounds.  A range whose candidates
+// head whole subtrees is long enough from 2 candidates on; one whose
+// candidates only lead to the last level (one set operation each) needs
+// `split` and is cut into pieces of at least half of that.
+__device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, WarpState& S, int n, int L0, int L, int plan_id,
+                                                int root_id) {
   const int lane = lane_id();
+  int k = L0, q = 0;
+  unsigned long long first = 0;
   if (lane == 0) {
-    const unsigned int act = *((volatile unsigned int*)a.active);
-    const unsigned long long head = *((volatile unsigned long long*)a.don_head);
-    const unsigned long long tail = *((volatile unsigned long long*)a.don_tail);
-    if (act < a.total_warps && head - tail < (unsigned long long)(a.total_warps - act) &&
-        head - tail < (unsigned long long)a.don_mask) {
-      for (int k = L0; k <= L; k++) {
-        const int it = S.iter[k], iend = S.iend[k];
-        if (iend - it < ((k + 1 == n - 2) ? max(S.split, 2) : 2)) continue;
-        const int mid = it + (iend - it) / 2;  // it < mid < iend
-        const unsigned long long slot = atomicAdd(a.don_head, 1ull);
-        int4* dst = a.don_items + 3 * (slot & a.don_mask);
-        dst[0] = make_int4(plan_id, root_id, k, mid);
-        dst[1] = make_int4(iend, S.path[2], S.path[3], S.path[4]);
-        dst[2] = make_int4(S.path[5], S.path[6], 0, 0);
-        st_release(&a.don_ready[slot & a.don_mask], slot + 1);
-        atomicAdd(&a.stats[ST_SPLITS], 1ull);
-        S.iend[k] = mid;
+    const unsigned long long cur = ld_vol_u64(a.sched);
+    const int waiting = (int)((unsigned)(cur >> 32) - (unsigned)cur);
+    if (waiting > 0) {
+      const int busy = max(1, (int)a.total_warps - waiting);
+      const int want = min(32, (waiting + busy - 1) / busy);
+      for (; k <= L; k++) {
+        const int len = S.iend[k] - S.iter[k];
+        const int unit = (k + 1 == n - 2) ? max(S.split, 2) : 2;
+        if (len < unit) continue;
+        q = min(want, 2 * len / unit - 1);  // >= 1
         break;
       }
+      if (q > 0 && atomicCAS(a.sched, cur, cur + (unsigned long long)q) != cur) q = 0;  // look again later
+      first = cur & 0xffffffffull;
     }
   }
+  q = __shfl_sync(FULL, q, 0);
+  if (q == 0) return 0;
+  k = __shfl_sync(FULL, k, 0);
+  first = __shfl_sync(FULL, first, 0);
+  const int it = S.iter[k], len = S.iend[k] - it;
+  // part 0 of q + 1 stays here, part lane + 1 goes out
+  unsigned err = 0;
+  if (lane < q) {
+    const int b = it + (int)((long long)len * (lane + 1) / (q + 1));
+    const int e = it + (int)((long long)len * (lane + 2) / (q + 1));
+    const unsigned long long slot = first + (unsigned long long)lane;
+    unsigned long long* ready = &a.don_ready[slot & a.don_mask];
+    // the slot's holder of one lap ago is reading it: a bounded wait
+    int spin = 0;
+    while (ld_acquire(ready) != 0ull && spin < (1 << 20)) { __nanosleep(64); spin++; }
+    if (spin == (1 << 20)) err = DEV_TIMEOUT;
+    int4* dst = a.don_items + 3 * (slot & a.don_mask);
+    dst[0] = make_int4(plan_id, root_id, k, b);
+    dst[1] = make_int4(e, S.path[2], S.path[3], S.path[4]);
+    dst[2] = make_int4(S.path[5], S.path[6], 0, 0);
+    st_release(ready, slot + 1);
+  }
   __syncwarp();
+  if (lane == 0) {
+    S.iend[k] = it + len / (q + 1);
+    atomicAdd(&a.stats[ST_SPLITS], (unsigned long long)q);
+  }
+  __syncwarp();
+  return __any_sync(FULL, err != 0) ? DEV_TIMEOUT : 0u;
 }
 
 // Depth-first enumeration below a fixed path prefix.  path[0..L0] must be
@@ -1381,23 +1426,30 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
   }
   int L = L0;
   while (true) {
-    // liveness signal for idle warps and the launch-wide deadline, then the
-    // periodic look for idle warps to hand work to
-    if (w.setops >= S.next_beat) {
+    // by the clock: the launch-wide deadline, the liveness signal for waiting
+    // warps, and the look for waiting warps to hand work to (set operations
+    // take from under a microsecond to hundreds, so counting them is no clock)
+    if (__any_sync(FULL, clock64() >= S.next_check)) {
       int late = 0;
       if (lane == 0) {
-        atomicAdd(a.heartbeat, 1ull);
-        S.next_beat = w.setops + 1024;
         late = (global_ns() - S.t_start) > a.timeout_ns;
+        late = late ? (int)DEV_TIMEOUT : 0;
+        if ((S.checks++ & 15) == 0) {
+          atomicAdd(a.heartbeat, 1ull);
+          late |= (int)*(volatile unsigned int*)a.status;  // another warp failed: so has the launch
+        }
       }
-      if (__shfl_sync(FULL, late, 0)) {
-        w.err |= DEV_TIMEOUT;
+      late = __shfl_sync(FULL, late, 0);
+      if (late) {
+        w.err |= (unsigned)late;
         return 0;
       }
-    }
-    if (a.split_min > 0 && w.setops >= S.next_split) {
-      if (lane == 0) S.next_split = w.setops + 64;
-      maybe_donate(a, S, n, L0, L, plan_id, root_id);
+      if (a.split_min > 0 && __any_sync(FULL, clock64() - S.began >= PM_CHECK_CYCLES)) {
+        w.err |= publish_pieces(a, S, n, L0, L, plan_id, root_id);
+        if (w.err) return 0;
+      }
+      if (lane == 0) S.next_check = clock64() + PM_CHECK_CYCLES;
+      __syncwarp();
     }
     const int m = P.level_begin[L];
     const int it = S.iter[L];
@@ -1446,38 +1498,62 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
   return cnt;
 }
 
-// Takes one donated piece if any is queued.  The caller is counted as active
-// before it claims, so "no active warp and nothing queued" is a safe exit
-// test for everyone.  Returns false if nothing was taken.
-__device__ bool take_donation(const MatchArgs& a, Donation& d) {
+constexpr unsigned long long kQuit = ~0ull;
+
+// Draws a ticket: the warp is out of work and will take the piece that lands
+// in the ticket's slot.  The warp whose ticket leaves none of the started
+// warps busy (pieces are counted before they are published, so their takers
+// count as busy) marks every slot a warp can be waiting on with kQuit.  Warps
+// that have not started hold nothing: the root queue is empty by now, and
+// they will find their own ticket's slot marked -- so the end does not wait
+// for blocks that other launches keep from starting.  A warp counts itself
+// started before its first pop, and the count is read here after a pop that
+// found the queue empty, so no warp with roots is missed.  `seen` is the
+// largest count this warp has read: it only grows, so fewer waiting warps
+// than that need no new look.  Returns the ticket, or kQuit for the last warp.
+__device__ unsigned long long draw_ticket(const MatchArgs& a, unsigned& seen) {
+  const int lane = lane_id();
+  unsigned long long old = 0;
+  __syncwarp();
+  if (lane == 0) old = atomicAdd(a.sched, 1ull << 32);
+  old = __shfl_sync(FULL, old, 0);
+  const unsigned tickets = (unsigned)(old >> 32), pieces = (unsigned)old;
+  const unsigned waiting = tickets + 1u - pieces;
+  if (waiting < seen) return tickets;
+  if (lane == 0) {
+    __threadfence();  // after the pop that found the queue empty
+    seen = atomicAdd(a.started, 0u);
+  }
+  seen = __shfl_sync(FULL, seen, 0);
+  if (waiting != seen) return tickets;
+  const unsigned long long last = min((unsigned long long)a.total_warps, (unsigned long long)a.don_mask + 1ull);
+  for (unsigned long long i = lane; i < last; i += 32) {
+    const unsigned long long slot = (unsigned long long)pieces + i;
+    *(volatile unsigned long long*)&a.don_ready[slot & a.don_mask] = kQuit;
+  }
+  return kQuit;
+}
+
+// One look at the ticket's slot: 0 nothing yet, 1 a piece (in d), -1 no more
+// work.
+__device__ int wait_piece(const MatchArgs& a, unsigned long long ticket, Donation& d) {
   int got = 0;
   int v[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (lane_id() == 0) {
-    const unsigned long long tail = *((volatile unsigned long long*)a.don_tail);
-    const unsigned long long head = *((volatile unsigned long long*)a.don_head);
-    if (tail < head) {
-      // counted as active before claiming (no fence: if another warp reads
-      // the claim before the count it may leave early, never lose work)
-      atomicAdd(a.active, 1u);
-      if (atomicCAS(a.don_tail, tail, tail + 1) == tail) {
-        // bounded wait for the donor to finish writing this slot
-        for (int spin = 0; spin < (1 << 22); spin++) {
-          if (ld_acquire(&a.don_ready[tail & a.don_mask]) == tail + 1) { got = 1; break; }
-          __nanosleep(64);
-        }
-        if (got) {
-          const volatile int* src = (const volatile int*)(a.don_items + 3 * (tail & a.don_mask));
-          for (int i = 0; i < 12; i++) v[i] = src[i];
-        } else {
-          atomicOr(a.status, (unsigned)DEV_TIMEOUT);
-          atomicSub(a.active, 1u);
-        }
-      } else {
-        atomicSub(a.active, 1u);
-      }
+    unsigned long long* ready = &a.don_ready[ticket & a.don_mask];
+    // polled with plain volatile reads: an acquire read drops the SM's L1
+    // contents, which the busy warps beside this one live on
+    const unsigned long long r = ld_vol_u64(ready);
+    if (r == kQuit) got = -1;
+    else if (r == ticket + 1 && ld_acquire(ready) == r) {
+      got = 1;
+      const volatile int* src = (const volatile int*)(a.don_items + 3 * (ticket & a.don_mask));
+      for (int i = 0; i < 12; i++) v[i] = src[i];
+      st_release(ready, 0ull);  // read: the slot is free for the ticket one lap on
     }
   }
   got = __shfl_sync(FULL, got, 0);
+  if (got <= 0) return got;
   int u[12];
 #pragma unroll
   for (int i = 0; i < 12; i++) u[i] = __shfl_sync(FULL, v[i], 0);
@@ -1493,7 +1569,7 @@ __device__ bool take_donation(const MatchArgs& a, Donation& d) {
   d.path[4] = u[7];
   d.path[5] = u[8];
   d.path[6] = u[9];
-  return got != 0;
+  return 1;
 }
 
 // MINB = 4: 64 registers, four 256-thread blocks per SM (more warps in flight,
@@ -1508,8 +1584,8 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wib;
   int32_t* own = a.arena + gw * a.arena_words;
   if (lane == 0) {
-    S.next_beat = 0;
-    S.next_split = 0;
+    S.next_check = 0;
+    S.checks = 0;
     S.t_start = global_ns();
     S.arena = own;
     S.cap = a.slot_words;
@@ -1519,6 +1595,8 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
     S.mphase = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.mbar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    atomicAdd(a.started, 1u);  // before the first pop (draw_ticket)
+    __threadfence();
   }
   __syncwarp();
   Work w;
@@ -1530,18 +1608,22 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   // phase 1: root chunks from the per-plan cursors
   while (exhausted < np && !w.err) {
     const DPlan& P = a.plans[p];
+    // a pop is `pop` roots of one shard unit of `chunk` roots (the last pop of
+    // a unit, and the last unit, may be shorter)
+    const unsigned long long per = (unsigned long long)((a.chunk + a.pop - 1) / a.pop);
     const unsigned long long nchunks = (unsigned long long)((P.nroots + a.chunk - 1) / a.chunk);
     unsigned long long c = 0;
     if (lane == 0) c = atomicAdd(&a.cursors[p], 1ull);
     c = __shfl_sync(FULL, c, 0);
-    const unsigned long long gc = c * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
+    const unsigned long long gc = c / per * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
     if (gc >= nchunks) {
       exhausted++;
       p = (p + 1 == np) ? 0 : p + 1;
       continue;
     }
+    const long long sub = (long long)(c % per) * a.pop;  // within the unit
     exhausted = 0;
-    if (PAGED && a.pf_off && p == 0) {
+    if (PAGED && a.pf_off && p == 0 && sub == 0) {
       // post the predicted pages of a chunk this warp's successors will reach
       const long long pc = (long long)gc + (long long)a.pf_ahead * a.shard_count;
       // only while the host's queue is short: a page posted behind a long
@@ -1566,8 +1648,8 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
         w.prefetched += v[0];
       }
     }
-    const long long rb = (long long)gc * a.chunk;
-    const long long re = min((long long)P.nroots, rb + a.chunk);
+    const long long rb = (long long)gc * a.chunk + sub;
+    const long long re = min((long long)P.nroots, (long long)gc * a.chunk + min((long long)a.chunk, sub + a.pop));
     unsigned long long local = 0;
     for (long long r = rb; r < re && !w.err; r++) {
       // position r of the range; with an order, the order's entry there
@@ -1579,6 +1661,7 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
         S.path[0] = e.x;
         S.path[1] = e.y;
         S.split = (a.root_split && p == 0) ? a.root_split[rid] : a.split_min;
+        S.began = clock64();
       }
       __syncwarp();
       const unsigned long long c0 = dfs_from<LABELED, PAGED>(a, P, S, 1, 0, -1, true, p, (int)rid, w);
@@ -1594,16 +1677,21 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
     if (lane == 0 && local) atomicAdd(&a.counts[p], local);
     p = (p + 1 == np) ? 0 : p + 1;  // interleave plans chunk by chunk
   }
-  // phase 2: drain donated ranges until no warp holds work
-  __threadfence();
-  if (lane == 0) atomicSub(a.active, 1u);
-  __syncwarp();
+  // phase 2: take pieces until every warp is out of work.  A warp that failed
+  // draws no ticket (a piece given to it would be lost): the status word ends
+  // the others' wait.
+  if (w.err && lane == 0) atomicOr(a.status, w.err);
   unsigned long long last_beat = 0, last_change = global_ns();
   const unsigned long long t_drain = last_change;
   unsigned long long busy_ns = 0;
-  while (!w.err) {
+  unsigned seen = 0;
+  unsigned long long ticket = w.err ? kQuit : draw_ticket(a, seen);
+  int looks = 0;
+  while (!w.err && ticket != kQuit) {
     Donation item;
-    if (take_donation(a, item)) {
+    const int got = wait_piece(a, ticket, item);
+    if (got < 0) break;
+    if (got > 0) {
       const unsigned long long t_item = global_ns();
       const DPlan& P = a.plans[item.plan];
       const int2 e = P.roots[item.root];
@@ -1612,6 +1700,7 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
         S.path[1] = e.y;
         for (int k = 2; k <= item.level; k++) S.path[k] = item.path[k];
         S.split = (a.root_split && item.plan == 0) ? a.root_split[item.root] : a.split_min;
+        S.began = clock64();
       }
       __syncwarp();
       const unsigned long long b0 = w.bytes, r0 = w.reads;
@@ -1625,39 +1714,38 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
           if (a.root_cost) atomicAdd(&a.root_cost[item.root], (float)(w.bytes - b0));
           if (a.root_reads) atomicAdd(&a.root_reads[item.root], (float)(w.reads - r0));
         }
-        // no fence: a warp that reads this decrement before this warp's
-        // donations can only leave early; this warp drains them itself
-        atomicSub(a.active, 1u);
       }
       __syncwarp();
       last_change = global_ns();
       busy_ns += last_change - t_item;
+      if (w.err) {
+        if (lane == 0) atomicOr(a.status, w.err);
+        break;
+      }
+      ticket = draw_ticket(a, seen);
+      looks = 0;
       continue;
     }
-    unsigned int act = 0;
-    unsigned long long head = 0, tail = 0, beat = 0;
-    // no fence between these reads: a stale pair can only make a warp leave
-    // early, and the warp holding the work finishes (and drains) it itself
+    // poll the one word; the clock, the heartbeat and the status (words all
+    // waiting warps share) only every 64th time
+    __nanosleep(looks < 64 ? 100 : 400);
+    if (++looks & 63) continue;
+    unsigned long long beat = 0;
+    unsigned int failed = 0;
     if (lane == 0) {
-      act = *((volatile unsigned int*)a.active);
-      head = *((volatile unsigned long long*)a.don_head);
-      tail = *((volatile unsigned long long*)a.don_tail);
-      beat = *((volatile unsigned long long*)a.heartbeat);
+      beat = ld_vol_u64(a.heartbeat);
+      failed = *(volatile unsigned int*)a.status;
     }
-    act = __shfl_sync(FULL, act, 0);
-    head = __shfl_sync(FULL, head, 0);
-    tail = __shfl_sync(FULL, tail, 0);
     beat = __shfl_sync(FULL, beat, 0);
-    if (act == 0 && tail >= head) break;
+    if (__shfl_sync(FULL, failed, 0)) break;
     // bounded wait: give up (and report DEV_TIMEOUT) when no warp has made
     // progress for timeout_ns
     const unsigned long long now = global_ns();
     if (beat != last_beat) { last_beat = beat; last_change = now; }
-    else if (now - last_change > a.timeout_ns) {
+    else if (__any_sync(FULL, now > last_change && now - last_change > a.timeout_ns)) {
       if (lane == 0) atomicOr(a.status, (unsigned)DEV_TIMEOUT);
       break;
     }
-    __nanosleep(1000);
   }
   if (lane == 0) {
     const unsigned long long t_end = global_ns();
@@ -2340,10 +2428,9 @@ struct Launch {
   void (*kfn)(const MatchArgs) = nullptr;
   int64_t warps = 0;
   size_t ctl_words = 0;
-  unsigned int active0 = 0;  // initial active-warp count (host staging)
 };
 
-static constexpr unsigned kDonSlots = 1u << 15;
+static constexpr unsigned kDonSlots = 1u << 13;  // a launch has at most a few thousand warps
 // a warp's own arena: at most this many slot words and gather words
 static constexpr int64_t kOwnSlotWords = 1 << 16;
 static constexpr int64_t kOwnGatherWords = 1 << 15;
@@ -2472,8 +2559,8 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   L->n_big = n_big;
   L->own_bytes = own_bytes;
   L->big_bytes = big_bytes;
-  // control block: cursors[32] counts[32] stats[16] status/active head tail
-  // heartbeat, donation ready[] and items[]
+  // control block: cursors[32] counts[32] stats[] status sched heartbeat,
+  // hand-off ready[] and items[]
   L->ctl_words = 32 + 32 + kStatWords + 8 + kDonSlots + 6 * kDonSlots;
   st = ensure((void**)ctl, ctl_bytes, L->ctl_words * 8);
   if (st != PM_OK) return st;
@@ -2493,6 +2580,13 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.nplans = nplans;
   a.T = T;
   a.chunk = chunk;
+  // Unless the caller sets the pop size, a pop is as many roots as leave every
+  // warp eight pops (one at least, the shard unit at most): sixteen roots per
+  // pop left a query of 2,000 roots to 120 of 3,552 warps (the 4-clique on 400
+  // vertices: 225 us of kernel).
+  int64_t total_roots = 0;
+  for (int i = 0; i < nplans; i++) total_roots += L->dp[i].nroots / shard_count;
+  a.pop = o.chunk > 0 ? chunk : (int32_t)std::max<int64_t>(1, std::min<int64_t>(chunk, total_roots / (8 * L->warps)));
   a.shard_rank = o.shard_rank;
   a.shard_count = shard_count;
   a.split_min = o.split_level1 == 0 ? 64 : (o.split_level1 < 0 ? 0 : o.split_level1);
@@ -2501,10 +2595,9 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.cursors = w; w += 32;
   a.counts = w; w += 32;
   a.stats = w; w += kStatWords;
-  a.status = (unsigned int*)w;
-  a.active = (unsigned int*)w + 1; w += 1;
-  a.don_head = w; w += 1;
-  a.don_tail = w; w += 1;
+  a.status = (unsigned int*)w; w += 1;
+  a.sched = w; w += 1;
+  a.started = (unsigned int*)w; w += 1;
   a.heartbeat = w; w += 5;
   a.don_ready = w; w += kDonSlots;
   a.don_items = (int4*)w; w += 6 * kDonSlots;
@@ -2536,7 +2629,6 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
     a.pf_ahead = o.prefetch_ahead > 0 ? o.prefetch_ahead : 2;
   }
   for (int i = 0; i < nplans; i++) a.plans[i] = L->dp[i];
-  L->active0 = (unsigned int)L->warps;
   if (L->paged) {
     st = paged_prepare(c, const_cast<pm_graph*>(g), L->cold, &a.pg);
     if (st != PM_OK) return st;
@@ -2548,12 +2640,11 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
 // Enqueues one launch on the context stream: control reset, the persistent
 // kernel (its plans travel in its parameter block) between events eb/ee, and
 // the read-back of counts, stats and status into host_ctl.  Capturable into a
-// CUDA graph (host_ctl and active_src must then be pinned).
-static pm_status enqueue_launch(pm_ctx* c, Launch& L, const unsigned int* active_src,
-                                unsigned long long* host_ctl, cudaEvent_t eb, cudaEvent_t ee) {
-  CK(cudaMemsetAsync(L.a.cursors, 0, L.ctl_words * 8, c->stream));
+// CUDA graph (host_ctl must then be pinned).
+static pm_status enqueue_launch(pm_ctx* c, Launch& L, unsigned long long* host_ctl, cudaEvent_t eb, cudaEvent_t ee) {
+  // everything up to the hand-off items, which are written before they are read
+  CK(cudaMemsetAsync(L.a.cursors, 0, (size_t)((char*)L.a.don_items - (char*)L.a.cursors), c->stream));
   if (L.n_big) CK(cudaMemsetAsync(L.a.big_owner, 0, 4 * (size_t)L.n_big, c->stream));
-  CK(cudaMemcpyAsync(L.a.active, active_src, sizeof(unsigned int), cudaMemcpyHostToDevice, c->stream));
   if (eb) CK(cudaEventRecord(eb, c->stream));
   PM_CK_PENDING("pm_match");
   L.kfn<<<L.blocks, L.threads, L.smem, c->stream>>>(L.a);
@@ -2642,10 +2733,9 @@ extern "C" pm_status pm_match(pm_ctx* c, const pm_graph* g, const pm_plan* const
   pm_status st = setup_launch(c, g, plans, nplans, o, &c->d_roots, &c->roots_bytes, &c->d_arena, &c->arena_bytes,
                               &c->d_ctl, &c->ctl_bytes, L.get());
   if (st != PM_OK) return st;
-  c->h_active = L->active0;
   unsigned long long host_ctl[kCtlRead];
   pm_stats pst;
-  st = run_launch(c, g, *L, [&]() { return enqueue_launch(c, *L, &c->h_active, host_ctl, e1, e2); }, &pst);
+  st = run_launch(c, g, *L, [&]() { return enqueue_launch(c, *L, host_ctl, e1, e2); }, &pst);
   if (st != PM_OK) return st;
   float kms = 0, rms = 0;
   CK(cudaEventElapsedTime(&kms, e1, e2));
@@ -2667,7 +2757,6 @@ struct pm_query {
   size_t arena_bytes = 0;
   unsigned long long* d_ctl = nullptr;
   size_t ctl_bytes = 0;
-  unsigned int* h_active = nullptr;   // pinned
   unsigned long long* h_ctl = nullptr;  // pinned
   cudaEvent_t eb = nullptr, ee = nullptr;
   cudaGraph_t graph = nullptr;
@@ -2685,7 +2774,6 @@ extern "C" void pm_query_free(pm_query* q) {
   free_dev(q->d_roots);
   free_dev(q->d_arena);
   free_dev(q->d_ctl);
-  if (q->h_active) cudaFreeHost(q->h_active);
   if (q->h_ctl) cudaFreeHost(q->h_ctl);
   delete q;
 }
@@ -2707,14 +2795,12 @@ extern "C" pm_status pm_query_prepare(pm_ctx* c, const pm_graph* g, const pm_pla
   CK(cudaEventRecord(c->ev[1], c->stream));
   CK(cudaEventSynchronize(c->ev[1]));
   CK(cudaEventElapsedTime(&q->roots_ms, c->ev[0], c->ev[1]));
-  CK(cudaMallocHost(&q->h_active, sizeof(unsigned int)));
   CK(cudaMallocHost(&q->h_ctl, sizeof(unsigned long long) * kCtlRead));
-  *q->h_active = q->L.active0;
   CK(cudaEventCreate(&q->eb));
   CK(cudaEventCreate(&q->ee));
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   // timing events stay outside the graph (recorded around each replay)
-  pm_status est = enqueue_launch(c, q->L, q->h_active, q->h_ctl, nullptr, nullptr);
+  pm_status est = enqueue_launch(c, q->L, q->h_ctl, nullptr, nullptr);
   cudaError_t cerr = cudaStreamEndCapture(c->stream, &q->graph);
   if (est != PM_OK) return est;
   CK(cerr);
@@ -2918,6 +3004,8 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.nplans = 1;
   a.T = T;
   a.chunk = o.chunk > 0 ? o.chunk : 16;
+  a.pop = o.chunk > 0 ? o.chunk
+                      : (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, (int64_t)nroots / (8 * blocks * wpb)));
   a.shard_rank = 0;
   a.shard_count = 1;
   a.split_min = o.split_level1 == 0 ? 64 : (o.split_level1 < 0 ? 0 : o.split_level1);
@@ -2926,10 +3014,9 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.cursors = w; w += 32;
   a.counts = w; w += 32;
   a.stats = w; w += kStatWords;
-  a.status = (unsigned int*)w;
-  a.active = (unsigned int*)w + 1; w += 1;
-  a.don_head = w; w += 1;
-  a.don_tail = w; w += 1;
+  a.status = (unsigned int*)w; w += 1;
+  a.sched = w; w += 1;
+  a.started = (unsigned int*)w; w += 1;
   a.heartbeat = w; w += 5;
   a.don_ready = w; w += kStaticRing;
   a.don_items = (int4*)w; w += 6 * kStaticRing;
@@ -2942,8 +3029,6 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.gather_words = 0;
   a.n_big = 0;
   a.timeout_ns = (unsigned long long)(o.timeout_ms > 0 ? o.timeout_ms : 600000) * 1000000ull;
-  const unsigned int active0 = (unsigned int)warps;
-  CK(cudaMemcpyAsync(a.active, &active0, sizeof(active0), cudaMemcpyHostToDevice, st));
   PM_CK_PENDING("pm_match_static");
   kfn<<<(int)blocks, wpb * 32, sizeof(WarpState) * wpb, st>>>(a);
   CK(cudaGetLastError());

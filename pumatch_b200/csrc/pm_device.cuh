@@ -146,6 +146,5 @@ struct pm_ctx {
   int32_t* d_vcount = nullptr;
   int64_t* d_voff = nullptr;
   size_t vbuf_n = 0;
-  unsigned int h_active = 0;  // staging for the initial active-warp count
 };
 
