@@ -83,6 +83,14 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
   return v;
 }
 
+// One value a warp has worked out and may meet again (pair_levels).
+struct alignas(16) MemoEntry {
+  int32_t x;
+  uint32_t tag;   // epoch of the (h0, bound); 0: never written
+  int32_t value;  // |N(x) n h0| below the bound
+  int32_t len;    // length of x's operand (the reference's scan)
+};
+
 struct MatchArgs {
   const uint64_t* rowptr;
   const int32_t* colidx;        // HBM residency
@@ -92,6 +100,14 @@ struct MatchArgs {
   const int32_t* host_sorted;   // labeled paged: the id-sorted lists in mapped host memory
   int32_t leaf_flat;            // last level: 0 one candidate per lane, 1 flat in lane-contiguous parts,
                                 // 2 flat strided (leaf_flat)
+  int32_t clique_bits;          // cliques in bit sets
+  int32_t pairs;                // last two levels in one pass where the plan allows (pair_levels)
+  int32_t memo_entries;         // entries of a warp's value table (a power of two), and the tables: each
+  MemoEntry* memo;              // warp's entries, then one that holds the last epoch it used (null: none)
+  const unsigned long long* asym;  // 0 when every adjacency entry has its reverse
+  const int32_t* hub_slot;      // unlabeled, HBM: [n] bit row of a vertex with a long list, or -1 (null: none)
+  const unsigned* hub_bits;     // bit rows of hub_words words: bit u of v's row = u is in v's list
+  int32_t hub_words;
   int32_t lane_subtree_max;     // lane_subtree when the parent set is at most this long; 0 = never
   int32_t nl1;
   int32_t n;
@@ -152,6 +168,16 @@ struct MatchArgs {
   DPlan plans[PM_MAX_BATCH];
 };
 
+// The warps' value tables (pair_levels): kept with the context or the query,
+// zeroed when their layout changes -- epochs go on from launch to launch, so
+// what an earlier launch left is never taken for a value.
+struct MemoTables {
+  MemoEntry* d = nullptr;
+  size_t bytes = 0;
+  int64_t warps = 0;
+  int entries = 0;
+};
+
 enum { ST_SETOPS = 0, ST_BYTES = 1, ST_ROOTS = 2, ST_SPLITS = 3, ST_HITS = 4, ST_MISSES = 5,
        ST_ZC_BYTES = 6, ST_REQUESTS = 7, ST_EVICTIONS = 8, ST_DROPPED = 9, ST_WARP_NS = 10, ST_IDLE_NS = 11,
        ST_BORROWS = 12, ST_LEAF_CYC = 13, ST_LEVEL_CYC = 14, ST_PREFIX_CYC = 15, ST_PREFETCH = 16,
@@ -162,15 +188,29 @@ constexpr int kStatWords = 24;
 #define PM_SB_MAX 512      // ints of a leaf batch's common operand kept in shared memory
 #define PM_LANE_MAX 96     // longest first operand one lane handles alone in a leaf batch
 #define PM_LEAF_BATCH 512  // candidates per leaf batch
-#define PM_WIN 256         // window of a merged second operand held in shared memory
 
 struct alignas(16) WarpState {
   int32_t path[8];
   int32_t iter[8];
   int32_t iend[8];   // exclusive end of the iteration range per level
   int32_t top[9];    // arena offset where level L's slots start
-  int32_t off[16];
-  int32_t size[16];
+  int32_t size[16];          // members of each slot
+  int32_t raw[16];           // elements at ptr: the members and the path vertices among them
+  const int32_t* ptr[16];    // each slot's elements: in the arena, or in place in an adjacency array
+  unsigned long long id[16]; // names a slot's contents: same name and length, same elements
+  unsigned long long next_id;
+  unsigned long long sb_id;  // contents the structure in sb was built from (0: none), and what it is
+  int32_t sb_len, sb_mode, sb_lo, sb_hi;
+  unsigned long long cq_id;  // clique search in bit sets: the set its matrix is over, where, how many rows
+  unsigned* cq_rows;
+  int32_t cq_n;
+  // pair_levels: the warp's value table, the epoch in use and what it stands for
+  MemoEntry* memo;
+  unsigned long long memo_id;
+  uint32_t memo_epoch;
+  int32_t memo_len, memo_ub;
+  int32_t queue[64];
+  int32_t lcnt[32];
   long long next_check;          // SM clock at which to look for waiting warps and at the deadline
   long long began;               // SM clock at the start of the current root or piece
   int32_t checks;                // checks made (the heartbeat is bumped on every 16th)
@@ -186,7 +226,6 @@ struct alignas(16) WarpState {
                                          // bulk copy that starts up to 3 words before it
   unsigned long long mbar;               // completion barrier of the warp's bulk copies
   uint32_t mphase;                       // its current phase
-  int32_t wb[PM_WIN];               // intersections by merge: the current window of the second operand
   unsigned long long lrb[32];       // leaf batches: start of each candidate's first operand in colidx
   int32_t lexcl[33];                // leaf batches: offset of each candidate's operand in the flat layout
 };
@@ -282,14 +321,17 @@ __device__ __forceinline__ ListRef adj_label(const MatchArgs& a, WarpState& S, i
 // mbarrier) and returns where src[0] landed: the copy starts at src rounded
 // down to 16 bytes and covers whole 16-byte units, which stay inside the
 // arena's allocation (every arena allocation has at least 256 bytes of slack
-// after its last word).  The wait is bounded: a copy not complete after
+// after its last word); a slot read in place in an adjacency array is copied
+// by the lanes.  The wait is bounded: a copy not complete after
 // ~2^20 polls returns src itself (the caller reads B from global memory and
 // reports DEV_TIMEOUT).
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __noinline__ const int32_t* stage_bulk(WarpState& S, const int32_t* src, int n) {
   const int lane = lane_id();
-  if (n < PM_BULK_MIN) {
+  __syncwarp();
+  if (lane == 0) S.sb_id = 0;  // the buffer no longer holds the structure built last
+  if (n < PM_BULK_MIN || src < S.arena || src >= S.arena + S.cap) {
     __syncwarp();
     for (int i = lane; i < n; i += 32) S.sb[i] = src[i];
     __syncwarp();
@@ -359,6 +401,11 @@ __device__ __noinline__ unsigned borrow_arena(const MatchArgs& a, WarpState& S, 
   const int32_t* src = S.arena;
   for (int64_t i = lane; i < live; i += 32) dst[i] = src[i];
   __syncwarp();
+  if (lane < 16) {  // slots that live in the arena move with it
+    const int32_t* q = S.ptr[lane];
+    if (q >= src && q < src + live) S.ptr[lane] = dst + (q - src);
+  }
+  __syncwarp();
   if (lane == 0) {
     S.arena = dst;
     S.cap = a.big_slot_words;
@@ -415,167 +462,6 @@ __device__ __forceinline__ bool gather_room(const MatchArgs& a, WarpState& S, in
   return false;
 }
 
-// ---------------------------------------------------------------------
-// One slot of level L for the warp's current path.  Restates compute_set
-// (src/gpu_match.cu:238-319) with the operand choice of extend
-// (src/gpu_match.cu:409-812): returns the slot size (at the last level the
-// count), writes the slot to arena[top...] unless `last`.
-// ---------------------------------------------------------------------
-template <bool LABELED, bool PAGED>
-__device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int s, int top, bool last,
-                        Work& w) {
-  const int lane = lane_id();
-  const int kind = P.kind[s];
-  const int vL = S.path[L];
-  ListRef RA, RB{nullptr, 0, -1};
-  // one-label masks read only that label's part of an adjacency list: same
-  // survivors in the same order, no label gathers (accounting still charges
-  // the whole list, as the reference scans it)
-  const uint32_t mask0 = P.slot_labels[s];
-  const bool by_label = LABELED && a.lab_off && __popc(mask0) == 1 && (kind != SLOT_COPY || L == 1);
-  if (PAGED) {
-    // the adjacency operands may be copied into the gather halves: make room
-    auto list_len = [&](int v) -> int64_t {
-      return by_label ? label_range(a, v, __ffs(mask0) - 1).y : (int64_t)(a.rowptr[v + 1] - a.rowptr[v]);
-    };
-    int64_t need = 0;
-    if (kind != SLOT_COPY) need = list_len(vL);
-    else if (L == 1) need = list_len(S.path[0]);
-    if (kind == SLOT_INTERSECT && L == 1) need = max(need, list_len(S.path[0]));
-    if (!gather_room(a, S, top, need, w)) return 0;
-  }
-  int32_t* arena = S.arena;
-  int32_t* gatherA = S.gather;
-  int32_t* gatherB = S.gather + S.ghalf;
-  int full_len = -1;  // length of the whole list when by_label
-  int full_lenB = -1; // the same for a level-1 second operand read by label (paged)
-  if (by_label) {
-    const int v = (kind != SLOT_COPY) ? vL : S.path[0];
-    full_len = (int)(a.rowptr[v + 1] - a.rowptr[v]);
-    RA = adj_label<PAGED>(a, S, v, __ffs(mask0) - 1, gatherA, w);
-  } else if (kind != SLOT_COPY) {
-    RA = adj<PAGED>(a, S, vL, gatherA, w);
-  } else if (L > 1) {
-    RA = ListRef{arena + S.off[P.parent[s]], S.size[P.parent[s]], -1};
-  } else {
-    RA = adj<PAGED>(a, S, S.path[0], gatherA, w);
-  }
-  if (kind == SLOT_INTERSECT) {
-    if (L > 1) {
-      RB = ListRef{arena + S.off[P.parent[s]], S.size[P.parent[s]], -1};
-    } else if (PAGED && by_label) {
-      // only the label-l part of N(v0) can meet the label-l part of N(vL)
-      const int v0 = S.path[0];
-      full_lenB = (int)(a.rowptr[v0 + 1] - a.rowptr[v0]);
-      RB = adj_label<PAGED>(a, S, v0, __ffs(mask0) - 1, gatherB, w);
-    } else {
-      RB = adj<PAGED>(a, S, S.path[0], gatherB, w);
-    }
-  }
-  const int32_t* A = RA.p;
-  const int32_t* B = RB.p;
-  int lenA = RA.len;
-  const int lenB = RB.len;
-  const bool cgA = RA.cg;
-  bool cgB = RB.cg;
-  // a parent slot small enough goes to shared memory for the per-lane searches
-  bool b_shared = false;
-  if (kind == SLOT_INTERSECT && L > 1 && lenB <= PM_SB_MAX) {
-    if (lenB > 0) {
-      const int32_t* Bs = stage_bulk(S, B, lenB);
-      b_shared = Bs != B;
-      if (!b_shared) w.err |= DEV_TIMEOUT;
-      B = Bs;
-      cgB = cgB && !b_shared;
-    }
-  }
-
-  // symmetry-breaking upper bound (unlabeled only, src/gpu_match.cu:426-458)
-  if (!LABELED && P.partial[s]) {
-    const bool is_main = (s == P.level_begin[L]);
-    long long ub = is_main ? INT_MAX : -1;
-    for (int j = 0; j <= L; j++) {
-      if (!(P.partial[s] & (1u << j))) continue;
-      const long long v = S.path[j];
-      if (is_main) { if (v <= ub) ub = v; }
-      else if (ub < v) ub = v;
-    }
-    if (ub == -1) ub = INT_MAX;
-    if (ub != INT_MAX) lenA = warp_lower_bound<PAGED>(A, lenA, (int)ub, cgA);
-  }
-
-  const int T = a.T;
-  int scan = lenA;
-  const bool fresh_unl = (!LABELED && kind == SLOT_FRESH);
-  if (fresh_unl && T && scan > T) scan = T;  // first pass keeps A's prefix
-  int cnt = 0;
-  // the slot holds at most the first T survivors
-  if (!last && !slot_room(a, S, top, (T && scan > T) ? T : scan, w)) scan = 0;
-  int32_t* out = S.arena + top;
-  const uint32_t mask = P.slot_labels[s];
-  // an intersection whose second operand is not in shared memory and at
-  // most 4x the scanned part of the first: merge, B streamed through shared
-  // memory in coalesced windows; else a search per element of A (which reads
-  // less of a much longer B)
-  const bool merge = kind == SLOT_INTERSECT && !b_shared && lenB > PM_WIN && (long long)lenB <= 4ll * scan;
-  int bpos = 0;  // merge: B[0, bpos) is below every element still to come
-  for (int base = 0; base < scan; base += 32) {
-    const int i = base + lane;
-    const bool valid = i < scan;
-    const int x = valid ? ld<PAGED>(A + i, cgA) : 0;
-    bool keep = valid;
-    if (merge) {
-      const int xlo = __shfl_sync(FULL, x, 0);
-      const int xhi = __shfl_sync(FULL, x, min(31, scan - 1 - base));
-      bpos += warp_lower_bound<PAGED>(B + bpos, lenB - bpos, xlo, cgB);
-      bool open = valid;  // this lane's membership still undecided
-      keep = false;
-      while (__any_sync(FULL, open)) {
-        const int wn = min(PM_WIN, lenB - bpos);
-        if (wn <= 0) break;  // B exhausted: the rest of the tile is not in B
-        __syncwarp();
-        for (int k = lane; k < wn; k += 32) S.wb[k] = ld<PAGED>(B + bpos + k, cgB);
-        __syncwarp();
-        const int wlast = S.wb[wn - 1];
-        if (open && x <= wlast) {
-          keep = bsearch_in<false>(S.wb, wn, x);
-          open = false;
-        }
-        if (xhi <= wlast) break;
-        bpos += wn;
-      }
-      // bpos stays at the last window: it may hold elements of the next tile
-    } else if (kind == SLOT_INTERSECT && keep) {
-      keep = bsearch_in<PAGED>(B, lenB, x, cgB);
-    }
-    if (LABELED) {
-      if (keep && !by_label) keep = (mask >> a.labels[x]) & 1u;
-    } else if (kind == SLOT_COPY) {
-      keep = keep && x != vL;
-    } else if (kind == SLOT_FRESH) {
-      for (int j = 0; j <= L; j++) keep = keep && x != S.path[j];
-    }
-    const unsigned bal = __ballot_sync(FULL, keep);
-    if (!last && keep) {
-      const int pos = cnt + __popc(bal & lanemask_lt());
-      if (!T || pos < T) out[pos] = x;
-    }
-    cnt += __popc(bal);
-    if (T && cnt >= T && !fresh_unl) break;  // result is the first T survivors
-  }
-  if (PAGED) {
-    __syncwarp();
-    unpin(a.pg, RA);
-    unpin(a.pg, RB);
-  }
-  if (T && cnt > T) cnt = T;
-  const int alenA = by_label ? full_len : lenA;
-  const int alenB = full_lenB >= 0 ? full_lenB : lenB;
-  w.setops++;
-  w.bytes += 4ull * (unsigned long long)(alenA + alenB + cnt) + (LABELED ? (unsigned long long)alenA : 0ull);
-  return cnt;
-}
-
 // Bound of slot s at level L from the partial order: the smallest (main
 // slot) or largest (helper slot) constrained path vertex; INT_MAX if none.
 template <bool LABELED>
@@ -592,6 +478,457 @@ __device__ __forceinline__ int slot_bound(const DPlan& P, const WarpState& S, in
   return ub == -1 ? INT_MAX : (int)ub;
 }
 
+// Membership structures for a second operand B (sorted), built in the warp's
+// shared staging buffer (PM_SB_MAX words):
+enum : int {
+  MEMB_BITMAP = 0,  // max B < 32 * PM_SB_MAX: one bit per id in [0, max B]
+  MEMB_FILTER = 1,  // |B| <= PM_FILTER_MAX: a one-hash filter of 32 * PM_SB_MAX bits, then a search of B itself
+  MEMB_NONE = 2     // longer: a search of B for every element
+};
+// At this length a third of the filter's bits are set: two of three searches
+// are still spared.
+#define PM_FILTER_MAX 8192
+
+struct LeafSet {
+  const int32_t* t;
+  const int32_t* g;  // B itself (MEMB_FILTER)
+  int lenB;
+  int lo, hi;        // min and max of B: outside [lo, hi] nothing is a member
+};
+
+// Whether x can be a member: exact for the bitmap, what the filter says else.
+template <int MODE>
+__device__ __forceinline__ bool leaf_maybe(const LeafSet& m, int x) {
+  if (x < m.lo || x > m.hi) return false;
+  const unsigned f = MODE == MEMB_BITMAP ? (unsigned)x : ((unsigned)x * 0x2545F491u) >> 18;  // 14 bits: the buffer
+  return (((const unsigned int*)m.t)[f >> 5] >> (f & 31)) & 1u;
+}
+
+template <int MODE>
+__device__ __forceinline__ bool leaf_member(const LeafSet& m, int x) {
+  return leaf_maybe<MODE>(m, x) && (MODE == MEMB_BITMAP || bsearch_in<false>(m.g, m.lenB, x));
+}
+
+// The structure for B (whole warp); returns its mode.  `id` names B's
+// contents (WarpState::id; 0: unnamed): a structure built for the same
+// contents and length is still in the buffer and is used again -- the parent
+// set of a level is the second operand of every candidate of that level.
+template <bool CG = false>
+__device__ __forceinline__ int leaf_build(WarpState& S, const int32_t* B, int lenB, unsigned long long id, LeafSet& m,
+                                          bool cg = true) {
+  const int lane = lane_id();
+  m.t = S.sb;
+  m.g = B;
+  m.lenB = lenB;
+  if (id && id == S.sb_id && lenB == S.sb_len) {
+    m.lo = S.sb_lo;
+    m.hi = S.sb_hi;
+    return S.sb_mode;
+  }
+  m.lo = lenB ? ld<CG>(B, cg) : 1;
+  m.hi = lenB ? ld<CG>(B + lenB - 1, cg) : 0;
+  const int mode = m.hi < 32 * PM_SB_MAX ? MEMB_BITMAP : lenB <= PM_FILTER_MAX ? MEMB_FILTER : MEMB_NONE;
+  if (mode == MEMB_NONE) return mode;
+  __syncwarp();
+  unsigned int* bits = (unsigned int*)S.sb;
+  const int words = mode == MEMB_FILTER ? PM_SB_MAX : lenB ? (m.hi >> 5) + 1 : 0;
+  for (int i = lane; i < words; i += 32) bits[i] = 0;
+  __syncwarp();
+  for (int base = 0; base < lenB; base += 128) {  // four loads in flight
+    int x[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = base + 32 * q + lane;
+      x[q] = i < lenB ? ld<CG>(B + i, cg) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const unsigned f = mode == MEMB_FILTER ? ((unsigned)x[q] * 0x2545F491u) >> 18 : (unsigned)x[q];
+      if (x[q] >= 0) atomicOr(&bits[f >> 5], 1u << (f & 31));
+    }
+  }
+  if (lane == 0) {
+    S.sb_id = id;
+    S.sb_len = lenB;
+    S.sb_mode = mode;
+    S.sb_lo = m.lo;
+    S.sb_hi = m.hi;
+  }
+  __syncwarp();
+  return mode;
+}
+
+// Position of x in sorted A[0, len) (first element >= x), one search per
+// group of four lanes (x and len uniform within a group, len 0 = no search):
+// five-way steps, so eight searches run side by side in log5(len) round trips.
+template <bool CG>
+__device__ __forceinline__ int group_lower_bound(const int32_t* A, int len, int x, bool cg = true) {
+  const int lane = lane_id();
+  const int g4 = lane & 3, sh = lane & ~3;
+  int lo = 0, hi = len;
+  while (__any_sync(FULL, lo < hi)) {
+    const int span = hi - lo;
+    const int step = (span + 4) / 5;  // 0 for a finished group
+    const int idx = lo + (g4 + 1) * step - 1;
+    const bool lt = step > 0 && idx < hi && ld<CG>(A + idx, cg) < x;
+    const int k = __popc((__ballot_sync(FULL, lt) >> sh) & 15u);
+    if (step > 0) {
+      if (k < 4) hi = min(hi, lo + (k + 1) * step - 1);  // the first probe not below x
+      lo += k * step;
+    }
+  }
+  return lo;
+}
+
+// Four searches at once: whether each x[q] is in sorted B[0, len).  The steps
+// do not depend on what is found, so the four loads of a step are in flight
+// together.
+template <bool CG>
+__device__ __forceinline__ void bsearch4(const int32_t* B, int len, const int (&x)[4], bool (&in)[4], bool cg) {
+  int p[4] = {0, 0, 0, 0};
+  if (len <= 0) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) in[q] = false;
+    return;
+  }
+  for (int n = len; n > 1;) {
+    const int h = n >> 1;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (ld<CG>(B + p[q] + h, cg) <= x[q]) p[q] += h;
+    n -= h;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) in[q] = in[q] && ld<CG>(B + p[q], cg) == x[q];
+}
+
+// The elements of A[0, n) that `keep` leaves (keep(x, in): in[q] comes in as
+// "x[q] is an element"), in order: counted, and written to out (unless null)
+// up to T of them (T 0: all).  Four loads in flight per lane: one tile of 32
+// per step left the warp waiting a load's latency for every tile.
+template <bool CG, class Keep>
+__device__ __forceinline__ int compact(const int32_t* A, int n, bool cg, int32_t* out, int T, Keep keep) {
+  const int lane = lane_id();
+  int cnt = 0;
+  for (int base = 0; base < n; base += 128) {
+    int x[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = base + 32 * q + lane;
+      in[q] = i < n;
+      x[q] = in[q] ? ld<CG>(A + i, cg) : 0;
+    }
+    keep(x, in);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const unsigned bal = __ballot_sync(FULL, in[q]);
+      if (out && in[q]) {
+        const int pos = cnt + __popc(bal & lanemask_lt());
+        if (!T || pos < T) out[pos] = x[q];
+      }
+      cnt += __popc(bal);
+    }
+    if (T && cnt >= T) break;  // the result is the first T survivors
+  }
+  return cnt;
+}
+
+// Whether u in N(v) says v in N(u): an undirected graph, as the interface
+// asks for.  What is taken from one list about the other asks first.
+__device__ __forceinline__ bool symmetric(const MatchArgs& a) { return a.asym && *a.asym == 0ull; }
+
+// v's bit row (pm_graph::d_hub_bits), or null when its list is short.
+__device__ __forceinline__ const unsigned* hub_row(const MatchArgs& a, int v) {
+  if (!a.hub_slot) return nullptr;
+  const int k = a.hub_slot[v];
+  return k < 0 ? nullptr : a.hub_bits + (long long)k * a.hub_words;
+}
+
+// Makes slot s the elements [0, raw) at ptr, `size` of them members (the rest
+// are path vertices, skipped when the slot is walked).  Lane 0 writes.
+__device__ __forceinline__ void set_slot(WarpState& S, int s, const int32_t* ptr, int raw, int size,
+                                         unsigned long long id) {
+  if (lane_id() == 0) {
+    S.ptr[s] = ptr;
+    S.raw[s] = raw;
+    S.size[s] = size;
+    S.id[s] = id;
+  }
+}
+
+// Name of an adjacency array's part in device memory (its contents never
+// change): distinct from the running numbers of slots a warp wrote itself.
+__device__ __forceinline__ unsigned long long list_id(const int32_t* p) {
+  return (unsigned long long)(uintptr_t)p | (1ull << 63);
+}
+
+// ---------------------------------------------------------------------
+// One slot of level L for the warp's current path.  Restates compute_set
+// (src/gpu_match.cu:238-319) with the operand choice of extend
+// (src/gpu_match.cu:409-812).  With `last` returns the count; else fills the
+// slot and returns the arena words it took at `top`.
+//
+// What bounds a level is latency: dependent reads of L2-resident lists.  So
+// nothing is copied that can be read where it is: a fresh set is the
+// adjacency list itself, cut at its bound, with the path vertices in it
+// skipped by whoever walks it (DPlan.hole_ok: only where nothing else reads
+// the slot); a copy that removes nothing is its parent.  Intersections test
+// four elements per lane at a time against a structure in shared memory that
+// the candidates of a level share (leaf_build), or look the shorter operand
+// up in the longer when that is 16 times as long.
+// Measured (B200), cycles of all warps in levels above the last, the 20-pattern
+// labeled batch on an R-MAT graph of 65,536 vertices: 1.4e12 -> 1.0e12; the
+// launch 433 -> 309 ms.
+// ---------------------------------------------------------------------
+template <bool LABELED, bool PAGED>
+__device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int s, int top, bool last,
+                        Work& w) {
+  const int lane = lane_id();
+  const int kind = P.kind[s];
+  const int par = P.parent[s];
+  const int vL = S.path[L];
+  const int T = a.T;
+  const uint32_t mask = P.slot_labels[s];
+  // a labeled copy whose parent holds no other labels is its parent
+  if (LABELED && kind == SLOT_COPY && L > 1 && !(P.slot_labels[par] & ~mask)) {
+    const int len = S.size[par];
+    w.setops++;
+    w.bytes += 9ull * (unsigned long long)len;  // 4 (|A| + |C|) + |A|
+    if (!last) set_slot(S, s, S.ptr[par], len, len, S.id[par]);
+    return last ? len : 0;
+  }
+  ListRef RA, RB{nullptr, 0, -1};
+  // one-label masks read only that label's part of an adjacency list: same
+  // survivors in the same order, no label gathers (accounting still charges
+  // the whole list, as the reference scans it)
+  const bool by_label = LABELED && a.lab_off && __popc(mask) == 1 && (kind != SLOT_COPY || L == 1);
+  if (PAGED) {
+    // the adjacency operands may be copied into the gather halves: make room
+    auto list_len = [&](int v) -> int64_t {
+      return by_label ? label_range(a, v, __ffs(mask) - 1).y : (int64_t)(a.rowptr[v + 1] - a.rowptr[v]);
+    };
+    int64_t need = 0;
+    if (kind != SLOT_COPY) need = list_len(vL);
+    else if (L == 1) need = list_len(S.path[0]);
+    if (kind == SLOT_INTERSECT && L == 1) need = max(need, list_len(S.path[0]));
+    if (!gather_room(a, S, top, need, w)) {
+      if (!last) set_slot(S, s, S.arena + top, 0, 0, 0);
+      return 0;
+    }
+  }
+  int32_t* gatherA = S.gather;
+  int32_t* gatherB = S.gather + S.ghalf;
+  int full_len = -1;  // length of the whole list when by_label
+  int full_lenB = -1; // the same for a level-1 second operand read by label (paged)
+  unsigned long long idA = 0, idB = 0;
+  if (by_label) {
+    const int v = (kind != SLOT_COPY) ? vL : S.path[0];
+    full_len = (int)(a.rowptr[v + 1] - a.rowptr[v]);
+    RA = adj_label<PAGED>(a, S, v, __ffs(mask) - 1, gatherA, w);
+  } else if (kind != SLOT_COPY) {
+    RA = adj<PAGED>(a, S, vL, gatherA, w);
+  } else if (L > 1) {
+    RA = ListRef{S.ptr[par], S.size[par], -1};
+    idA = S.id[par];
+  } else {
+    RA = adj<PAGED>(a, S, S.path[0], gatherA, w);
+  }
+  if (!PAGED && !idA) idA = list_id(RA.p);
+  if (kind == SLOT_INTERSECT) {
+    if (L > 1) {
+      RB = ListRef{S.ptr[par], S.size[par], -1};
+      idB = S.id[par];
+    } else if (PAGED && by_label) {
+      // only the label-l part of N(v0) can meet the label-l part of N(vL)
+      const int v0 = S.path[0];
+      full_lenB = (int)(a.rowptr[v0 + 1] - a.rowptr[v0]);
+      RB = adj_label<PAGED>(a, S, v0, __ffs(mask) - 1, gatherB, w);
+    } else {
+      RB = adj<PAGED>(a, S, S.path[0], gatherB, w);
+      if (!PAGED) idB = list_id(RB.p);
+    }
+  }
+  const int32_t* A = RA.p;
+  const int32_t* B = RB.p;
+  int lenA = RA.len;
+  const int lenB = RB.len;
+  const bool cgA = RA.cg, cgB = RB.cg;
+  // elements that stay where they are: device memory that outlives the slot
+  const bool in_place = !PAGED || (kind == SLOT_COPY && L > 1);
+
+  // symmetry-breaking upper bound (unlabeled only, src/gpu_match.cu:426-458)
+  // and, for fresh sets and copies, the path vertices to leave out
+  const int ub = slot_bound<LABELED>(P, S, L, s);
+  int cnt = 0, used = 0;
+  bool done = false;
+  if (!LABELED && kind != SLOT_INTERSECT) {
+    const int g = lane >> 2;
+    const int first = kind == SLOT_FRESH ? 0 : L;  // a copy leaves out the newest vertex only
+    const int j = first + g;
+    const bool out_v = g < 7 && j <= L;
+    const int x = out_v ? S.path[j] : ub;
+    const bool search = out_v || (g == 7 && ub != INT_MAX);
+    const int pos = group_lower_bound<PAGED>(A, search ? lenA : 0, x, cgA);
+    bool hole = out_v && pos < lenA && ld<PAGED>(A + pos, cgA) == x;
+    if (hole)
+      for (int k = first; k < j; k++) hole = hole && S.path[k] != x;  // one element, left out once
+    if (ub != INT_MAX) lenA = __shfl_sync(FULL, pos, 28);
+    // a fresh set truncated to T is what remains of the first T elements
+    const int scan = (kind == SLOT_FRESH && T && lenA > T) ? T : lenA;
+    const int holes = __popc(__ballot_sync(FULL, hole && (lane & 3) == 0 && pos < scan));
+    cnt = scan - holes;
+    if (T && cnt > T) {  // a copy longer than T: its first T survivors
+      cnt = T;
+      done = last;
+      if (in_place && !holes && !last) {
+        set_slot(S, s, A, T, T, idA);
+        done = true;
+      }
+    } else if (last) {
+      done = true;
+    } else if (in_place && (!holes || P.hole_ok[s])) {
+      set_slot(S, s, A, scan, cnt, idA);
+      done = true;
+    }
+    if (!done) {
+      if (slot_room(a, S, top, cnt, w)) {
+        int32_t* out = S.arena + top;
+        const int want = cnt;
+        compact<PAGED>(A, scan, cgA, out, want, [&](const int (&v)[4], bool (&in)[4]) {
+          for (int k = first; k <= L; k++) {
+            const int pk = S.path[k];
+#pragma unroll
+            for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] != pk;
+          }
+        });
+      } else {
+        cnt = 0;
+      }
+      used = cnt;
+    }
+  } else if (LABELED && by_label && kind != SLOT_INTERSECT) {
+    cnt = (T && lenA > T) ? T : lenA;
+    if (!last) {
+      if (in_place) {
+        set_slot(S, s, A, cnt, cnt, idA);
+        done = true;
+      } else {
+        if (slot_room(a, S, top, cnt, w))
+          compact<PAGED>(A, cnt, cgA, S.arena + top, 0, [](const int (&)[4], bool (&)[4]) {});
+        else
+          cnt = 0;
+        used = cnt;
+      }
+    }
+  } else {
+    // labeled by mask, or an intersection
+    if (ub != INT_MAX) lenA = warp_lower_bound<PAGED>(A, lenA, ub, cgA);
+    const bool check = LABELED && !by_label;
+    auto labelled = [&](const int (&v)[4], bool (&in)[4]) {
+      if (check) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) in[q] = in[q] && ((mask >> a.labels[v[q]]) & 1u);
+      }
+    };
+    const unsigned* row = nullptr;
+    int room = kind == SLOT_INTERSECT ? min(lenA, lenB) : lenA;
+    if (T && room > T) room = T;
+    int32_t* out = nullptr;
+    bool fits = true;
+    if (!last) {
+      fits = slot_room(a, S, top, room, w);
+      out = S.arena + top;
+    }
+    if (!fits || room == 0) {
+      cnt = 0;
+    } else if (kind != SLOT_INTERSECT) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, labelled);
+    } else if (!LABELED && !PAGED && lenB <= lenA && (row = hub_row(a, vL))) {
+      // the newest vertex has a bit row: one load per element of the parent
+      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] < ub && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
+      });
+    } else if (!LABELED && !PAGED && L == 1 && (row = hub_row(a, S.path[0]))) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) in[q] = in[q] && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
+      });
+    } else if ((long long)lenB * 16 < lenA) {
+      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+        bsearch4<PAGED>(A, lenA, v, in, cgA);
+        labelled(v, in);
+      });
+    } else if ((long long)lenA * 16 < lenB && !(idB && idB == S.sb_id && lenB == S.sb_len)) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+        bsearch4<PAGED>(B, lenB, v, in, cgB);
+        labelled(v, in);
+      });
+    } else {
+      LeafSet m;
+      const int mode = leaf_build<PAGED>(S, B, lenB, idB, m, cgB);
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+        if (mode == MEMB_BITMAP) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) in[q] = in[q] && leaf_maybe<MEMB_BITMAP>(m, v[q]);
+        } else {
+          if (mode == MEMB_FILTER) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) in[q] = in[q] && leaf_maybe<MEMB_FILTER>(m, v[q]);
+          }
+          if (__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) bsearch4<PAGED>(B, lenB, v, in, cgB);
+        }
+        labelled(v, in);
+      });
+    }
+    if (T && cnt > T) cnt = T;
+    if (!last) used = cnt;
+  }
+  if (!last && !done) {
+    __syncwarp();
+    unsigned long long id = 0;
+    if (lane == 0) id = ++S.next_id;
+    set_slot(S, s, S.arena + top, cnt, cnt, id);
+  }
+  if (PAGED) {
+    __syncwarp();
+    unpin(a.pg, RA);
+    unpin(a.pg, RB);
+  }
+  const int alenA = by_label ? full_len : lenA;
+  const int alenB = full_lenB >= 0 ? full_lenB : lenB;
+  w.setops++;
+  w.bytes += 4ull * (unsigned long long)(alenA + alenB + cnt) + (LABELED ? (unsigned long long)alenA : 0ull);
+  return last ? cnt : used;
+}
+
+// run_slot counting only, out of line: for the callers that rarely need it
+// (the search's own calls are inlined once; the kernel's code has to stay
+// within the instruction cache).  Its counters come back in `t`, so that the
+// caller's stay in registers.
+template <bool LABELED, bool PAGED>
+__device__ __noinline__ int count_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int s, int top,
+                                       Work* t) {
+  return run_slot<LABELED, PAGED>(a, P, S, L, s, top, true, *t);
+}
+
+__device__ __forceinline__ void add_work(Work& w, const Work& t) {
+  w.setops += t.setops;
+  w.bytes += t.bytes;
+  w.reads += t.reads;
+  w.borrows += t.borrows;
+  w.err |= t.err;
+  w.pc.hits += t.pc.hits;
+  w.pc.misses += t.pc.misses;
+  w.pc.zc_bytes += t.pc.zc_bytes;
+  w.pc.requests += t.pc.requests;
+  w.pc.evictions += t.pc.evictions;
+  w.pc.dropped += t.pc.dropped;
+  w.pc.dev_loads += t.pc.dev_loads;
+  w.pc.dev_bytes += t.pc.dev_bytes;
+}
+
 // A slot equal to, or a prefix of, a slot already computed at this level:
 // no scan, only the reference's accounting for the set operation it stands
 // for (its first operand's length below its bound, its result length).
@@ -604,9 +941,8 @@ __device__ void alias_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int
     if ((P.kind[s] != SLOT_COPY || L == 1) && !gather_room(a, S, live, (int64_t)(a.rowptr[v + 1] - a.rowptr[v]), w))
       return;
   }
-  const int32_t* arena = S.arena;
   int size = S.size[t];
-  if (P.alias_prefix[s] && ub != INT_MAX) size = warp_lower_bound<false>(arena + S.off[t], size, ub);
+  if (P.alias_prefix[s] && ub != INT_MAX) size = warp_lower_bound<false>(S.ptr[t], size, ub);
   // first operand length as the reference would scan it
   const int kind = P.kind[s];
   int lenA, lenB = 0;
@@ -625,7 +961,7 @@ __device__ void alias_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int
     }
   } else if (L > 1) {
     lenA = S.size[P.parent[s]];
-    if (ub != INT_MAX) lenA = warp_lower_bound<false>(arena + S.off[P.parent[s]], lenA, ub);
+    if (ub != INT_MAX) lenA = warp_lower_bound<false>(S.ptr[P.parent[s]], lenA, ub);
   } else {
     const int v = S.path[0];
     lenA = (int)(a.rowptr[v + 1] - a.rowptr[v]);
@@ -646,7 +982,7 @@ __device__ void alias_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int
   }
   w.setops++;
   w.bytes += 4ull * (unsigned long long)(lenA + lenB + size) + (LABELED ? (unsigned long long)lenA : 0ull);
-  if (lane_id() == 0) { S.off[s] = S.off[t]; S.size[s] = size; }
+  set_slot(S, s, S.ptr[t], size, size, S.id[t]);
 }
 
 // Computes every slot of level L; returns the arena top after them.
@@ -655,9 +991,7 @@ __device__ __forceinline__ int run_level(const MatchArgs& a, const DPlan& P, War
   int top = S.top[L];
   for (int s = P.level_begin[L]; s < P.level_begin[L + 1]; s++) {
     if (P.alias[s] >= 0) continue;
-    const int sz = run_slot<LABELED, PAGED>(a, P, S, L, s, top, false, w);
-    if (lane_id() == 0) { S.off[s] = top; S.size[s] = sz; }
-    top += sz;
+    top += run_slot<LABELED, PAGED>(a, P, S, L, s, top, false, w);
   }
   __syncwarp();
   for (int s = P.level_begin[L]; s < P.level_begin[L + 1]; s++) {
@@ -722,101 +1056,15 @@ __device__ __forceinline__ int lane_intersect(const int32_t* A, int deg, int ub,
   }
 }
 
-// Membership of x (>= 0) in an open-addressing table of 2^bits slots, empty
-// slots -1, at most half full (so every probe run ends at an empty slot).
-__device__ __forceinline__ bool in_table(const int32_t* t, int bits, int x) {
-  unsigned h = ((unsigned)x * 0x9E3779B1u) >> (32 - bits);
-  const unsigned m = (1u << bits) - 1;
-  while (true) {
-    const int y = t[h];
-    if (y == x) return true;
-    if (y < 0) return false;
-    h = (h + 1) & m;
-  }
-}
-
-// Membership structures for a leaf batch's common operand B (sorted), built
-// in the warp's shared staging buffer (PM_SB_MAX words):
-enum : int {
-  MEMB_BITMAP = 0,  // max B < 32 * PM_SB_MAX: one bit per id in [0, max B]
-  MEMB_FILTER = 1,  // |B| <= PM_SB_MAX / 4: a one-hash filter of 16 * PM_SB_MAX bits, then a hash table
-  MEMB_HASH = 2,    // |B| <= PM_SB_MAX / 2: an open-addressing table at most half full
-  MEMB_SORTED = 3   // else: the sorted copy, binary search
-};
-
-struct LeafSet {
-  const int32_t* t;
-  int bits;       // hash table: log2(slots)
-  int lo, hi;     // min and max of B: outside [lo, hi] nothing is a member
-};
-
-__device__ __forceinline__ unsigned leaf_hash(int x, int bits) { return ((unsigned)x * 0x9E3779B1u) >> (32 - bits); }
-
-template <int MODE>
-__device__ __forceinline__ bool leaf_member(const LeafSet& m, int lenB, int x) {
-  if (x < m.lo || x > m.hi) return false;
-  if (MODE == MEMB_BITMAP) return (((const unsigned int*)m.t)[x >> 5] >> (x & 31)) & 1u;
-  if (MODE == MEMB_FILTER) {
-    const unsigned f = ((unsigned)x * 0x2545F491u) >> 19;  // 13 bits: PM_SB_MAX / 2 words of filter
-    if (!((((const unsigned int*)m.t)[f >> 5] >> (f & 31)) & 1u)) return false;
-    return in_table(m.t + PM_SB_MAX / 2, m.bits, x);
-  }
-  if (MODE == MEMB_HASH) return in_table(m.t, m.bits, x);
-  return bsearch_in<false>(m.t, lenB, x);
-}
-
-// Builds the structure for B (whole warp) and returns its mode.
-__device__ int leaf_build(WarpState& S, const int32_t* B, int lenB, LeafSet& m) {
-  const int lane = lane_id();
-  m.t = S.sb;
-  m.lo = lenB ? B[0] : 1;
-  m.hi = lenB ? B[lenB - 1] : 0;
-  m.bits = 5;
-  int mode;
-  if (m.hi < 32 * PM_SB_MAX) {
-    mode = MEMB_BITMAP;
-    const int words = lenB ? (m.hi >> 5) + 1 : 0;
-    for (int i = lane; i < words; i += 32) S.sb[i] = 0;
-    __syncwarp();
-    for (int i = lane; i < lenB; i += 32) atomicOr((unsigned int*)&S.sb[B[i] >> 5], 1u << (B[i] & 31));
-  } else if (lenB <= PM_SB_MAX / 2) {
-    mode = lenB <= PM_SB_MAX / 4 ? MEMB_FILTER : MEMB_HASH;
-    int32_t* tab = S.sb + (mode == MEMB_FILTER ? PM_SB_MAX / 2 : 0);
-    const int cap = mode == MEMB_FILTER ? PM_SB_MAX / 2 : PM_SB_MAX;
-    while ((1 << m.bits) < 2 * lenB) m.bits++;
-    if (mode == MEMB_FILTER) {
-      while ((2 << m.bits) <= cap && (1 << m.bits) < 4 * lenB) m.bits++;  // at most a quarter full
-      for (int i = lane; i < PM_SB_MAX / 2; i += 32) S.sb[i] = 0;
-    }
-    const int size = 1 << m.bits;  // <= cap
-    for (int i = lane; i < size; i += 32) tab[i] = -1;
-    __syncwarp();
-    for (int i = lane; i < lenB; i += 32) {
-      const int x = B[i];
-      if (mode == MEMB_FILTER) {
-        const unsigned f = ((unsigned)x * 0x2545F491u) >> 19;
-        atomicOr((unsigned int*)&S.sb[f >> 5], 1u << (f & 31));
-      }
-      unsigned h = leaf_hash(x, m.bits);
-      while (atomicCAS(&tab[h], -1, x) != -1) h = (h + 1) & (unsigned)(size - 1);
-    }
-  } else {
-    mode = MEMB_SORTED;
-    for (int i = lane; i < lenB; i += 32) S.sb[i] = B[i];
-  }
-  __syncwarp();
-  return mode;
-}
-
 // One lane's contiguous part [t, tend) of a leaf batch's flat layout
 // (candidate j's first operand occupies [lexcl[j], lexcl[j+1]) and starts at
-// colidx[lrb[j]]): members of B, label-checked when LABELED.
+// lists[lrb[j]]): members of B, label-checked when LABELED.
 template <bool LABELED, int MODE>
-__device__ __forceinline__ unsigned leaf_walk(const MatchArgs& a, const WarpState& S, const LeafSet& m, int lenB,
-                                              uint32_t mask, int t, int tend) {
+__device__ __forceinline__ unsigned leaf_walk(const MatchArgs& a, const WarpState& S, const LeafSet& m,
+                                              const int32_t* lists, uint32_t mask, int t, int tend) {
   unsigned k = 0;
   auto test = [&](int x) {
-    bool hit = leaf_member<MODE>(m, lenB, x);
+    bool hit = leaf_member<MODE>(m, x);
     if (LABELED && hit) hit = (mask >> a.labels[x]) & 1u;
     k += hit ? 1u : 0u;
   };
@@ -827,7 +1075,7 @@ __device__ __forceinline__ unsigned leaf_walk(const MatchArgs& a, const WarpStat
   while (t < tend) {
     const int jbeg = S.lexcl[j];
     const int stop = min(tend, S.lexcl[j + 1]);
-    const int32_t* src = a.colidx + S.lrb[j] + (unsigned long long)(t - jbeg);
+    const int32_t* src = lists + S.lrb[j] + (unsigned long long)(t - jbeg);
     const int n = stop - t;
     // scalar up to a 16-byte boundary, then 128-bit loads, four in flight (two, one at the tail)
     int q = min(n, (int)((4 - ((reinterpret_cast<uintptr_t>(src) >> 2) & 3)) & 3));
@@ -858,32 +1106,55 @@ __device__ __forceinline__ unsigned leaf_walk(const MatchArgs& a, const WarpStat
   return k;
 }
 
-// The last-level intersections of candidates [b, e) with the common operand B
-// (|B| <= PM_SB_MAX), work-balanced across the warp: the first operands of 32
-// candidates (each cut at its symmetry-breaking bound) are laid end to end
-// and split into 32 contiguous parts, one per lane.  A lane finds the
-// candidate owning its part's start once and walks on through the following
-// lists, four 128-bit loads in flight, testing each element against B's structure in
-// shared memory (leaf_build).  Counts only; no truncation.  Same set
-// operations, counts and accounting as lane_intersect per candidate.
+// A candidate that is a path vertex left standing in its slot (WarpState::raw
+// above size): skipped.
+__device__ __forceinline__ bool on_path(const WarpState& S, int L, int v) {
+  bool on = false;
+  for (int j = 0; j <= L; j++) on = on || S.path[j] == v;
+  return on;
+}
+
+// The last-level intersections of candidates [b, e) with the common operand
+// B, work-balanced across the warp: the first operands of 32 candidates (each
+// cut at its symmetry-breaking bound, or one label's part of the list when
+// `group` >= 0) are laid end to end and split into 32 contiguous parts, one
+// per lane.  A lane finds the candidate owning its part's start once and
+// walks on through the following lists, four 128-bit loads in flight, testing
+// each element against B's structure in shared memory (leaf_build).  Counts
+// only.  Truncation needs no care here: B is a slot, at most T long already.
+// Same set operations, counts and accounting as lane_intersect per candidate.
 // Batches averaging under 16 elements per lane, and a.leaf_flat == 2, use
 // the strided layout instead (element t0 + lane, owner found per element by
-// shuffles): it has no per-lane setup per candidate.
+// shuffles): it has no per-lane setup per candidate.  Returns false, having
+// done nothing, when B is too long for a structure.
 template <bool LABELED>
-__device__ unsigned long long leaf_flat(const MatchArgs& a, WarpState& S, const int32_t* cand, int b, int e,
-                                        const int32_t* B, int lenB, uint32_t mask, int common_ub, bool self_ub,
-                                        Work& w) {
+__device__ bool leaf_flat(const MatchArgs& a, WarpState& S, int L, bool holes, const int32_t* cand, int b, int e,
+                          const int32_t* B, int lenB, unsigned long long idB, uint32_t mask, int group,
+                          int common_ub, bool self_ub, Work& w, unsigned long long* total_cnt) {
   const int lane = lane_id();
   LeafSet m;
-  const int mode = leaf_build(S, B, lenB, m);
+  const int mode = leaf_build(S, B, lenB, idB, m);
+  if (mode == MEMB_NONE) return false;
+  const int32_t* lists = LABELED && group >= 0 ? a.colidx_lab : a.colidx;
+  const bool check = LABELED && group < 0;
   unsigned long long cnt = 0, bytes = 0, ops = 0;  // per lane
   for (int base = b; base < e; base += 32) {
     const int i = base + lane;
-    const bool mine = i < e;
+    const int c = i < e ? cand[i] : 0;
+    const bool mine = i < e && !(holes && on_path(S, L, c));
     int lenA = 0;
     unsigned long long rb = 0;
-    if (mine) {
-      const int c = cand[i];
+    if (LABELED && group >= 0) {
+      if (mine) {
+        rb = a.rowptr[c];
+        const int deg = (int)(a.rowptr[c + 1] - rb);
+        const int2 gr = label_range(a, c, group);
+        rb += (unsigned long long)gr.x;
+        lenA = gr.y;
+        bytes += 4ull * (unsigned long long)(deg + lenB) + (unsigned long long)deg;
+        ops++;
+      }
+    } else if (mine) {
       rb = a.rowptr[c];
       const int deg = (int)(a.rowptr[c + 1] - rb);
       const int ub = self_ub ? min(common_ub, c) : common_ub;
@@ -911,12 +1182,9 @@ __device__ unsigned long long leaf_flat(const MatchArgs& a, WarpState& S, const 
         }
         const unsigned long long rbj = __shfl_sync(FULL, rb, j);
         if (t < total) {
-          const int x = a.colidx[rbj + (unsigned long long)(t - ej)];
-          bool hit = mode == MEMB_BITMAP   ? leaf_member<MEMB_BITMAP>(m, lenB, x)
-                     : mode == MEMB_FILTER ? leaf_member<MEMB_FILTER>(m, lenB, x)
-                     : mode == MEMB_HASH   ? leaf_member<MEMB_HASH>(m, lenB, x)
-                                           : leaf_member<MEMB_SORTED>(m, lenB, x);
-          if (LABELED && hit) hit = (mask >> a.labels[x]) & 1u;
+          const int x = lists[rbj + (unsigned long long)(t - ej)];
+          bool hit = mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(m, x) : leaf_member<MEMB_FILTER>(m, x);
+          if (check && hit) hit = (mask >> a.labels[x]) & 1u;
           cnt += hit ? 1u : 0u;
         }
       }
@@ -930,10 +1198,13 @@ __device__ unsigned long long leaf_flat(const MatchArgs& a, WarpState& S, const 
     const int t = min(total, lane * chunk);
     const int tend = min(total, t + chunk);
     unsigned k;
-    if (mode == MEMB_BITMAP) k = leaf_walk<LABELED, MEMB_BITMAP>(a, S, m, lenB, mask, t, tend);
-    else if (mode == MEMB_FILTER) k = leaf_walk<LABELED, MEMB_FILTER>(a, S, m, lenB, mask, t, tend);
-    else if (mode == MEMB_HASH) k = leaf_walk<LABELED, MEMB_HASH>(a, S, m, lenB, mask, t, tend);
-    else k = leaf_walk<LABELED, MEMB_SORTED>(a, S, m, lenB, mask, t, tend);
+    if (LABELED && check) {
+      if (mode == MEMB_BITMAP) k = leaf_walk<true, MEMB_BITMAP>(a, S, m, lists, mask, t, tend);
+      else k = leaf_walk<true, MEMB_FILTER>(a, S, m, lists, mask, t, tend);
+    } else {
+      if (mode == MEMB_BITMAP) k = leaf_walk<false, MEMB_BITMAP>(a, S, m, lists, mask, t, tend);
+      else k = leaf_walk<false, MEMB_FILTER>(a, S, m, lists, mask, t, tend);
+    }
     cnt += k;
     __syncwarp();
   }
@@ -945,7 +1216,8 @@ __device__ unsigned long long leaf_flat(const MatchArgs& a, WarpState& S, const 
   }
   w.setops += ops;
   w.bytes += bytes;
-  return cnt;
+  *total_cnt = cnt;
+  return true;
 }
 
 // The last level for the candidates [b, e) of level L's main slot (each is
@@ -962,14 +1234,14 @@ __device__ unsigned long long leaf_flat(const MatchArgs& a, WarpState& S, const 
 template <bool LABELED, bool PAGED>
 __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b, int e,
                                          Work& w) {
-  const int32_t* arena = S.arena;
   const int lane = lane_id();
   const int s = P.last_slot;
   const int kind = P.kind[s];
   const int Lf = L + 1;
-  const int32_t* cand = arena + S.off[P.level_begin[L]];
+  const int32_t* cand = S.ptr[P.level_begin[L]];
+  const bool holes = !LABELED && S.raw[P.level_begin[L]] != S.size[P.level_begin[L]];
   const int par = P.parent[s];
-  const int32_t* B = arena + S.off[par];  // intersect: second operand; copy: first operand
+  const int32_t* B = S.ptr[par];  // intersect: second operand; copy: first operand
   const int lenB = S.size[par];
   const uint32_t mask = P.slot_labels[s];
   const int T = a.T;
@@ -992,9 +1264,13 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
       if (P.partial[s] & (1u << j)) common_ub = min(common_ub, S.path[j]);
     self_ub = (P.partial[s] >> Lf) & 1u;
   }
-  if (!PAGED && kind == SLOT_INTERSECT && T == 0 && lenB <= PM_SB_MAX && a.leaf_flat &&
-      !(LABELED && a.lab_off && __popc(mask) == 1))
-    return leaf_flat<LABELED>(a, S, cand, b, e, B, lenB, mask, common_ub, self_ub, w);
+  if (!PAGED && kind == SLOT_INTERSECT && a.leaf_flat) {
+    const int group = (LABELED && a.lab_off && __popc(mask) == 1) ? __ffs(mask) - 1 : -1;
+    unsigned long long k;
+    if (leaf_flat<LABELED>(a, S, L, holes, cand, b, e, B, lenB, S.id[par], mask, group, common_ub, self_ub, w, &k))
+      return k;
+  }
+  const unsigned adjacent = !PAGED && symmetric(a) ? P.leaf_adj : 0u;  // path vertices in every candidate's list
   const int32_t* Bs = B;
   if (kind == SLOT_INTERSECT && lenB <= PM_SB_MAX && lenB > 0) {
     Bs = stage_bulk(S, B, lenB);
@@ -1004,8 +1280,8 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
   PageCounters lpc = {};                           // per lane (paged residency)
   for (int base = b; base < e; base += 32) {
     const int i = base + lane;
-    const bool mine = i < e;
-    const int c = mine ? cand[i] : 0;
+    const int c = i < e ? cand[i] : 0;
+    const bool mine = i < e && !(holes && on_path(S, L, c));
     bool deferred = false;
     int32_t want = -1;  // an absent page this lane read around, for the warp to load
     if (mine) {
@@ -1124,9 +1400,15 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
         } else if (!LABELED && kind == SLOT_FRESH) {
           // first min(lenA, T) elements, minus the path vertices among them
           const int lim = (T && lenA > T) ? T : lenA;
+          // (a path vertex below the bound that the plan made the candidate's
+          // neighbour needs no search)
           int k = lim;
           for (int j = 0; j <= L; j++) {
             const int pj = S.path[j];
+            if (lim == lenA && ((adjacent >> j) & 1u)) {
+              k -= pj < ub ? 1 : 0;
+              continue;
+            }
             const int pos = lane_lower_bound<PAGED>(A, lim, pj, cgl);
             k -= (pos < lim && ld<PAGED>(A + pos, cgl) == pj) ? 1 : 0;
           }
@@ -1173,8 +1455,12 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
       const int cc = __shfl_sync(FULL, c, src);
       if (lane == 0) S.path[Lf] = cc;
       __syncwarp();
-      cnt_warp += (unsigned long long)run_slot<LABELED, PAGED>(a, P, S, Lf, s, S.top[Lf], true, w);
+      Work t;
+      memset(&t, 0, sizeof(t));
+      cnt_warp += (unsigned long long)count_slot<LABELED, PAGED>(a, P, S, Lf, s, S.top[Lf], &t);
+      add_work(w, t);
     }
+    if (Bs != B && S.sb_id != 0) Bs = stage_bulk(S, B, lenB);  // run_slot built its own structure there
     if (PAGED) {
       // pages the lanes read around: the warp loads up to two of them per
       // 32 candidates (one page copy each), so later reads hit
@@ -1224,13 +1510,14 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
   const int X = P.l2_x, Y = P.l2_y, M = P.level_begin[Lq], last = P.last_slot;
   const int p1 = P.parent[X];
   const int lenB1 = S.size[p1];
-  const int32_t* B1 = arena + S.off[p1];
+  const int32_t* B1 = S.ptr[p1];
   const int32_t* Bs = lenB1 > 0 ? stage_bulk(S, B1, lenB1) : B1;
   if (lenB1 > 0 && Bs == B1) w.err |= DEV_TIMEOUT;
-  const int32_t* cand = arena + S.off[P.level_begin[L]];
+  const int32_t* cand = S.ptr[P.level_begin[L]];
+  const bool holes = S.raw[P.level_begin[L]] != S.size[P.level_begin[L]];
   unsigned long long cnt = 0, bytes = 0, ops = 0;
   const int i = b + lane;
-  if (i < e) {
+  if (i < e && !(holes && on_path(S, L, cand[i]))) {
     const int v = cand[i];
     // slot bounds with path[Lq] = v: main slots take the smallest constrained
     // path vertex, helpers the largest (slot_bound)
@@ -1301,6 +1588,784 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
     cnt += __shfl_xor_sync(FULL, cnt, o);
     bytes += __shfl_xor_sync(FULL, bytes, o);
     ops += __shfl_xor_sync(FULL, ops, o);
+  }
+  w.setops += ops;
+  w.bytes += bytes;
+  return cnt;
+}
+
+// The rest of a clique search below one node of level L, in bit sets: the
+// helper slot of level L (the common neighbours of the path, m of them) is
+// numbered, row i of a bit matrix in the arena holds which of them are
+// neighbours of number i, and every deeper candidate set is an AND of rows --
+// the main set of a candidate is the part of its row below itself, the last
+// level is a popcount.  A set operation of the reference's search costs a few
+// words instead of a walk over an adjacency list; its operands' lengths are
+// known from the rows, two positions per list (len_m: elements below the
+// candidate, len_h: elements below the largest path vertex) and the sets'
+// sizes, so the accounting is the same.
+// Bound: the rows, m^2 / 32 words looked up in the m lists (four searches per
+// lane in flight), then L1-resident words.  Measured (B200), 5-clique on an
+// R-MAT graph of 32,768 vertices and 524,288 edges: 524 ms with one
+// candidate per lane walking its list (lane_subtree), 35 ms so.
+#define PM_CLIQUE_MAX 1024  // most common neighbours: 32 words per row, one per lane
+
+__device__ __forceinline__ int64_t clique_words(int m) {
+  int wd = 1;
+  while (wd * 32 < m) wd <<= 1;
+  return 32 + (int64_t)m * (wd + 2);
+}
+
+// Bits below number j in word k of a set.
+__device__ __forceinline__ unsigned bits_below(int j, int k) {
+  const int d = j - 32 * k;
+  return d >= 32 ? 0xffffffffu : d <= 0 ? 0u : (1u << d) - 1u;
+}
+
+// Rows [0, rows) of the matrix (stride wd words, a power of two) and the two
+// lengths of each.  A vertex with a bit row of its own (pm_graph::d_hub_bits)
+// answers "is x a neighbour" with one load, 32 numbers a word, eight rows in
+// flight; the other lists are short and are scanned -- read in coalesced
+// tiles, each element tested against the set's structure in shared memory,
+// the few that pass queued and looked up in the set 32 at a time -- or, when
+// still much longer than the set, searched for each of its numbers.
+// Measured on the 5-clique case above, cycles of all warps in this function:
+// searching every row 2.1e11, scanning (hub lists of thousands) 2.1e11, both
+// bound by instructions; with bit rows 5.0e10.
+#define PM_CLIQUE_SEARCH 448  // list elements per word of the set from which a row is searched
+
+__device__ __noinline__ void clique_rows(const MatchArgs& a, WarpState& S, const int32_t* nb, int m, int wd, int rows,
+                                         int ub_h, unsigned long long id, unsigned* R, int32_t* len_m,
+                                         int32_t* len_h) {
+  const int lane = lane_id();
+  const int nw = (m + 31) >> 5;
+  int lw = 0;
+  while ((1 << lw) < wd) lw++;
+  int32_t* queue = (int32_t*)S.lrb;       // 64 words
+  unsigned* row_bits = (unsigned*)S.lexcl;  // 32 words
+  LeafSet set;
+  int mode = MEMB_NONE;  // built when the first row is scanned
+  for (int r0 = 0; r0 < rows; r0 += 32) {
+    int deg = 0, lh = 0;
+    unsigned long long rb = 0;
+    if (r0 + lane < rows) {
+      const int v = nb[r0 + lane];
+      rb = a.rowptr[v];
+      deg = (int)(a.rowptr[v + 1] - rb);
+      lh = lane_lower_bound(a.colidx + rb, deg, ub_h);
+      len_m[r0 + lane] = lane_lower_bound(a.colidx + rb, deg, v);
+      len_h[r0 + lane] = lh;
+    }
+    const int slot = a.hub_slot && r0 + lane < rows ? a.hub_slot[nb[r0 + lane]] : -1;
+    const unsigned hubs = __ballot_sync(FULL, slot >= 0);
+    if (hubs) {
+      const unsigned* bits = a.hub_bits + (long long)max(slot, 0) * a.hub_words;
+      for (int k = 0; k < wd; k++) {
+        const int x = 32 * k + lane < m ? nb[32 * k + lane] : -1;
+        const int at = max(x, 0) >> 5, sh = x & 31;
+        for (int r = 0; r < 32; r += 8) {
+          if (!((hubs >> r) & 255u)) continue;
+          unsigned got[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const unsigned* row = (const unsigned*)__shfl_sync(FULL, (unsigned long long)bits, r + q);
+            got[q] = x >= 0 && ((hubs >> (r + q)) & 1u) ? (__ldg(row + at) >> sh) & 1u : 0u;
+          }
+          unsigned mine = 0;
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const unsigned word = __ballot_sync(FULL, got[q]);
+            if (lane == r + q) mine = word;
+          }
+          if (lane >= r && lane < r + 8 && ((hubs >> lane) & 1u)) R[(r0 + lane) * wd + k] = mine;
+        }
+      }
+    }
+    unsigned todo = __ballot_sync(FULL, lh > PM_CLIQUE_SEARCH * nw) & ~hubs;
+    const unsigned scans = __ballot_sync(FULL, r0 + lane < rows) & ~todo & ~hubs;
+    // searched rows: 8 / wd rows a step, or eight words of one row
+    const int per = wd < 8 ? 8 >> lw : 1;
+    while (todo) {
+      int src[8];
+      unsigned left = todo;
+#pragma unroll
+      for (int q = 0; q < 8; q++) src[q] = -1;
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        if (k >= per || !left) continue;
+        const int r = __ffs(left) - 1;
+        left &= left - 1;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if ((wd < 8 ? q >> lw : 0) == k) src[q] = r;
+      }
+      todo = left;
+      for (int k0 = 0; k0 < wd; k0 += 8) {
+        const int32_t* A[8];
+        int n[8], x[8], most = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const int k = wd < 8 ? q & (wd - 1) : k0 + q;
+          A[q] = a.colidx + __shfl_sync(FULL, rb, src[q] & 31);
+          n[q] = src[q] >= 0 ? __shfl_sync(FULL, lh, src[q] & 31) : 0;
+          most = max(most, n[q]);
+          x[q] = n[q] > 0 && 32 * k + lane < m ? nb[32 * k + lane] : -1;
+          if (n[q] == 0) A[q] = nb;  // something readable
+        }
+        while (most > 1) {
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const int h = n[q] >> 1;
+            if (A[q][h] <= x[q]) A[q] += h;
+            n[q] -= h;
+          }
+          most -= most >> 1;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const unsigned word = __ballot_sync(FULL, x[q] >= 0 && *A[q] == x[q]);
+          const int k = wd < 8 ? q & (wd - 1) : k0 + q;
+          if (lane == 0 && src[q] >= 0 && k < wd) R[(r0 + src[q]) * wd + k] = word;
+        }
+      }
+    }
+    if (scans && mode == MEMB_NONE) mode = leaf_build(S, nb, m, id, set);
+    for (unsigned left = scans; left; left &= left - 1) {
+      const int r = __ffs(left) - 1;
+      const int32_t* A = a.colidx + __shfl_sync(FULL, rb, r);
+      const int len = __shfl_sync(FULL, lh, r);
+      int queued = 0;
+      row_bits[lane] = 0u;
+      __syncwarp();
+      auto place = [&](int count) {  // the queue's first `count` (at most 32)
+        const int x = lane < count ? queue[lane] : -1;
+        int at = 0;
+        for (int n = m; n > 1;) {
+          const int h = n >> 1;
+          if (nb[at + h] <= x) at += h;
+          n -= h;
+        }
+        if (x >= 0 && nb[at] == x) atomicOr(&row_bits[at >> 5], 1u << (at & 31));
+      };
+      for (int base = 0; base < len; base += 128) {
+        int x[4];
+        bool in[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int i = base + 32 * q + lane;
+          in[q] = i < len;
+          x[q] = in[q] ? A[i] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          in[q] = in[q] && (mode == MEMB_BITMAP ? leaf_maybe<MEMB_BITMAP>(set, x[q]) : leaf_maybe<MEMB_FILTER>(set, x[q]));
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const unsigned bal = __ballot_sync(FULL, in[q]);
+          if (in[q]) queue[queued + __popc(bal & lanemask_lt())] = x[q];
+          queued += __popc(bal);
+          __syncwarp();
+          if (queued >= 32) {
+            place(32);
+            __syncwarp();
+            const int rest = lane < queued - 32 ? queue[32 + lane] : 0;
+            __syncwarp();
+            queued -= 32;
+            if (lane < queued) queue[lane] = rest;
+            __syncwarp();
+          }
+        }
+      }
+      if (queued) place(queued);
+      __syncwarp();
+      if (lane < wd) R[(r0 + r) * wd + lane] = row_bits[lane];
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+}
+
+// Candidates [b, e) of level L's main slot (the first numbers of the helper
+// slot's): matches below them.
+__device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
+                                                       int e, unsigned long long* ops_out,
+                                                       unsigned long long* bytes_out) {
+  const int lane = lane_id();
+  const int hs = P.level_begin[L] + 1;
+  const int32_t* nb = S.ptr[hs];
+  const int m = S.size[hs];
+  int wd = 1;
+  while (wd * 32 < m) wd <<= 1;
+  unsigned* R = (unsigned*)(S.arena + ((S.top[L + 1] + 31) & ~31));
+  int32_t* len_m = (int32_t*)(R + m * wd);
+  int32_t* len_h = len_m + m;
+  if (S.cq_id != S.id[hs] || S.cq_rows != R || S.cq_n < e) {
+    int ub_h = 0;
+    for (int j = 0; j <= L; j++) ub_h = max(ub_h, S.path[j]);
+    const int rows = S.iend[L];
+    __syncwarp();
+    clique_rows(a, S, nb, m, wd, rows, ub_h, S.id[hs], R, len_m, len_h);
+    if (lane == 0) {
+      S.cq_id = S.id[hs];
+      S.cq_rows = R;
+      S.cq_n = rows;
+      S.sb_id = 0;
+    }
+    __syncwarp();
+  }
+  const int depth = P.nnodes - 4 - L;  // levels between the candidates' and the last
+  unsigned long long cnt = 0, ops = 0, bytes = 0;  // per lane
+  if (m <= 32) {
+    // one candidate per lane, every set one word
+    unsigned* rs = (unsigned*)S.sb;
+    int32_t* lm = S.sb + 32;
+    int32_t* lh = S.sb + 64;
+    if (lane == 0) S.sb_id = 0;
+    for (int i = lane; i < e; i += 32) {
+      rs[i] = R[i];
+      lm[i] = len_m[i];
+      lh[i] = len_h[i];
+    }
+    __syncwarp();
+    const int i = b + lane;
+    if (i < e) {
+      unsigned H[3], M[3];
+      int d = 0;
+      H[0] = rs[i];
+      M[0] = H[0] & bits_below(i, 0);
+      auto node = [&](int v, int size_up, unsigned h, unsigned mm) {  // the two set operations of a level
+        const int nh = __popc(h), nm = __popc(mm);
+        ops += 2;
+        bytes += 4ull * (unsigned long long)(lm[v] + lh[v] + 2 * size_up + nh + nm);
+      };
+      node(i, m, H[0], M[0]);
+      while (d >= 0) {
+        // (depth at most 2: selects instead of indexed registers)
+        const unsigned h = d == 0 ? H[0] : d == 1 ? H[1] : H[2];
+        unsigned mm = d == 0 ? M[0] : d == 1 ? M[1] : M[2];
+        if (d == depth) {
+          const int nh = __popc(h);
+          while (mm) {
+            const int j = __ffs(mm) - 1;
+            mm &= mm - 1;
+            const int k = __popc(rs[j] & h & bits_below(j, 0));
+            cnt += k;
+            ops++;
+            bytes += 4ull * (unsigned long long)(lm[j] + nh + k);
+          }
+          d--;
+          continue;
+        }
+        if (!mm) {
+          d--;
+          continue;
+        }
+        const int j = __ffs(mm) - 1;
+        mm &= mm - 1;
+        if (d == 0) M[0] = mm; else M[1] = mm;
+        const unsigned h2 = h & rs[j], m2 = h2 & bits_below(j, 0);
+        node(j, __popc(h), h2, m2);
+        d++;
+        if (d == 1) { H[1] = h2; M[1] = m2; } else { H[2] = h2; M[2] = m2; }
+      }
+    }
+    __syncwarp();
+  } else {
+    // one candidate at a time, word `lane` of every set in lane `lane`; the
+    // last level takes 32 / wd candidates a step, wd lanes each
+    unsigned short* lst = (unsigned short*)S.sb;
+    if (lane == 0) S.sb_id = 0;
+    const int grp = lane / wd, gw = lane & (wd - 1), groups = 32 / wd;
+    for (int i = b; i < e; i++) {
+      unsigned H[3], M[3];
+      int size[3];
+      int d = 0, v = i;
+      unsigned up = lane < ((m + 31) >> 5) ? 0xffffffffu : 0u;  // level L's helper set (all numbers)
+      int size_up = m;
+      bool fresh = true;  // v was chosen: its sets are to be computed at depth d
+      while (d >= 0) {
+        if (fresh) {
+          const unsigned row = lane < wd ? R[v * wd + lane] : 0u;
+          const unsigned h = row & up, mm = h & bits_below(v, lane);
+          const int nh = __reduce_add_sync(FULL, __popc(h)), nm = __reduce_add_sync(FULL, __popc(mm));
+          if (d == 0) { H[0] = h; M[0] = mm; size[0] = nh; }
+          else if (d == 1) { H[1] = h; M[1] = mm; size[1] = nh; }
+          else { H[2] = h; M[2] = mm; size[2] = nh; }
+          if (lane == 0) {
+            ops += 2;
+            bytes += 4ull * (unsigned long long)(len_m[v] + len_h[v] + 2 * size_up + nh + nm);
+          }
+          fresh = false;
+        }
+        const unsigned h = d == 0 ? H[0] : d == 1 ? H[1] : H[2];
+        const unsigned mm = d == 0 ? M[0] : d == 1 ? M[1] : M[2];
+        const int nh = d == 0 ? size[0] : d == 1 ? size[1] : size[2];
+        if (d == depth) {
+          // the main set's numbers, listed in shared memory
+          int incl = __popc(mm);
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+          }
+          const int total = __shfl_sync(FULL, incl, 31);
+          __syncwarp();
+          {
+            int at = incl - __popc(mm);
+            unsigned left = mm;
+            while (left) {
+              lst[at++] = (unsigned short)(32 * lane + __ffs(left) - 1);
+              left &= left - 1;
+            }
+          }
+          __syncwarp();
+          const unsigned hw = __shfl_sync(FULL, h, gw);
+          unsigned k = 0;
+          for (int t = grp; t < total; t += 4 * groups) {
+            unsigned r4[4];
+            int j4[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const bool on = t + q * groups < total;
+              j4[q] = on ? lst[t + q * groups] : 0;
+              r4[q] = on ? R[j4[q] * wd + gw] : 0u;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) k += __popc(r4[q] & hw & bits_below(j4[q], gw));
+          }
+          cnt += k;
+          bytes += 4ull * k;
+          for (int t = lane; t < total; t += 32) bytes += 4ull * (unsigned long long)(len_m[lst[t]] + nh);
+          if (lane == 0) ops += (unsigned long long)total;
+          __syncwarp();
+          d--;
+        } else {
+          const unsigned any = __ballot_sync(FULL, mm != 0u);
+          if (!any) {
+            d--;
+          } else {
+            const int src = __ffs(any) - 1;
+            const int bit = __ffs(__shfl_sync(FULL, mm, src)) - 1;
+            v = 32 * src + bit;
+            const unsigned left = lane == src ? mm & (mm - 1) : mm;
+            if (d == 0) M[0] = left; else M[1] = left;
+            up = h;
+            size_up = nh;
+            d++;
+            fresh = true;
+          }
+        }
+        // back at a shallower level: its own helper set is `up` again when
+        // the next candidate there is entered (set above)
+      }
+    }
+  }
+  for (int o = 16; o; o >>= 1) {
+    cnt += __shfl_xor_sync(FULL, cnt, o);
+    bytes += __shfl_xor_sync(FULL, bytes, o);
+    ops += __shfl_xor_sync(FULL, ops, o);
+  }
+  *ops_out = ops;
+  *bytes_out = bytes;
+  return cnt;
+}
+
+// ---------------------------------------------------------------------
+// The last two levels in one pass.  Level q = n-3's main slot is a list of
+// each candidate v for path[q] (N(v), or its part in a parent slot), and the
+// last level adds a value f(x) for every element x of it:
+//   PAIR_COPY   the last slot is a copy of a set h of level q (itself a copy
+//               of h0, a slot of level q-1): |h|, less one if x is in h;
+//   PAIR_FRESH  x's own list: its length (below a bound of the path), less
+//               the path vertices in it;
+//   PAIR_MEET   x's list intersected with h: |N(x) n h0|, less one when v is
+//               in h0 (v is a neighbour of x).  The value depends on x and h0
+//               only, and the same x is met under many v: each warp keeps the
+//               values in a table of its own in device memory (MemoEntry),
+//               tagged with the number of the (h0, bound) they belong to.
+// So no slot of level q is built, and no call is made per candidate of level
+// q: elements come in tiles of 32 (one list each), four tiles in flight.
+// Set operations, counts and accounting are those of run_level + leaf_batch.
+//
+// What bounded the search before was instructions, not bytes: about 1,400 per
+// candidate of level q for two slots and a batch whose lists have a few tens
+// of elements (house on 3,000 vertices: 2.3 million candidates, 3.2e9 warp
+// instructions, 7.4 ms), and for cycles the walk over every list again under
+// every v.  Measured (B200), launch before and after: house on 3,000 vertices
+// 6.5 -> 1.7 ms; one of 64 shards of the 6-cycle on Chung-Lu 20,000 / 100,000
+// 372 -> 68 ms; labeled on R-MAT, the 5-cycle (8 labels, 32,768 vertices, sets
+// capped at 4,096) 37 -> 5.3 ms, the 5-cycle with a tail (32 labels, 131,072
+// vertices) 18 -> 12.6 ms, paged 47 -> 27 ms.
+// ---------------------------------------------------------------------
+// Counters of one pass (per lane).
+struct PairSums {
+  unsigned long long cnt, bytes, elems;
+};
+
+// Queued elements whose PAIR_MEET value is not in the table: the first
+// `count` (at most 32) of S.queue.  Their lists, cut at the bound or to one
+// label's part, are laid end to end and walked in equal parts, a part at a
+// time per lane, matches added to the owner's counter in shared memory.
+template <bool LABELED>
+__device__ __forceinline__ void meet_values(const MatchArgs& a, WarpState& S, const LeafSet& m, int mode, int group,
+                                            int ub, int count, PairSums& r) {
+  const int lane = lane_id();
+  const int32_t* lists = LABELED ? a.colidx_lab : a.colidx;
+  int lenA = 0, scan_len = 0, x = -1;
+  unsigned long long rb = 0;
+  if (lane < count) {
+    x = S.queue[lane];
+    rb = a.rowptr[x];
+    const int deg = (int)(a.rowptr[x + 1] - rb);
+    if (LABELED) {
+      const int2 gr = label_range(a, x, group);
+      rb += (unsigned long long)gr.x;
+      lenA = gr.y;
+      scan_len = deg;
+    } else {
+      lenA = ub == INT_MAX ? deg : lane_lower_bound(a.colidx + rb, deg, ub);
+      scan_len = lenA;
+    }
+  }
+  int incl = lenA;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const int total = __shfl_sync(FULL, incl, 31);
+  S.lrb[lane] = rb;
+  S.lexcl[lane] = incl - lenA;
+  if (lane == 31) S.lexcl[32] = total;
+  S.lcnt[lane] = 0;
+  __syncwarp();
+  for (int t0 = 0; t0 < total; t0 += 128) {
+    int y[4], own[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int t = t0 + 32 * q + lane;
+      int j = 0;
+#pragma unroll
+      for (int step = 16; step; step >>= 1)
+        if (S.lexcl[j + step] <= t) j += step;
+      own[q] = j;
+      y[q] = t < total ? __ldg(lists + S.lrb[j] + (unsigned long long)(t - S.lexcl[j])) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool hit = y[q] >= 0 && (mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(m, y[q])
+                                                          : leaf_member<MEMB_FILTER>(m, y[q]));
+      if (hit) atomicAdd(&S.lcnt[own[q]], 1);
+    }
+  }
+  __syncwarp();
+  if (lane < count) {
+    const int k = S.lcnt[lane];
+    r.cnt += (unsigned long long)k;
+    r.bytes += 4ull * (unsigned long long)(scan_len + k) + (LABELED ? (unsigned long long)scan_len : 0ull);
+  }
+  // one lane per table entry stores
+  const int at = x & (a.memo_entries - 1);
+  const unsigned same = __match_any_sync(FULL, lane < count ? at : -1 - lane);
+  if (lane < count && (same & lanemask_lt()) == 0)
+    *reinterpret_cast<int4*>(S.memo + at) = make_int4(x, (int)S.memo_epoch, S.lcnt[lane], scan_len);
+  __syncwarp();
+}
+
+// True when this node's last two levels can be taken in one pass.
+template <bool LABELED, bool PAGED>
+__device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, const WarpState& S) {
+  // (truncated: an unlabeled list's first T elements less the path vertices
+  // among them is not its length less them)
+  if (!P.pair || !a.pairs || (!LABELED && a.T && P.pair == PAIR_FRESH) || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
+  if (P.pair == PAIR_MEET) {
+    if (PAGED || !a.memo) return false;
+    const int n0 = S.size[P.pair_h0];
+    return n0 <= PM_FILTER_MAX || (n0 > 0 && S.ptr[P.pair_h0][n0 - 1] < 32 * PM_SB_MAX);
+  }
+  if (P.kind[P.level_begin[P.nnodes - 3]] == SLOT_INTERSECT) {
+    const int par = P.parent[P.level_begin[P.nnodes - 3]], n0 = S.size[par];
+    return (n0 <= PM_FILTER_MAX || (n0 > 0 && S.ptr[par][n0 - 1] < 32 * PM_SB_MAX));
+  }
+  return true;
+}
+
+// Candidates [b, e) (at most 32) of level L = n-4's main slot.
+template <bool LABELED, bool PAGED>
+__device__ __noinline__ unsigned long long pair_levels(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
+                                                       int e, Work* wt) {
+  Work& w = *wt;
+  const int lane = lane_id();
+  const int q = L + 1;
+  const int ms = P.level_begin[q], last = P.last_slot;
+  const int kind = P.pair;
+  const bool meet_main = P.kind[ms] == SLOT_INTERSECT;
+  const int main_group = LABELED ? __ffs(P.slot_labels[ms]) - 1 : -1;
+  const int last_group = LABELED ? __ffs(P.slot_labels[last]) - 1 : -1;
+  // the parent a main intersection meets, and the set a copy or a meeting reads
+  LeafSet set;
+  int mode = MEMB_NONE;
+  int lenBm = 0;
+  if (meet_main) {
+    const int par = P.parent[ms];
+    lenBm = S.size[par];
+    mode = leaf_build(S, S.ptr[par], lenBm, S.id[par], set);
+  }
+  const int h0 = P.pair_h0;
+  const int32_t* H0 = kind != PAIR_FRESH ? S.ptr[h0] : nullptr;
+  const int len0 = kind != PAIR_FRESH ? S.size[h0] : 0;
+  // the last slot's bound (a main slot: the smallest constrained path vertex; up to L only in these plans)
+  int ub_last = INT_MAX;
+  if (!LABELED)
+    for (int j = 0; j <= L; j++)
+      if ((P.partial[last] >> j) & 1u) ub_last = min(ub_last, S.path[j]);
+  int len_h = len0;  // h0 below h's bound (a helper slot: the largest constrained path vertex)
+  if (kind == PAIR_MEET) {
+    const int ub_h = slot_bound<LABELED>(P, S, L, P.parent[last]);
+    if (!LABELED && ub_h != INT_MAX) len_h = warp_lower_bound<false>(H0, len0, ub_h);
+    mode = leaf_build(S, H0, len_h, S.id[h0], set);
+    if (S.memo_id != S.id[h0] || S.memo_len != len_h || S.memo_ub != ub_last) {
+      __syncwarp();
+      if (S.memo_epoch == 0xffffffffu) {  // numbers used up: forget everything
+        for (int i = lane; i < a.memo_entries; i += 32) *reinterpret_cast<int4*>(S.memo + i) = make_int4(0, 0, 0, 0);
+        __syncwarp();
+        if (lane == 0) S.memo_epoch = 0;
+        __syncwarp();
+      }
+      if (lane == 0) {
+        S.memo_id = S.id[h0];
+        S.memo_len = len_h;
+        S.memo_ub = ub_last;
+        S.memo_epoch++;
+      }
+      __syncwarp();
+    }
+  }
+  const unsigned epoch = S.memo_epoch;
+  // the candidates, one per lane
+  const int32_t* cand = S.ptr[P.level_begin[L]];
+  const bool holes = !LABELED && S.raw[P.level_begin[L]] != S.size[P.level_begin[L]];
+  const int v = b + lane < e ? cand[b + lane] : -1;
+  const bool mine = v >= 0 && !(holes && on_path(S, L, v));
+  unsigned long long rb = 0;
+  int len = 0;     // elements of v's list to look at
+  int h_v = 0;     // |h| under v (a copy's or a meeting's second operand)
+  int less = 0;    // PAIR_MEET: 1 when v is in h0 below the bound
+  PairSums r = {0, 0, 0};
+  unsigned long long ops = 0;
+  if (mine) {
+    rb = a.rowptr[v];
+    const int deg = (int)(a.rowptr[v + 1] - rb);
+    int lenA = deg;
+    len = deg;
+    if (LABELED) {
+      const int2 gr = label_range(a, v, main_group);
+      rb += (unsigned long long)gr.x;
+      len = gr.y;
+    } else if (P.partial[ms]) {
+      int ub = INT_MAX;  // a main slot: the smallest constrained path vertex, v among them
+      for (int j = 0; j <= L; j++)
+        if ((P.partial[ms] >> j) & 1u) ub = min(ub, S.path[j]);
+      if ((P.partial[ms] >> q) & 1u) ub = min(ub, v);
+      if (ub != INT_MAX) lenA = len = lane_lower_bound(a.colidx + rb, deg, ub);
+    }
+    // a fresh set holds at most its first T elements; what is made of slots is
+    // no longer than they are
+    if (a.T && !meet_main) len = min(len, a.T);
+    ops = 1;
+    r.bytes += 4ull * (unsigned long long)(lenA + lenBm) + (LABELED ? (unsigned long long)lenA : 0ull);
+    if (kind != PAIR_FRESH) {
+      // h: h0 without v (labeled: h0 itself), below h's bound
+      bool in0 = false;
+      if (!LABELED) {
+        const int at = lane_lower_bound(H0, len_h, v);
+        in0 = at < len_h && H0[at] == v;
+      }
+      h_v = len_h - (in0 ? 1 : 0);
+      less = in0 && v < ub_last ? 1 : 0;
+      // the reference scans h0 below the bound for the copy
+      ops++;
+      r.bytes += 4ull * (unsigned long long)(len_h + h_v) + (LABELED ? (unsigned long long)len_h : 0ull);
+    }
+  }
+  w.reads += __popc(__ballot_sync(FULL, mine));
+  // PAIR_FRESH: path vertices whose adjacency to x has to be looked up
+  int pv[4];
+  const unsigned* prow[4];
+  int known = 0, n_ask = 0;  // neighbours of every x, below the bound
+  if (!LABELED && kind == PAIR_FRESH) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) { pv[j] = -1; prow[j] = nullptr; }
+    for (int j = 0; j <= L; j++) {
+      const int p = S.path[j];
+      if (p >= ub_last) continue;
+      if ((P.leaf_adj >> j) & 1u) known++;
+      else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (k == n_ask) { pv[k] = p; prow[k] = hub_row(a, p); }
+        n_ask++;
+      }
+    }
+  }
+  // walk: tiles of 32 elements of one list, four in flight
+  int queued = 0;
+  unsigned left = __ballot_sync(FULL, len > 0);
+  int j = left ? __ffs(left) - 1 : 0, o = 0;
+  ListRef cur{nullptr, 0, -1};  // PAGED: the current candidate's resolved list
+  while (left) {
+    const int32_t* src[4];
+    int own[4], cnt4[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      src[t] = nullptr;
+      own[t] = 0;
+      cnt4[t] = 0;
+      if (!left) continue;
+      const int n = __shfl_sync(FULL, len, j);
+      const unsigned long long base = __shfl_sync(FULL, rb, j);
+      if (PAGED) {
+        if (t > 0 && o == 0) continue;  // one list at a time: the next one after this round's reads
+        if (o == 0) {
+          if (!gather_room(a, S, S.top[q], n, w)) { left = 0; continue; }
+          cur = paged_list(a.pg, base, n, S.gather, S.pins, w.pc);
+        }
+        src[t] = cur.p + o;
+      } else {
+        src[t] = (LABELED ? a.colidx_lab : a.colidx) + base + o;
+      }
+      own[t] = j;
+      cnt4[t] = min(32, n - o);
+      o += 32;
+      if (o >= n) {
+        left &= left - 1;
+        j = left ? __ffs(left) - 1 : 0;
+        o = 0;
+      }
+    }
+    int x[4];
+    bool in[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      in[t] = lane < cnt4[t];
+      x[t] = in[t] ? ld<PAGED>(src[t] + lane, cur.cg) : 0;
+    }
+    if (PAGED && o == 0) {
+      __syncwarp();
+      unpin(a.pg, cur);
+      cur.pinned = -1;
+    }
+    if (meet_main) {
+#pragma unroll
+      for (int t = 0; t < 4; t++)
+        in[t] = in[t] && (mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(set, x[t]) : leaf_member<MEMB_FILTER>(set, x[t]));
+    } else if (!LABELED) {
+      for (int k = 0; k <= L; k++) {
+        const int p = S.path[k];
+#pragma unroll
+        for (int t = 0; t < 4; t++) in[t] = in[t] && x[t] != p;
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int vo = __shfl_sync(FULL, v, own[t]);
+        in[t] = in[t] && x[t] != vo;
+      }
+    }
+    if (kind == PAIR_COPY) {
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int h = __shfl_sync(FULL, h_v, own[t]), vo = __shfl_sync(FULL, v, own[t]);
+        if (!in[t]) continue;
+        r.elems++;
+        const int f = LABELED ? h : h - (x[t] != vo && bsearch_in<false>(H0, len0, x[t]) ? 1 : 0);
+        r.cnt += (unsigned long long)f;
+        r.bytes += 4ull * (unsigned long long)(h + f) + (LABELED ? (unsigned long long)h : 0ull);
+      }
+    } else if (kind == PAIR_FRESH) {
+      int deg[4], f[4];
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        deg[t] = f[t] = 0;
+        if (!in[t]) continue;
+        const uint64_t xb = a.rowptr[x[t]];
+        deg[t] = (int)(a.rowptr[x[t] + 1] - xb);
+        if (LABELED) {
+          f[t] = label_range(a, x[t], last_group).y;
+          if (a.T) f[t] = min(f[t], a.T);
+        }
+        else if (ub_last != INT_MAX) deg[t] = lane_lower_bound(a.colidx + xb, deg[t], ub_last);
+      }
+      if (!LABELED) {
+#pragma unroll
+        for (int t = 0; t < 4; t++) f[t] = deg[t] - known - (__shfl_sync(FULL, v, own[t]) < ub_last ? 1 : 0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (k >= n_ask) continue;
+          if (prow[k]) {
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+              if (in[t]) f[t] -= (__ldg(prow[k] + (x[t] >> 5)) >> (x[t] & 31)) & 1u;
+          } else {
+            const uint64_t pb = a.rowptr[pv[k]];
+            const int pn = (int)(a.rowptr[pv[k] + 1] - pb);
+            bool hit[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) hit[t] = in[t];
+            bsearch4<false>(a.colidx + pb, pn, x, hit, false);
+#pragma unroll
+            for (int t = 0; t < 4; t++) f[t] -= hit[t] ? 1 : 0;
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        if (!in[t]) continue;
+        r.elems++;
+        r.cnt += (unsigned long long)f[t];
+        r.bytes += 4ull * (unsigned long long)(deg[t] + f[t]) + (LABELED ? (unsigned long long)deg[t] : 0ull);
+      }
+    } else {
+      int4 en[4];
+#pragma unroll
+      for (int t = 0; t < 4; t++)
+        en[t] = in[t] ? *reinterpret_cast<const int4*>(S.memo + (x[t] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int h = __shfl_sync(FULL, h_v, own[t]), l1 = __shfl_sync(FULL, less, own[t]);
+        const bool hit = in[t] && en[t].x == x[t] && (unsigned)en[t].y == epoch;
+        if (in[t]) {  // what does not depend on the value
+          r.elems++;
+          r.cnt -= (unsigned long long)l1;
+          r.bytes += 4ull * (unsigned long long)(h - l1);
+        }
+        if (hit) {
+          r.cnt += (unsigned long long)en[t].z;
+          r.bytes += 4ull * (unsigned long long)(en[t].w + en[t].z) + (LABELED ? (unsigned long long)en[t].w : 0ull);
+        }
+        const unsigned miss = __ballot_sync(FULL, in[t] && !hit);
+        if (miss) {
+          if (in[t] && !hit) S.queue[queued + __popc(miss & lanemask_lt())] = x[t];
+          queued += __popc(miss);
+          __syncwarp();
+          if (queued >= 32) {
+            meet_values<LABELED>(a, S, set, mode, last_group, ub_last, 32, r);
+            const int rest = lane < queued - 32 ? S.queue[32 + lane] : 0;
+            __syncwarp();
+            queued -= 32;
+            if (lane < queued) S.queue[lane] = rest;
+            __syncwarp();
+          }
+        }
+      }
+    }
+  }
+  if (queued) meet_values<LABELED>(a, S, set, mode, last_group, ub_last, queued, r);
+  // one operation per candidate and its copy, one per element; the main
+  // operations' results are the elements
+  unsigned long long cnt = r.cnt, bytes = r.bytes + 4ull * r.elems;
+  ops += r.elems;
+  for (int d = 16; d; d >>= 1) {
+    cnt += __shfl_xor_sync(FULL, cnt, d);
+    bytes += __shfl_xor_sync(FULL, bytes, d);
+    ops += __shfl_xor_sync(FULL, ops, d);
   }
   w.setops += ops;
   w.bytes += bytes;
@@ -1402,30 +2467,44 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
   const int n = P.nnodes;
   if (lane == 0) S.top[1] = 0;
   __syncwarp();
-  if (n == 3) return (unsigned long long)run_slot<LABELED, PAGED>(a, P, S, 1, P.level_begin[1], 0, true, w);
-  {
-    const unsigned long long so = w.setops, by = w.bytes, rd = w.reads;
-    const long long c0 = clock64();
-    for (int k = 1; k <= L0 && !w.err; k++) run_level<LABELED, PAGED>(a, P, S, k, w);
-    if (!counted_prefix) {
-      w.setops = so;
-      w.bytes = by;
-      w.reads = rd;
-      w.prefix_cyc += (unsigned long long)(clock64() - c0);
-    } else {
-      w.level_cyc += (unsigned long long)(clock64() - c0);
-    }
+  if (n == 3) {
+    Work t;
+    memset(&t, 0, sizeof(t));
+    const unsigned long long c = (unsigned long long)count_slot<LABELED, PAGED>(a, P, S, 1, P.level_begin[1], 0, &t);
+    add_work(w, t);
+    return c;
   }
-  if (w.err) return 0;
+  const unsigned long long so = w.setops, by = w.bytes, rd = w.reads;
   unsigned long long cnt = 0;
-  {
-    int end0 = S.size[P.level_begin[L0]];
-    if (e >= 0 && e < end0) end0 = e;
-    if (lane == 0) { S.iter[L0] = b; S.iend[L0] = end0; }
-    __syncwarp();
-  }
-  int L = L0;
+  int L = 1;
+  bool enter = true, prefix = true;  // level L's slots are still to be computed; L is on the given path
   while (true) {
+    if (enter) {
+      const long long c0 = clock64();
+      run_level<LABELED, PAGED>(a, P, S, L, w);
+      const unsigned long long cyc = (unsigned long long)(clock64() - c0);
+      if (prefix && !counted_prefix) w.prefix_cyc += cyc;
+      else w.level_cyc += cyc;
+      if (w.err) return 0;
+      if (L < L0) {
+        L++;
+        continue;
+      }
+      int it0 = 0, end0 = S.raw[P.level_begin[L]];
+      if (prefix) {
+        prefix = false;
+        if (!counted_prefix) {
+          w.setops = so;
+          w.bytes = by;
+          w.reads = rd;
+        }
+        it0 = b;
+        if (e >= 0 && e < end0) end0 = e;
+      }
+      if (lane == 0) { S.iter[L] = it0; S.iend[L] = end0; }
+      __syncwarp();
+      enter = false;
+    }
     // by the clock: the launch-wide deadline, the liveness signal for waiting
     // warps, and the look for waiting warps to hand work to (set operations
     // take from under a microsecond to hundreds, so counting them is no clock)
@@ -1444,7 +2523,10 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
         w.err |= (unsigned)late;
         return 0;
       }
-      if (a.split_min > 0 && __any_sync(FULL, clock64() - S.began >= PM_CHECK_CYCLES)) {
+      bool worth = __any_sync(FULL, clock64() - S.began >= PM_CHECK_CYCLES);
+      if constexpr (!LABELED && !PAGED)  // (a clique's matrix: long to build)
+        worth = worth || (P.clique && a.clique_bits && S.size[P.level_begin[L] + 1] > 128);
+      if (a.split_min > 0 && worth) {
         w.err |= publish_pieces(a, S, n, L0, L, plan_id, root_id);
         if (w.err) return 0;
       }
@@ -1454,12 +2536,40 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
     const int m = P.level_begin[L];
     const int it = S.iter[L];
     const int iend = S.iend[L];
-    bool subtree = false;
-    if constexpr (!LABELED && !PAGED)
-      subtree = P.l2_x >= 0 && L + 4 == n && it < iend && a.lane_subtree_max > 0 &&
+    bool subtree = false, bits = false;
+    if constexpr (!LABELED && !PAGED) {
+      const int hs = P.level_begin[L] + 1;
+      bits = a.clique_bits && P.clique && L + 4 <= n && it < iend && S.size[hs] <= PM_CLIQUE_MAX &&
+             S.top[L + 1] + clique_words(S.size[hs]) <= S.cap;
+      subtree = !bits && P.l2_x >= 0 && L + 4 == n && it < iend && a.lane_subtree_max > 0 &&
                 S.size[P.parent[P.l2_x]] <= a.lane_subtree_max &&
                 S.top[L + 1] + 32ll * S.size[P.parent[P.l2_x]] <= S.cap;
-    if (subtree) {
+    }
+    if (!bits && it < iend && L + 4 == n && pair_ready<LABELED, PAGED>(a, P, S)) {
+      const int e2 = min(iend, it + 32);
+      const long long c0 = clock64();
+      Work t;
+      memset(&t, 0, sizeof(t));
+      cnt += pair_levels<LABELED, PAGED>(a, P, S, L, it, e2, &t);
+      add_work(w, t);
+      w.leaf_cyc += (unsigned long long)(clock64() - c0);
+      if (lane == 0) S.iter[L] = e2;
+      __syncwarp();
+      if (w.err) return 0;
+    } else if (bits) {
+      // (a look for waiting warps between: every candidate below a large set
+      // may be long, the more so with levels between it and the last)
+      const int e2 = min(iend, it + (S.size[P.level_begin[L] + 1] <= 32 ? 32 : L + 4 == n ? 8 : 1));
+      const long long c0 = clock64();
+      unsigned long long ops, bytes;
+      cnt += clique_bits(a, P, S, L, it, e2, &ops, &bytes);
+      w.setops += ops;
+      w.bytes += bytes;
+      w.reads++;
+      w.leaf_cyc += (unsigned long long)(clock64() - c0);
+      if (lane == 0) S.iter[L] = e2;
+      __syncwarp();
+    } else if (subtree) {
       const int e2 = min(iend, it + 32);
       const long long c0 = clock64();
       cnt += lane_subtree(a, P, S, L, it, e2, w);
@@ -1475,21 +2585,14 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
       __syncwarp();
       if (w.err) return 0;
     } else if (it < iend) {
-      const int v = S.arena[S.off[m] + it];
+      const int v = S.ptr[m][it];
+      const bool skip = !LABELED && S.raw[m] != S.size[m] && on_path(S, L, v);
+      __syncwarp();
       if (lane == 0) { S.iter[L] = it + 1; S.path[L + 1] = v; }
       __syncwarp();
-      const long long c0 = clock64();
-      if (L + 1 == n - 2) {
-        cnt += (unsigned long long)run_slot<LABELED, PAGED>(a, P, S, L + 1, P.last_slot, S.top[L + 1], true, w);
-        w.leaf_cyc += (unsigned long long)(clock64() - c0);
-      } else {
-        L++;
-        run_level<LABELED, PAGED>(a, P, S, L, w);
-        w.level_cyc += (unsigned long long)(clock64() - c0);
-        if (lane == 0) { S.iter[L] = 0; S.iend[L] = S.size[P.level_begin[L]]; }
-        __syncwarp();
-      }
-      if (w.err) return 0;
+      if (skip) continue;
+      L++;
+      enter = true;
     } else {
       L--;
       if (L < L0) break;
@@ -1586,6 +2689,15 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   if (lane == 0) {
     S.next_check = 0;
     S.checks = 0;
+    S.next_id = 0;
+    S.sb_id = 0;
+    S.cq_id = 0;
+    S.memo = a.memo ? a.memo + gw * (a.memo_entries + 1) : nullptr;
+    S.memo_epoch = a.memo ? (uint32_t)S.memo[a.memo_entries].x : 0u;
+    S.memo_id = 0;
+    S.memo_len = -1;
+    S.memo_ub = 0;
+    for (int k = 0; k < 16; k++) S.ptr[k] = nullptr;
     S.t_start = global_ns();
     S.arena = own;
     S.cap = a.slot_words;
@@ -1605,152 +2717,150 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   const int np = a.nplans;
   int p = (int)(gw % np);
   int exhausted = 0;
-  // phase 1: root chunks from the per-plan cursors
-  while (exhausted < np && !w.err) {
-    const DPlan& P = a.plans[p];
-    // a pop is `pop` roots of one shard unit of `chunk` roots (the last pop of
-    // a unit, and the last unit, may be shorter)
-    const unsigned long long per = (unsigned long long)((a.chunk + a.pop - 1) / a.pop);
-    const unsigned long long nchunks = (unsigned long long)((P.nroots + a.chunk - 1) / a.chunk);
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(&a.cursors[p], 1ull);
-    c = __shfl_sync(FULL, c, 0);
-    const unsigned long long gc = c / per * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
-    if (gc >= nchunks) {
-      exhausted++;
-      p = (p + 1 == np) ? 0 : p + 1;
-      continue;
-    }
-    const long long sub = (long long)(c % per) * a.pop;  // within the unit
-    exhausted = 0;
-    if (PAGED && a.pf_off && p == 0 && sub == 0) {
-      // post the predicted pages of a chunk this warp's successors will reach
-      const long long pc = (long long)gc + (long long)a.pf_ahead * a.shard_count;
-      // only while the host's queue is short: a page posted behind a long
-      // queue stays LOADING, and warps that miss on it meanwhile can neither
-      // read it from a frame nor load it themselves
-      unsigned long long queued = 0;
-      if (lane == 0) queued = *(volatile unsigned long long*)a.pg.ring_head - *(volatile unsigned long long*)a.pg.host_tail;
-      queued = __shfl_sync(FULL, queued, 0);  // one decision for the warp (the block below shuffles)
-      if (pc < a.pf_chunks && queued < 64) {
-        PageCounters lpc = {};
-        for (int k = a.pf_off[pc] + lane; k < a.pf_off[pc + 1]; k += 32) {
-          const int32_t pg = a.pf_pages[k];
-          if (pg >= 0 && pg < a.pg.n_pages && ld_vol(&a.pg.page_frame[pg]) == PAGE_ABSENT) request_page(a.pg, pg, lpc);
-        }
-        unsigned long long v[3] = {lpc.requests, lpc.evictions, lpc.dropped};
-#pragma unroll
-        for (int q = 0; q < 3; q++)
-          for (int o = 16; o; o >>= 1) v[q] += __shfl_xor_sync(FULL, v[q], o);
-        w.pc.requests += v[0];
-        w.pc.evictions += v[1];
-        w.pc.dropped += v[2];
-        w.prefetched += v[0];
-      }
-    }
-    const long long rb = (long long)gc * a.chunk + sub;
-    const long long re = min((long long)P.nroots, (long long)gc * a.chunk + min((long long)a.chunk, sub + a.pop));
-    unsigned long long local = 0;
-    for (long long r = rb; r < re && !w.err; r++) {
-      // position r of the range; with an order, the order's entry there
-      const long long pos = P.rbase + r;
-      const long long rid = a.root_order ? (long long)a.root_order[pos] : pos;
-      const int2 e = P.roots[rid];
-      const unsigned long long b0 = w.bytes, r0 = w.reads;
-      if (lane == 0) {
-        S.path[0] = e.x;
-        S.path[1] = e.y;
-        S.split = (a.root_split && p == 0) ? a.root_split[rid] : a.split_min;
-        S.began = clock64();
-      }
-      __syncwarp();
-      const unsigned long long c0 = dfs_from<LABELED, PAGED>(a, P, S, 1, 0, -1, true, p, (int)rid, w);
-      return_arena(a, S, own);
-      local += c0;
-      roots++;
-      if (lane == 0 && p == 0) {
-        if (a.root_counts) atomicAdd(&a.root_counts[rid], c0);
-        if (a.root_cost) atomicAdd(&a.root_cost[rid], (float)(w.bytes - b0 + 8));
-        if (a.root_reads) atomicAdd(&a.root_reads[rid], (float)(w.reads - r0));
-      }
-    }
-    if (lane == 0 && local) atomicAdd(&a.counts[p], local);
-    p = (p + 1 == np) ? 0 : p + 1;  // interleave plans chunk by chunk
-  }
-  // phase 2: take pieces until every warp is out of work.  A warp that failed
-  // draws no ticket (a piece given to it would be lost): the status word ends
-  // the others' wait.
-  if (w.err && lane == 0) atomicOr(a.status, w.err);
-  unsigned long long last_beat = 0, last_change = global_ns();
-  const unsigned long long t_drain = last_change;
-  unsigned long long busy_ns = 0;
+  long long r = 0, re = 0;        // phase 1: roots [r, re) of the last pop
+  unsigned long long local = 0;   // matches of plan `plan` not yet in a.counts
+  int plan = p;
+  // phase 2: the ticket, and for how long
+  bool waiting = false;
+  unsigned long long ticket = kQuit, last_beat = 0, last_change = 0, t_drain = 0, busy_ns = 0, t_item = 0;
   unsigned seen = 0;
-  unsigned long long ticket = w.err ? kQuit : draw_ticket(a, seen);
   int looks = 0;
-  while (!w.err && ticket != kQuit) {
+  while (!w.err) {
     Donation item;
-    const int got = wait_piece(a, ticket, item);
-    if (got < 0) break;
-    if (got > 0) {
-      const unsigned long long t_item = global_ns();
-      const DPlan& P = a.plans[item.plan];
-      const int2 e = P.roots[item.root];
-      if (lane == 0) {
-        S.path[0] = e.x;
-        S.path[1] = e.y;
-        for (int k = 2; k <= item.level; k++) S.path[k] = item.path[k];
-        S.split = (a.root_split && item.plan == 0) ? a.root_split[item.root] : a.split_min;
-        S.began = clock64();
+    item.level = 1;
+    item.begin = 0;
+    item.end = -1;
+    bool whole = true;  // a root, not a piece of one
+    if (r < re) {
+      // position r of the range; with an order, the order's entry there
+      const long long pos = a.plans[plan].rbase + r;
+      item.root = (int)(a.root_order ? (long long)a.root_order[pos] : pos);
+      r++;
+      roots++;
+    } else if (exhausted < np) {
+      // phase 1: root chunks from the per-plan cursors, plans in turn
+      if (lane == 0 && local) atomicAdd(&a.counts[plan], local);
+      local = 0;
+      const DPlan& P = a.plans[p];
+      // a pop is `pop` roots of one shard unit of `chunk` roots (the last pop of
+      // a unit, and the last unit, may be shorter)
+      const unsigned long long per = (unsigned long long)((a.chunk + a.pop - 1) / a.pop);
+      const unsigned long long nchunks = (unsigned long long)((P.nroots + a.chunk - 1) / a.chunk);
+      unsigned long long c = 0;
+      if (lane == 0) c = atomicAdd(&a.cursors[p], 1ull);
+      c = __shfl_sync(FULL, c, 0);
+      const unsigned long long gc = c / per * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
+      plan = p;
+      p = (p + 1 == np) ? 0 : p + 1;
+      if (gc >= nchunks) {
+        exhausted++;
+        continue;
       }
-      __syncwarp();
-      const unsigned long long b0 = w.bytes, r0 = w.reads;
-      const unsigned long long c0 = dfs_from<LABELED, PAGED>(a, P, S, item.level, item.begin, item.end, false,
-                                                             item.plan, item.root, w);
-      return_arena(a, S, own);
-      if (lane == 0) {
-        if (c0) atomicAdd(&a.counts[item.plan], c0);
-        if (item.plan == 0) {
-          if (a.root_counts) atomicAdd(&a.root_counts[item.root], c0);
-          if (a.root_cost) atomicAdd(&a.root_cost[item.root], (float)(w.bytes - b0));
-          if (a.root_reads) atomicAdd(&a.root_reads[item.root], (float)(w.reads - r0));
+      const long long sub = (long long)(c % per) * a.pop;  // within the unit
+      exhausted = 0;
+      if (PAGED && a.pf_off && plan == 0 && sub == 0) {
+        // post the predicted pages of a chunk this warp's successors will reach
+        const long long pc = (long long)gc + (long long)a.pf_ahead * a.shard_count;
+        // only while the host's queue is short: a page posted behind a long
+        // queue stays LOADING, and warps that miss on it meanwhile can neither
+        // read it from a frame nor load it themselves
+        unsigned long long queued = 0;
+        if (lane == 0)
+          queued = *(volatile unsigned long long*)a.pg.ring_head - *(volatile unsigned long long*)a.pg.host_tail;
+        queued = __shfl_sync(FULL, queued, 0);  // one decision for the warp (the block below shuffles)
+        if (pc < a.pf_chunks && queued < 64) {
+          PageCounters lpc = {};
+          for (int k = a.pf_off[pc] + lane; k < a.pf_off[pc + 1]; k += 32) {
+            const int32_t pg = a.pf_pages[k];
+            if (pg >= 0 && pg < a.pg.n_pages && ld_vol(&a.pg.page_frame[pg]) == PAGE_ABSENT)
+              request_page(a.pg, pg, lpc);
+          }
+          unsigned long long v[3] = {lpc.requests, lpc.evictions, lpc.dropped};
+#pragma unroll
+          for (int q = 0; q < 3; q++)
+            for (int o = 16; o; o >>= 1) v[q] += __shfl_xor_sync(FULL, v[q], o);
+          w.pc.requests += v[0];
+          w.pc.evictions += v[1];
+          w.pc.dropped += v[2];
+          w.prefetched += v[0];
         }
       }
-      __syncwarp();
-      last_change = global_ns();
-      busy_ns += last_change - t_item;
-      if (w.err) {
-        if (lane == 0) atomicOr(a.status, w.err);
-        break;
-      }
-      ticket = draw_ticket(a, seen);
-      looks = 0;
+      r = (long long)gc * a.chunk + sub;
+      re = min((long long)P.nroots, (long long)gc * a.chunk + min((long long)a.chunk, sub + a.pop));
       continue;
+    } else {
+      // phase 2: take pieces until every warp is out of work
+      if (!waiting) {
+        if (lane == 0 && local) atomicAdd(&a.counts[plan], local);
+        local = 0;
+        last_change = global_ns();
+        if (!t_drain) t_drain = last_change;
+        if (t_item) busy_ns += last_change - t_item;
+        ticket = draw_ticket(a, seen);
+        if (ticket == kQuit) break;
+        waiting = true;
+        looks = 0;
+      }
+      const int got = wait_piece(a, ticket, item);
+      if (got < 0) break;
+      if (got == 0) {
+        // poll the one word; the clock, the heartbeat and the status (words
+        // all waiting warps share) only every 64th time
+        __nanosleep(looks < 64 ? 100 : 400);
+        if (++looks & 63) continue;
+        unsigned long long beat = 0;
+        unsigned int failed = 0;
+        if (lane == 0) {
+          beat = ld_vol_u64(a.heartbeat);
+          failed = *(volatile unsigned int*)a.status;
+        }
+        beat = __shfl_sync(FULL, beat, 0);
+        if (__shfl_sync(FULL, failed, 0)) break;
+        // bounded wait: give up (and report DEV_TIMEOUT) when no warp has made
+        // progress for timeout_ns
+        const unsigned long long now = global_ns();
+        if (beat != last_beat) { last_beat = beat; last_change = now; }
+        else if (__any_sync(FULL, now > last_change && now - last_change > a.timeout_ns)) {
+          if (lane == 0) atomicOr(a.status, (unsigned)DEV_TIMEOUT);
+          break;
+        }
+        continue;
+      }
+      waiting = false;
+      whole = false;
+      plan = item.plan;
+      t_item = global_ns();
     }
-    // poll the one word; the clock, the heartbeat and the status (words all
-    // waiting warps share) only every 64th time
-    __nanosleep(looks < 64 ? 100 : 400);
-    if (++looks & 63) continue;
-    unsigned long long beat = 0;
-    unsigned int failed = 0;
+    const DPlan& P = a.plans[plan];
+    const int2 e = P.roots[item.root];
     if (lane == 0) {
-      beat = ld_vol_u64(a.heartbeat);
-      failed = *(volatile unsigned int*)a.status;
+      S.path[0] = e.x;
+      S.path[1] = e.y;
+      for (int k = 2; k <= item.level; k++) S.path[k] = item.path[k];
+      S.split = (a.root_split && plan == 0) ? a.root_split[item.root] : a.split_min;
+      S.began = clock64();
     }
-    beat = __shfl_sync(FULL, beat, 0);
-    if (__shfl_sync(FULL, failed, 0)) break;
-    // bounded wait: give up (and report DEV_TIMEOUT) when no warp has made
-    // progress for timeout_ns
-    const unsigned long long now = global_ns();
-    if (beat != last_beat) { last_beat = beat; last_change = now; }
-    else if (__any_sync(FULL, now > last_change && now - last_change > a.timeout_ns)) {
-      if (lane == 0) atomicOr(a.status, (unsigned)DEV_TIMEOUT);
-      break;
+    __syncwarp();
+    const unsigned long long b0 = w.bytes, r0 = w.reads;
+    const unsigned long long c0 = dfs_from<LABELED, PAGED>(a, P, S, item.level, item.begin, item.end, whole, plan,
+                                                           item.root, w);
+    return_arena(a, S, own);
+    local += c0;
+    if (lane == 0 && plan == 0) {
+      if (a.root_counts) atomicAdd(&a.root_counts[item.root], c0);
+      if (a.root_cost) atomicAdd(&a.root_cost[item.root], (float)(w.bytes - b0 + (whole ? 8 : 0)));
+      if (a.root_reads) atomicAdd(&a.root_reads[item.root], (float)(w.reads - r0));
     }
   }
+  // a warp that failed draws no ticket (a piece given to it would be lost):
+  // the status word ends the others' wait
+  if (w.err && lane == 0) atomicOr(a.status, w.err);
+  __syncwarp();
   if (lane == 0) {
+    if (a.memo) S.memo[a.memo_entries].x = (int32_t)S.memo_epoch;
     const unsigned long long t_end = global_ns();
     atomicAdd(&a.stats[ST_WARP_NS], t_end - S.t_start);
-    atomicAdd(&a.stats[ST_IDLE_NS], t_end - t_drain - min(busy_ns, t_end - t_drain));
+    if (t_drain) atomicAdd(&a.stats[ST_IDLE_NS], t_end - t_drain - min(busy_ns, t_end - t_drain));
     atomicAdd(&a.stats[ST_SETOPS], w.setops);
     atomicAdd(&a.stats[ST_BYTES], w.bytes + 8ull * roots);
     atomicAdd(&a.stats[ST_ROOTS], roots);
@@ -1771,7 +2881,6 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
         atomicAdd(&a.stats[ST_DEV_BYTES], w.pc.dev_bytes);
       }
     }
-    if (w.err) atomicOr(a.status, w.err);
   }
 }
 
@@ -1782,19 +2891,33 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
 // adjacency order), so root ids match the reference's Job[] indices.
 // =====================================================================
 
-__global__ void maxnbrdeg_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n, int32_t* out) {
+// Also sums a hash of every entry's vertex pair into *asym, with the sign of
+// the entry's direction: 0 when each entry has its reverse (and, but for one
+// graph in 2^64 or so, only then).
+__device__ __forceinline__ unsigned long long pair_hash(unsigned lo, unsigned hi) {
+  uint64_t x = ((uint64_t)hi << 32 | lo) + 0x9E3779B97F4A7C15ull;
+  return Rng::splitmix(x);
+}
+
+__global__ void maxnbrdeg_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n, int32_t* out,
+                                 unsigned long long* asym) {
   const int lane = lane_id();
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  unsigned long long sum = 0;
   for (long long v = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
     const uint64_t b = rowptr[v], e = rowptr[v + 1];
     int m = 0;
     for (uint64_t i = b + lane; i < e; i += 32) {
       const int u = colidx[i];
       m = max(m, (int)(rowptr[u + 1] - rowptr[u]));
+      if (u > v) sum += pair_hash((unsigned)v, (unsigned)u);
+      else if (u < v) sum -= pair_hash((unsigned)u, (unsigned)v);
     }
     for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
     if (lane == 0) out[v] = m;
   }
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+  if (lane == 0 && sum) atomicAdd(asym, sum);
 }
 
 // Regroups each list by label, keeping id order within a label (a stable
@@ -1844,6 +2967,40 @@ __global__ void label_group_kernel(const uint64_t* rowptr, const int32_t* colidx
       if (valid && (same & lanemask_lt()) == 0) base[lb] += __popc(same);
       __syncwarp();
     }
+  }
+}
+
+// Vertices per power of two of their degree (bin k: degree in [2^k, 2^(k+1))).
+__global__ void degree_bins_kernel(const uint64_t* rowptr, int64_t n, unsigned int* bins) {
+  __shared__ unsigned int b[32];
+  if (threadIdx.x < 32) b[threadIdx.x] = 0;
+  __syncthreads();
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned deg = (unsigned)(rowptr[v + 1] - rowptr[v]);
+    if (deg) atomicAdd(&b[31 - __clz(deg)], 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && b[threadIdx.x]) atomicAdd(&bins[threadIdx.x], b[threadIdx.x]);
+}
+
+// Gives every vertex of at least min_deg neighbours a bit row and fills it
+// (rows zeroed before), one warp per vertex.
+__global__ void hub_rows_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n, int min_deg, int64_t words,
+                                unsigned int* next, int32_t* slot, unsigned int* bits) {
+  const int lane = lane_id();
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long v = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
+    const uint64_t b = rowptr[v], e = rowptr[v + 1];
+    int k = -1;
+    if ((long long)(e - b) >= min_deg) {
+      if (lane == 0) k = (int)atomicAdd(next, 1u);
+      k = __shfl_sync(FULL, k, 0);
+      for (uint64_t i = b + lane; i < e; i += 32) {
+        const int u = colidx[i];
+        if (u >= 0 && u < n) atomicOr(&bits[k * words + (u >> 5)], 1u << (u & 31));
+      }
+    }
+    if (lane == 0) slot[v] = k;
   }
 }
 
@@ -1953,6 +3110,58 @@ DPlan to_dplan(const Plan& p) {
       }
     }
   }
+  // Slots that may be left in place with path vertices standing in them: main
+  // slots (their candidates are checked one by one) that no later set
+  // operation reads and no other slot stands for.
+  // leaf_adj: the path vertices that are neighbours of every candidate for
+  // vertex n-2, by the operations its slot is made of.
+  uint8_t made_of[16] = {1};  // slot 0 is N(v0)
+  for (int L = 1; L + 1 < p.nnodes; L++)
+    for (int s = p.level_begin[L]; s < (L + 2 < p.nnodes ? p.level_begin[L + 1] : p.nslots); s++) {
+      const uint8_t own = d.kind[s] == SLOT_COPY ? 0 : (uint8_t)(1u << L);
+      made_of[s] = own | (d.kind[s] == SLOT_FRESH ? 0 : made_of[d.parent[s]]);
+      d.hole_ok[s] = !p.labeled && s == p.level_begin[L] && d.alias[s] < 0;
+      for (int t = 1; t < p.nslots; t++)
+        if ((t != s && d.alias[t] == s) || (d.kind[t] != SLOT_FRESH && d.parent[t] == s)) d.hole_ok[s] = 0;
+    }
+  if (p.nnodes > 3) d.leaf_adj = made_of[p.level_begin[p.nnodes - 3]];
+  // The last two levels in one pass (pair_levels): level n-3 is a list of its
+  // vertex, or that list met with a slot of the level before, and at most a
+  // copy the last slot reads; no bound may involve the last two vertices but
+  // the main slot's own.
+  const int q2 = p.nnodes - 3;
+  if (q2 >= 2) {
+    const int b = p.level_begin[q2], k = p.level_begin[q2 + 1] - b, last = d.last_slot;
+    const uint32_t early = (1u << q2) - 1u;  // bounds by v_0 .. v_{n-4}
+    const bool met = d.kind[b] == SLOT_INTERSECT;
+    bool ok = (d.kind[b] == SLOT_FRESH || met) && d.alias[b] < 0;
+    if (p.labeled) ok = ok && __builtin_popcount(p.slot_labels[b]) == 1 && __builtin_popcount(p.slot_labels[last]) == 1;
+    auto within = [&](int small, int large) { return (p.slot_labels[small] & ~p.slot_labels[large]) == 0; };
+    if (ok && k == 1) {
+      if (d.kind[last] == SLOT_FRESH && !(p.partial[last] & ~early)) d.pair = PAIR_FRESH;
+    } else if (ok && k == 2 && d.alias[b + 1] < 0 && d.kind[b + 1] == SLOT_COPY && d.kind[last] != SLOT_FRESH &&
+               d.parent[last] == b + 1) {
+      const int h = b + 1;
+      d.pair_h0 = (int8_t)d.parent[h];
+      if (d.kind[last] == SLOT_COPY) {
+        if (p.labeled ? within(d.parent[h], h) && within(h, last) : !p.partial[h] && !p.partial[last])
+          d.pair = PAIR_COPY;
+      } else if (!met && (p.labeled ? within(d.parent[h], h) : !(p.partial[h] & ~early) && !(p.partial[last] & ~early))) {
+        d.pair = PAIR_MEET;
+      }
+    }
+  }
+  // Cliques (unlabeled, five vertices or more): on every level a main slot
+  // that is the prefix of the one helper below the smallest path vertex, both
+  // the intersection of the newest vertex's list with the helper before.
+  d.clique = !p.labeled && p.nnodes >= 5 && p.partial[0] == 1;
+  for (int L = 1; L + 1 < p.nnodes && d.clique; L++) {
+    const int b = p.level_begin[L], k = (L + 2 < p.nnodes ? p.level_begin[L + 1] : p.nslots) - b;
+    const int up = L == 1 ? 0 : p.level_begin[L - 1] + 1;
+    if (k != (L + 2 < p.nnodes ? 2 : 1)) d.clique = 0;
+    for (int s = b; s < b + k; s++)
+      if (d.kind[s] != SLOT_INTERSECT || d.parent[s] != up || p.partial[s] != (2u << L) - 1u) d.clique = 0;
+  }
   // Shape for lane_subtree (unlabeled): level n-3 is one intersection X with
   // a parent at an earlier level, plus at most one alias Y of it; the last
   // slot intersects with X or Y.
@@ -2004,13 +3213,21 @@ int64_t arena_words_for(const Plan& p, int32_t maxdeg, int T) {
 
 }  // namespace
 
+// d_maxnbrdeg: n entries and, after them, the 64-bit word maxnbrdeg_kernel sums
+// the entries' directions into.
+static size_t maxnbrdeg_bytes(int64_t n) { return sizeof(int32_t) * (size_t)((n + 1) & ~1ll) + 8; }
+static unsigned long long* asym_word(const pm_graph* g) {
+  return reinterpret_cast<unsigned long long*>(g->d_maxnbrdeg + ((g->n + 1) & ~1ll));
+}
+
 namespace pm {
 // Fills g->d_maxnbrdeg from an adjacency array the device can read (HBM or
 // mapped host memory).
 pm_status compute_maxnbrdeg(pm_graph* g, const int32_t* colidx) {
   if (g->n > 0) {
     PM_CK_PENDING("max neighbour degree");
-    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, colidx, g->n, g->d_maxnbrdeg);
+    CK(cudaMemset(asym_word(g), 0, 8));
+    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
   }
@@ -2020,13 +3237,48 @@ pm_status compute_maxnbrdeg(pm_graph* g, const int32_t* colidx) {
 
 static pm_status graph_finish(pm_graph* g) {
   // per-vertex max neighbour degree, used by the root filter
-  CK(cudaMalloc(&g->d_maxnbrdeg, sizeof(int32_t) * std::max<int64_t>(g->n, 1)));
+  CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
   g->device_bytes += sizeof(int32_t) * g->n;
   if (g->n > 0 && g->residency == PM_RESIDENT_HBM) {
     PM_CK_PENDING("max neighbour degree");
-    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg);
+    CK(cudaMemset(asym_word(g), 0, 8));
+    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
+  }
+  if (!g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0 && g->nadj > 0) {
+    // Bit rows for the vertices with the longest lists: the lowest power of
+    // two of a degree from 64 on (shorter lists are read as fast as a row)
+    // from which all rows fit as many bytes as the adjacency array, or 64 MB
+    // if that is more, and 256 MB at most -- half of them stay in L2.
+    unsigned int* bins = nullptr;
+    unsigned int h[33];
+    CK(cudaMalloc(&bins, sizeof(h)));
+    cudaError_t e = cudaMemset(bins, 0, sizeof(h));
+    if (e == cudaSuccess) {
+      degree_bins_kernel<<<256, 256>>>(g->d_rowptr, g->n, bins);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(h, bins, sizeof(h), cudaMemcpyDeviceToHost);
+    const int64_t words = (g->n + 31) / 32;
+    const size_t budget = std::min<size_t>(256ull << 20, std::max<size_t>(64ull << 20, 4 * (size_t)g->nadj));
+    size_t rows = 0;
+    int k = 31;
+    for (; e == cudaSuccess && k > 6 && (rows + h[k - 1]) * words * 4 <= budget; k--) rows += h[k - 1];
+    if (e == cudaSuccess && rows) {
+      e = cudaMalloc(&g->d_hub_slot, sizeof(int32_t) * g->n);
+      if (e == cudaSuccess) e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
+      if (e == cudaSuccess) e = cudaMemset(g->d_hub_bits, 0, rows * words * 4);
+      if (e == cudaSuccess) {
+        hub_rows_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->n, 1 << k, words, bins + 32, g->d_hub_slot,
+                                       g->d_hub_bits);
+        e = cudaGetLastError();
+      }
+      if (e == cudaSuccess) e = cudaDeviceSynchronize();
+      g->device_bytes += sizeof(int32_t) * g->n + rows * words * 4;
+    }
+    cudaFree(bins);
+    CK(e);
   }
   if (g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0) {
     g->nl1 = (g->nlabels > 0 ? g->nlabels : 32) + 1;
@@ -2151,7 +3403,7 @@ extern "C" pm_status pm_graph_from_host(int64_t n, int64_t nadj, const uint64_t*
   if (o.residency == PM_RESIDENT_PAGED) {
     st = paged_place(g.get(), colidx, &o, nullptr);
     if (st != PM_OK) return st;
-    CK(cudaMalloc(&g->d_maxnbrdeg, sizeof(int32_t) * std::max<int64_t>(g->n, 1)));
+    CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
     g->device_bytes += sizeof(int32_t) * g->n;
     st = paged_maxnbrdeg(g.get());
     if (st != PM_OK) return st;
@@ -2196,7 +3448,7 @@ extern "C" pm_status pm_graph_from_paged_source(int64_t n, int64_t nadj, const u
   // the id-sorted lists: root filter, features, and a labeled graph's whole
   // lists (read in place)
   g->h_colidx_dev = const_cast<int32_t*>(sorted);
-  CK(cudaMalloc(&g->d_maxnbrdeg, sizeof(int32_t) * std::max<int64_t>(g->n, 1)));
+  CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
   g->device_bytes += sizeof(int32_t) * g->n;
   st = paged_maxnbrdeg(g.get());
   if (st != PM_OK) return st;
@@ -2277,6 +3529,8 @@ extern "C" void pm_graph_close(pm_graph* g) {
   free_dev(g->d_maxnbrdeg);
   free_dev(g->d_colidx_lab);
   free_dev(g->d_lab_off);
+  free_dev(g->d_hub_slot);
+  free_dev(g->d_hub_bits);
   paged_release(g);
   delete g;
 }
@@ -2304,6 +3558,8 @@ extern "C" void pm_ctx_destroy(pm_ctx* c) {
   cudaStreamSynchronize(c->copy_stream);
   free_dev(c->d_arena);
   free_dev(c->d_ctl);
+  if (c->memo) free_dev(c->memo->d);
+  delete c->memo;
   free_dev(c->d_roots);
   free_dev(c->d_tmp);
   free_dev(c->d_vcount);
@@ -2428,6 +3684,7 @@ struct Launch {
   void (*kfn)(const MatchArgs) = nullptr;
   int64_t warps = 0;
   size_t ctl_words = 0;
+  int memo_entries = 0;       // per warp (pair_levels)
 };
 
 static constexpr unsigned kDonSlots = 1u << 13;  // a launch has at most a few thousand warps
@@ -2437,13 +3694,19 @@ static constexpr int64_t kOwnGatherWords = 1 << 15;
 static constexpr size_t kBigPoolMaxBytes = 48ull << 30;
 static constexpr int kCtlRead = 32 + 32 + kStatWords + 1;  // cursors, counts, stats, status word
 
+static MemoTables* memo_of(pm_ctx* c) {
+  if (!c->memo) c->memo = new MemoTables;
+  return c->memo;
+}
+
 // Validates the plans and options, builds the root lists into *roots,
 // sizes the persistent grid and the arenas, and fills L.  Buffers are grown
 // as needed (they belong to the caller: the context for pm_match, the query
 // for pm_query_prepare).
 static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const* plans, int nplans,
                               const pm_run_opts& o, int2** roots, size_t* roots_bytes, int32_t** arena,
-                              size_t* arena_bytes, unsigned long long** ctl, size_t* ctl_bytes, Launch* L) {
+                              size_t* arena_bytes, unsigned long long** ctl, size_t* ctl_bytes, MemoTables* mt,
+                              Launch* L) {
   if (nplans < 1 || nplans > PM_MAX_BATCH) return fail(PM_ERR_INVALID, "between 1 and %d plans per launch", PM_MAX_BATCH);
   CK(cudaSetDevice(c->device));
   L->labeled = plan_of(plans[0]) && plan_of(plans[0])->labeled != 0;
@@ -2565,6 +3828,31 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   st = ensure((void**)ctl, ctl_bytes, L->ctl_words * 8);
   if (st != PM_OK) return st;
 
+  // value tables for plans that meet lists at the last level: one entry per
+  // vertex up to 16,384 (a warp's lookups go to the lists of a few roots'
+  // surroundings, not to the whole graph), within an eighth of free memory
+  MemoEntry* none = nullptr;
+  MemoEntry** memo = &none;
+  bool meets = false;
+  for (int i = 0; i < nplans; i++) meets = meets || L->dp[i].pair == PAIR_MEET;
+  if (meets && !L->paged && o.leaf_per_lane == 0) {
+    int entries = 256;
+    while (entries < 16384 && entries < g->n) entries <<= 1;
+    auto need = [&]() { return (size_t)L->warps * (size_t)(entries + 1) * sizeof(MemoEntry); };
+    while (entries > 256 && need() > (free_b + mt->bytes) / 8) entries >>= 1;
+    if (need() <= (free_b + mt->bytes) / 8) {
+      const bool fresh = mt->bytes < need() || !mt->d;
+      st = ensure((void**)&mt->d, &mt->bytes, need());
+      if (st != PM_OK) return st;
+      if (fresh || mt->warps != L->warps || mt->entries != entries)
+        CK(cudaMemsetAsync(mt->d, 0, need(), c->stream));
+      mt->warps = L->warps;
+      mt->entries = entries;
+      L->memo_entries = entries;
+      memo = &mt->d;
+    }
+  }
+
   MatchArgs& a = L->a;
   memset(&a, 0, sizeof(a));
   a.rowptr = g->d_rowptr;
@@ -2572,9 +3860,17 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.labels = g->d_labels;
   a.colidx_lab = g->d_colidx_lab;
   a.lab_off = g->d_lab_off;
+  a.pairs = o.leaf_per_lane == 0;
+  a.asym = g->n > 0 ? asym_word(g) : nullptr;
+  a.memo = *memo;
+  a.memo_entries = L->memo_entries;
+  a.hub_slot = g->d_hub_slot;
+  a.hub_bits = g->d_hub_bits;
+  a.hub_words = (int32_t)((g->n + 31) / 32);
   a.host_sorted = (g->residency == PM_RESIDENT_PAGED && g->d_lab_off) ? g->h_colidx_dev : nullptr;
   a.leaf_flat = o.leaf_per_lane == 1 ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
+  a.clique_bits = o.lane_subtree_max == 0;
   a.nl1 = g->nl1;
   a.n = (int32_t)g->n;
   a.nplans = nplans;
@@ -2731,7 +4027,7 @@ extern "C" pm_status pm_match(pm_ctx* c, const pm_graph* g, const pm_plan* const
   CK(cudaEventRecord(e0, c->stream));
   std::unique_ptr<Launch> L(new Launch);
   pm_status st = setup_launch(c, g, plans, nplans, o, &c->d_roots, &c->roots_bytes, &c->d_arena, &c->arena_bytes,
-                              &c->d_ctl, &c->ctl_bytes, L.get());
+                              &c->d_ctl, &c->ctl_bytes, memo_of(c), L.get());
   if (st != PM_OK) return st;
   unsigned long long host_ctl[kCtlRead];
   pm_stats pst;
@@ -2757,6 +4053,7 @@ struct pm_query {
   size_t arena_bytes = 0;
   unsigned long long* d_ctl = nullptr;
   size_t ctl_bytes = 0;
+  MemoTables memo;
   unsigned long long* h_ctl = nullptr;  // pinned
   cudaEvent_t eb = nullptr, ee = nullptr;
   cudaGraph_t graph = nullptr;
@@ -2774,6 +4071,7 @@ extern "C" void pm_query_free(pm_query* q) {
   free_dev(q->d_roots);
   free_dev(q->d_arena);
   free_dev(q->d_ctl);
+  free_dev(q->memo.d);
   if (q->h_ctl) cudaFreeHost(q->h_ctl);
   delete q;
 }
@@ -2790,7 +4088,7 @@ extern "C" pm_status pm_query_prepare(pm_ctx* c, const pm_graph* g, const pm_pla
   q->g = g;
   CK(cudaEventRecord(c->ev[0], c->stream));
   pm_status st = setup_launch(c, g, plans, nplans, o, &q->d_roots, &q->roots_bytes, &q->d_arena, &q->arena_bytes,
-                              &q->d_ctl, &q->ctl_bytes, &q->L);
+                              &q->d_ctl, &q->ctl_bytes, &q->memo, &q->L);
   if (st != PM_OK) return st;
   CK(cudaEventRecord(c->ev[1], c->stream));
   CK(cudaEventSynchronize(c->ev[1]));
@@ -3000,6 +4298,7 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.labels = d_labels;
   a.leaf_flat = o.leaf_per_lane == 1 ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
+  a.clique_bits = o.lane_subtree_max == 0;
   a.n = (int32_t)n;
   a.nplans = 1;
   a.T = T;

@@ -19,6 +19,9 @@ enum : uint32_t {
   DEV_BAD_ROOT = 1u << 2,        // root id out of range
 };
 
+// What the last level adds per element of level n-3's main slot (pair_levels).
+enum PairKind : uint8_t { PAIR_NONE = 0, PAIR_COPY = 1, PAIR_FRESH = 2, PAIR_MEET = 3 };
+
 // One plan as the kernel reads it (constant memory).
 struct DPlan {
   int32_t nnodes;
@@ -38,7 +41,12 @@ struct DPlan {
   // intersection of level nnodes-3, its alias (or -1); l2_x = -1 when the
   // plan does not have that shape
   int8_t l2_x, l2_y;
-  int8_t pad_[6];
+  uint8_t leaf_adj;               // path vertices adjacent to every candidate for vertex nnodes-2 (bit j: v_j)
+  uint8_t clique;                 // the plan is an unlabeled clique's (clique_bits)
+  uint8_t pair;                   // PairKind of the last two levels (pair_levels), 0: none
+  int8_t pair_h0;                 // the slot its copy or meeting reads
+  int8_t pad_[2];
+  uint8_t hole_ok[16];            // 1: the slot may be read in place, path vertices skipped by its walker
   const int2* roots;              // (v0, v1) root edges, reference order (the whole list)
   int64_t nroots;                 // positions this launch processes
   int64_t rbase;                  // first position: root_begin (0 = all)
@@ -113,6 +121,10 @@ struct pm_graph {
   int32_t* d_colidx_lab = nullptr;
   int32_t* d_lab_off = nullptr;    // [n][nl1]: start of label l within v's list; [n][nl1-1] = deg
   int32_t nl1 = 0;
+  // unlabeled graphs in HBM: a bit row over all vertices for each vertex with
+  // a long list, and which row is whose
+  int32_t* d_hub_slot = nullptr;   // [n], -1: none
+  uint32_t* d_hub_bits = nullptr;  // [rows][(n + 31) / 32]
   uint64_t device_bytes = 0;
   // paged residency (pm_paging.cu)
   int32_t* h_colidx = nullptr;     // pinned, mapped copy of the adjacency array
@@ -128,6 +140,8 @@ struct pm_graph {
   pm::PagedState* ps = nullptr;
 };
 
+struct MemoTables;
+
 struct pm_ctx {
   int device = 0;
   int nsm = 0;
@@ -141,6 +155,7 @@ struct pm_ctx {
   size_t ctl_bytes = 0;
   int2* d_roots = nullptr;
   size_t roots_bytes = 0;
+  MemoTables* memo = nullptr;  // the warps' value tables
   void* d_tmp = nullptr;
   size_t tmp_bytes = 0;
   int32_t* d_vcount = nullptr;
