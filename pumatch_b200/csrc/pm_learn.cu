@@ -9,9 +9,10 @@
 //
 // The layers are far too small for tensor cores to matter (5,378 parameters;
 // a 64-wide layer is one 64x64 product per sample), so they run on the FMA
-// pipes: one thread per sample forward, and a tiled backward where each block
-// stages 64 samples' activations in shared memory and each thread then owns a
-// slice of the weight gradients (an outer-product accumulation over the tile).
+// pipes, in FP32 throughout (activations are not rounded): a block takes tiles
+// of samples through shared memory and each thread a register tile of every
+// layer's product, so that two 16-byte shared-memory reads feed 16 or 32
+// multiply-adds.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -49,152 +50,335 @@ static_assert(NPARAM == PM_MLP_PARAMS, "parameter count");
 
 __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
 
+// Two FP32 multiply-adds in one instruction (each rounded as fmaf rounds).
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
 // ---------------------------------------------------------------- forward
-__global__ void mlp_forward_kernel(const __nv_bfloat16* __restrict__ wq, const float* __restrict__ x, int64_t n,
-                                   float* __restrict__ y) {
-  __shared__ float w[NPARAM];
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) w[i] = bf(wq[i]);
-  __syncthreads();
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-    float xin[NIN];
-#pragma unroll
-    for (int i = 0; i < NIN; i++) xin[i] = x[s * NIN + i];
-    float h1[NH];
+// 128 samples per tile, 256 threads: thread (tx, ty) computes samples
+// [8 ty, 8 ty + 8) x units [4 tx, 4 tx + 4) of each 64-unit layer, sample
+// pairs packed.  Activations are kept unit-major, so a thread's eight samples
+// of a unit are two 16-byte reads; the last layer's two outputs are summed
+// over the 16 threads of a sample group by shuffles.  Bound: multiply-adds
+// (5,248 per sample).  Measured (B200), 262,144 samples: 325 us with one
+// thread per sample and a weight read per multiply-add, 79 us so.
+constexpr int FT = 128, FTP = FT + 4;
+
+struct ForwardSmem {  // (16-byte vectors are read from every array)
+  alignas(16) float w[NPARAM];
+  alignas(16) float xt[NIN][FTP];
+  alignas(16) float ht[NH][FTP];
+};
+static_assert(OFF_W2 % 4 == 0 && FTP % 4 == 0, "16-byte rows");
+
+template <int K>
+__device__ __forceinline__ void layer8x4(const float* __restrict__ in, const float* __restrict__ w, int tx, int ty,
+                                         unsigned long long (&acc)[4][4]) {
 #pragma unroll 8
-    for (int j = 0; j < NH; j++) {
-      float z = w[OFF_B1 + j];
+  for (int k = 0; k < K; k++) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(in + k * FTP + 8 * ty);
+    const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(in + k * FTP + 8 * ty + 4);
+    const float4 b = *reinterpret_cast<const float4*>(w + k * NH + 4 * tx);
+    const unsigned long long b2[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
 #pragma unroll
-      for (int i = 0; i < NIN; i++) z = fmaf(xin[i], w[OFF_W1 + i * NH + j], z);
-      h1[j] = fmaxf(z, 0.f);
+    for (int j = 0; j < 4; j++) {
+      acc[0][j] = fma2(a0.x, b2[j], acc[0][j]);
+      acc[1][j] = fma2(a0.y, b2[j], acc[1][j]);
+      acc[2][j] = fma2(a1.x, b2[j], acc[2][j]);
+      acc[3][j] = fma2(a1.y, b2[j], acc[3][j]);
     }
-    float o0 = w[OFF_B3], o1 = w[OFF_B3 + 1];
-    for (int k = 0; k < NH; k++) {
-      float z = w[OFF_B2 + k];
-#pragma unroll 8
-      for (int j = 0; j < NH; j++) z = fmaf(h1[j], w[OFF_W2 + j * NH + k], z);
-      const float a = fmaxf(z, 0.f);
-      o0 = fmaf(a, w[OFF_W3 + k * NOUT], o0);
-      o1 = fmaf(a, w[OFF_W3 + k * NOUT + 1], o1);
+  }
+}
+
+__global__ void __launch_bounds__(256) mlp_forward_kernel(const __nv_bfloat16* __restrict__ wq,
+                                                          const float* __restrict__ x, int64_t n,
+                                                          float* __restrict__ y) {
+  extern __shared__ float4 smem_raw[];
+  ForwardSmem& S = *reinterpret_cast<ForwardSmem*>(smem_raw);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < NPARAM; i += 256) S.w[i] = bf(wq[i]);
+  const int64_t tiles = (n + FT - 1) / FT;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t base = tile * FT;
+    __syncthreads();  // the last tile's reads (and the weights' writes)
+    for (int i = tid; i < FT * NIN; i += 256) {
+      const int r = i / NIN, k = i % NIN;
+      S.xt[k][r] = base + r < n ? x[(base + r) * NIN + k] : 0.f;
     }
-    y[s * NOUT] = o0;
-    y[s * NOUT + 1] = o1;
+    __syncthreads();
+    unsigned long long acc[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float b = S.w[OFF_B1 + 4 * tx + j];
+#pragma unroll
+      for (int r = 0; r < 4; r++) acc[r][j] = pack2(b, b);
+    }
+    layer8x4<NIN>(&S.xt[0][0], S.w + OFF_W1, tx, ty, acc);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 v0 = unpack2(acc[0][j]), v1 = unpack2(acc[1][j]), v2 = unpack2(acc[2][j]), v3 = unpack2(acc[3][j]);
+      float4* o = reinterpret_cast<float4*>(&S.ht[4 * tx + j][8 * ty]);
+      o[0] = make_float4(fmaxf(v0.x, 0.f), fmaxf(v0.y, 0.f), fmaxf(v1.x, 0.f), fmaxf(v1.y, 0.f));
+      o[1] = make_float4(fmaxf(v2.x, 0.f), fmaxf(v2.y, 0.f), fmaxf(v3.x, 0.f), fmaxf(v3.y, 0.f));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float b = S.w[OFF_B2 + 4 * tx + j];
+#pragma unroll
+      for (int r = 0; r < 4; r++) acc[r][j] = pack2(b, b);
+    }
+    layer8x4<NH>(&S.ht[0][0], S.w + OFF_W2, tx, ty, acc);
+    float o0[8], o1[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) o0[r] = o1[r] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float w0 = S.w[OFF_W3 + (4 * tx + j) * NOUT], w1 = S.w[OFF_W3 + (4 * tx + j) * NOUT + 1];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float2 v = unpack2(acc[r][j]);
+        const float a0 = fmaxf(v.x, 0.f), a1 = fmaxf(v.y, 0.f);
+        o0[2 * r] = fmaf(a0, w0, o0[2 * r]);
+        o1[2 * r] = fmaf(a0, w1, o1[2 * r]);
+        o0[2 * r + 1] = fmaf(a1, w0, o0[2 * r + 1]);
+        o1[2 * r + 1] = fmaf(a1, w1, o1[2 * r + 1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+#pragma unroll
+      for (int d = 8; d; d >>= 1) {
+        o0[r] += __shfl_xor_sync(0xffffffffu, o0[r], d);
+        o1[r] += __shfl_xor_sync(0xffffffffu, o1[r], d);
+      }
+      const int64_t s = base + 8 * ty + r;
+      if (tx == r && s < n) {
+        y[s * NOUT] = o0[r] + S.w[OFF_B3];
+        y[s * NOUT + 1] = o1[r] + S.w[OFF_B3 + 1];
+      }
+    }
   }
 }
 
 // ---------------------------------------------------------------- backward
-// Mean-squared-error gradients over the batch, accumulated in FP32.
-constexpr int TILE = 64;
+// Mean-squared-error gradients over the batch, accumulated in FP32.  64
+// samples per tile, 256 threads: thread (tx, ty) holds samples [4 ty, 4 ty + 4)
+// x units [4 tx, 4 tx + 4) of every layer in registers.  What the next product
+// contracts over decides the layout it reads: activations and their gradients
+// go to shared memory unit-major for the layers' products and sample-major
+// for the weights' outer products.  Weight gradients stay in registers over
+// all of a block's tiles and are added to the result once.  Bound: multiply-
+// adds (14,720 per sample), 16 per two 16-byte reads.  Measured (B200), 8,192
+// samples: 86 us with a quarter of the threads taking one sample
+// each (serial chains, 32-way bank conflicts), 18 us so.
+constexpr int TILE = 64, TP = TILE + 4;
+static_assert(TP % 4 == 0 && NH % 4 == 0, "16-byte rows");
 
 struct BackwardSmem {
-  float w[NPARAM];
-  float sx[TILE][NIN];
-  float sh1[TILE][NH];    // relu(z1)
-  float sdz1[TILE][NH];   // dL/dz1
-  float sa2[TILE][NH];    // relu(z2)
-  float sdz2[TILE][NH];   // dL/dz2
-  float sdo[TILE][NOUT];  // dL/dout
-  float sloss[TILE];
+  alignas(16) float w[NPARAM];
+  alignas(16) float w2t[NH][NH];   // W2 transposed: [k][j]
+  alignas(16) float xt[NIN][TP];
+  alignas(16) float h1[TILE][NH];    // relu(z1)
+  alignas(16) float h1t[NH][TP];
+  alignas(16) float dz2[TILE][NH];   // dL/dz2
+  alignas(16) float dz2t[NH][TP];
+  alignas(16) float dz1[TILE][NH];   // dL/dz1
+  float x[TILE][NIN];
+  float t[TILE][NOUT];
+  float red[16][4 * NH + 4];          // per sample group: b1, b2, W3 (two outputs) sums; b3, loss
 };
 
+// acc[r][j] += sum over k of in[k][4 ty + r] * w[k][4 tx + j] (rows of `in`
+// TP apart, of `w` NH apart).
+template <int K>
+__device__ __forceinline__ void tile4x4(const float* __restrict__ in, const float* __restrict__ w, int tx, int ty,
+                                        float (&acc)[4][4]) {
+#pragma unroll 8
+  for (int k = 0; k < K; k++) {
+    const float4 a = *reinterpret_cast<const float4*>(in + k * TP + 4 * ty);
+    const float4 b = *reinterpret_cast<const float4*>(w + k * NH + 4 * tx);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[r][j] = fmaf(av[r], bv[j], acc[r][j]);
+  }
+}
+
+// A thread's 4 x 4 values to the sample-major and (unless null) unit-major arrays.
+__device__ __forceinline__ void put4x4(const float (&v)[4][4], float (*rows)[NH], float (*units)[TP], int tx, int ty) {
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+    *reinterpret_cast<float4*>(&rows[4 * ty + r][4 * tx]) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+  if (units) {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      *reinterpret_cast<float4*>(&units[4 * tx + j][4 * ty]) = make_float4(v[0][j], v[1][j], v[2][j], v[3][j]);
+  }
+}
+
+__device__ __forceinline__ void add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// out: NPARAM gradients, then the loss (zeroed before).
 __global__ void __launch_bounds__(256) mlp_backward_kernel(const __nv_bfloat16* __restrict__ wq,
                                                            const float* __restrict__ x, const float* __restrict__ t,
-                                                           int64_t n, float* __restrict__ grad,
-                                                           float* __restrict__ loss) {
+                                                           int64_t n, float* __restrict__ out) {
   extern __shared__ float4 smem_raw[];
   BackwardSmem& S = *reinterpret_cast<BackwardSmem*>(smem_raw);
-  float* w = S.w;
-  auto& sx = S.sx;
-  auto& sh1 = S.sh1;
-  auto& sdz1 = S.sdz1;
-  auto& sa2 = S.sa2;
-  auto& sdz2 = S.sdz2;
-  auto& sdo = S.sdo;
-  auto& sloss = S.sloss;
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) w[i] = bf(wq[i]);
-  __syncthreads();
-  float g[(NPARAM + 255) / 256];  // this thread's slice of the gradient
-  for (int i = 0; i < (NPARAM + 255) / 256; i++) g[i] = 0.f;
-  float lsum = 0.f;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int i = tid; i < NPARAM; i += 256) {
+    const float v = bf(wq[i]);
+    S.w[i] = v;
+    if (i >= OFF_W2 && i < OFF_B2) S.w2t[(i - OFF_W2) % NH][(i - OFF_W2) / NH] = v;
+  }
   const float inv_n = 1.f / (float)(n * NOUT);
+  float gw2[4][4] = {}, gw1[4] = {};                    // W2 rows 4 ty.., columns 4 tx..; W1 row ty, columns 4 tx..
+  float gb1[4] = {}, gb2[4] = {}, gw3[4][NOUT] = {}, gb3[NOUT] = {}, lsum = 0.f;  // over this thread's samples
   for (int64_t base = (int64_t)blockIdx.x * TILE; base < n; base += (int64_t)gridDim.x * TILE) {
-    // phase A: one thread per sample -- forward and backward of the activations
-    if (threadIdx.x < TILE) {
-      const int r = threadIdx.x;
-      const int64_t s = base + r;
-      if (s < n) {
-        for (int i = 0; i < NIN; i++) sx[r][i] = x[s * NIN + i];
-        float z1[NH];
-        for (int j = 0; j < NH; j++) {
-          float z = w[OFF_B1 + j];
-          for (int i = 0; i < NIN; i++) z = fmaf(sx[r][i], w[OFF_W1 + i * NH + j], z);
-          z1[j] = z;
-          sh1[r][j] = fmaxf(z, 0.f);
-        }
-        float o0 = w[OFF_B3], o1 = w[OFF_B3 + 1];
-        for (int k = 0; k < NH; k++) {
-          float z = w[OFF_B2 + k];
-          for (int j = 0; j < NH; j++) z = fmaf(sh1[r][j], w[OFF_W2 + j * NH + k], z);
-          const float a = fmaxf(z, 0.f);
-          sa2[r][k] = a;
-          sdz2[r][k] = z > 0.f ? 1.f : 0.f;  // mask, scaled below
-          o0 = fmaf(a, w[OFF_W3 + k * NOUT], o0);
-          o1 = fmaf(a, w[OFF_W3 + k * NOUT + 1], o1);
-        }
-        const float e0 = o0 - t[s * NOUT], e1 = o1 - t[s * NOUT + 1];
-        sloss[r] = e0 * e0 + e1 * e1;
-        const float d0 = 2.f * e0 * inv_n, d1 = 2.f * e1 * inv_n;
-        sdo[r][0] = d0;
-        sdo[r][1] = d1;
-        for (int k = 0; k < NH; k++)
-          sdz2[r][k] *= fmaf(w[OFF_W3 + k * NOUT], d0, w[OFF_W3 + k * NOUT + 1] * d1);
-        for (int j = 0; j < NH; j++) {
-          float d = 0.f;
-          for (int k = 0; k < NH; k++) d = fmaf(w[OFF_W2 + j * NH + k], sdz2[r][k], d);
-          sdz1[r][j] = z1[j] > 0.f ? d : 0.f;
-        }
-      } else {
-        for (int i = 0; i < NIN; i++) sx[r][i] = 0.f;
-        for (int j = 0; j < NH; j++) { sh1[r][j] = 0.f; sdz1[r][j] = 0.f; sa2[r][j] = 0.f; sdz2[r][j] = 0.f; }
-        sdo[r][0] = sdo[r][1] = 0.f;
-        sloss[r] = 0.f;
+    __syncthreads();  // the last tile's reads (and the weights' writes)
+    for (int i = tid; i < TILE * NIN; i += 256) {
+      const int r = i / NIN, k = i % NIN;
+      const float v = base + r < n ? x[(base + r) * NIN + k] : 0.f;
+      S.x[r][k] = v;
+      S.xt[k][r] = v;
+    }
+    if (tid < TILE * NOUT) S.t[tid / NOUT][tid % NOUT] = base + tid / NOUT < n ? t[base * NOUT + tid] : 0.f;
+    __syncthreads();
+    float h1[4][4], v[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) h1[r][j] = S.w[OFF_B1 + 4 * tx + j];
+    tile4x4<NIN>(&S.xt[0][0], S.w + OFF_W1, tx, ty, h1);
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) h1[r][j] = fmaxf(h1[r][j], 0.f);
+    put4x4(h1, S.h1, S.h1t, tx, ty);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[r][j] = S.w[OFF_B2 + 4 * tx + j];
+    tile4x4<NH>(&S.h1t[0][0], S.w + OFF_W2, tx, ty, v);
+    // outputs, summed over the 16 threads of the sample group
+    float o0[4] = {}, o1[4] = {}, w30[4], w31[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      w30[j] = S.w[OFF_W3 + (4 * tx + j) * NOUT];
+      w31[j] = S.w[OFF_W3 + (4 * tx + j) * NOUT + 1];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float a = fmaxf(v[r][j], 0.f);
+        o0[r] = fmaf(a, w30[j], o0[r]);
+        o1[r] = fmaf(a, w31[j], o1[r]);
       }
     }
-    __syncthreads();
-    // phase B: each thread accumulates its parameters over the tile
-    for (int q = 0; q < (NPARAM + 255) / 256; q++) {
-      const int pidx = threadIdx.x + q * 256;
-      if (pidx >= NPARAM) break;
-      float acc = 0.f;
-      if (pidx < OFF_B1) {
-        const int i = pidx / NH, j = pidx % NH;
-        for (int r = 0; r < TILE; r++) acc = fmaf(sx[r][i], sdz1[r][j], acc);
-      } else if (pidx < OFF_W2) {
-        const int j = pidx - OFF_B1;
-        for (int r = 0; r < TILE; r++) acc += sdz1[r][j];
-      } else if (pidx < OFF_B2) {
-        const int j = (pidx - OFF_W2) / NH, k = (pidx - OFF_W2) % NH;
-        for (int r = 0; r < TILE; r++) acc = fmaf(sh1[r][j], sdz2[r][k], acc);
-      } else if (pidx < OFF_W3) {
-        const int k = pidx - OFF_B2;
-        for (int r = 0; r < TILE; r++) acc += sdz2[r][k];
-      } else if (pidx < OFF_B3) {
-        const int k = (pidx - OFF_W3) / NOUT, o = (pidx - OFF_W3) % NOUT;
-        for (int r = 0; r < TILE; r++) acc = fmaf(sa2[r][k], sdo[r][o], acc);
-      } else {
-        const int o = pidx - OFF_B3;
-        for (int r = 0; r < TILE; r++) acc += sdo[r][o];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+#pragma unroll
+      for (int d = 8; d; d >>= 1) {
+        o0[r] += __shfl_xor_sync(0xffffffffu, o0[r], d);
+        o1[r] += __shfl_xor_sync(0xffffffffu, o1[r], d);
       }
-      g[q] += acc;
+      const int row = 4 * ty + r;
+      const bool valid = base + row < n;
+      const float e0 = valid ? o0[r] + S.w[OFF_B3] - S.t[row][0] : 0.f;
+      const float e1 = valid ? o1[r] + S.w[OFF_B3 + 1] - S.t[row][1] : 0.f;
+      const float d0 = 2.f * e0 * inv_n, d1 = 2.f * e1 * inv_n;
+      if (tx == 0) {
+        lsum += e0 * e0 + e1 * e1;
+        gb3[0] += d0;
+        gb3[1] += d1;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float z = v[r][j], a = fmaxf(z, 0.f);
+        gw3[j][0] = fmaf(a, d0, gw3[j][0]);
+        gw3[j][1] = fmaf(a, d1, gw3[j][1]);
+        const float dz = z > 0.f ? fmaf(w30[j], d0, w31[j] * d1) : 0.f;
+        v[r][j] = dz;
+        gb2[j] += dz;
+      }
     }
-    if (threadIdx.x == 0)
-      for (int r = 0; r < TILE; r++) lsum += sloss[r];
+    put4x4(v, S.dz2, S.dz2t, tx, ty);
     __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[r][j] = 0.f;
+    tile4x4<NH>(&S.dz2t[0][0], &S.w2t[0][0], tx, ty, v);
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        v[r][j] = h1[r][j] > 0.f ? v[r][j] : 0.f;
+        gb1[j] += v[r][j];
+      }
+    put4x4(v, S.dz1, nullptr, tx, ty);
+    __syncthreads();
+    // outer products over the tile's samples
+#pragma unroll 4
+    for (int r = 0; r < TILE; r++) {
+      const float4 a = *reinterpret_cast<const float4*>(&S.h1[r][4 * ty]);
+      const float4 b = *reinterpret_cast<const float4*>(&S.dz2[r][4 * tx]);
+      const float4 c = *reinterpret_cast<const float4*>(&S.dz1[r][4 * tx]);
+      const float xi = S.x[r][ty];
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w}, cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) gw2[i][j] = fmaf(av[i], bv[j], gw2[i][j]);
+        gw1[i] = fmaf(xi, cv[i], gw1[i]);
+      }
+    }
   }
-  for (int q = 0; q < (NPARAM + 255) / 256; q++) {
-    const int pidx = threadIdx.x + q * 256;
-    if (pidx < NPARAM) atomicAdd(&grad[pidx], g[q]);
+  static_assert(NIN == 16 && NH == 64 && NOUT == 2, "thread layout");
+  add4(out + OFF_W1 + ty * NH + 4 * tx, gw1[0], gw1[1], gw1[2], gw1[3]);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    add4(out + OFF_W2 + (4 * ty + i) * NH + 4 * tx, gw2[i][0], gw2[i][1], gw2[i][2], gw2[i][3]);
+  // the sums over samples: per group, then over the groups
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const int u = 4 * tx + j;
+    S.red[ty][u] = gb1[j];
+    S.red[ty][NH + u] = gb2[j];
+    S.red[ty][2 * NH + NOUT * u] = gw3[j][0];
+    S.red[ty][2 * NH + NOUT * u + 1] = gw3[j][1];
   }
-  if (threadIdx.x == 0) atomicAdd(loss, lsum * inv_n);
+  if (tx == 0) {
+    S.red[ty][4 * NH] = gb3[0];
+    S.red[ty][4 * NH + 1] = gb3[1];
+    S.red[ty][4 * NH + 2] = lsum;
+  }
+  __syncthreads();
+  for (int i = tid; i < 4 * NH + 3; i += 256) {
+    float sum = 0.f;
+#pragma unroll
+    for (int g = 0; g < 16; g++) sum += S.red[g][i];
+    if (i < NH) atomicAdd(out + OFF_B1 + i, sum);
+    else if (i < 2 * NH) atomicAdd(out + OFF_B2 + i - NH, sum);
+    else if (i < 4 * NH) atomicAdd(out + OFF_W3 + i - 2 * NH, sum);
+    else if (i < 4 * NH + 2) atomicAdd(out + OFF_B3 + i - 4 * NH, sum);
+    else atomicAdd(out + NPARAM, sum * inv_n);
+  }
 }
 
 // ---------------------------------------------------------------- Adam
@@ -319,10 +503,10 @@ struct pm_mlp {
   int device = 0;
   float* w = nullptr;            // FP32 master weights
   __nv_bfloat16* wq = nullptr;   // BF16 copy used by forward/backward
-  float* g = nullptr;
+  float* g = nullptr;            // gradients, then the loss
   float* m = nullptr;
   float* v = nullptr;
-  float* loss = nullptr;
+  float h_out[NPARAM + 1];       // gradients and loss on their way to the caller
   int64_t step = 0;
   int nsm = 148;
 };
@@ -331,11 +515,6 @@ extern "C" void pm_mlp_free(pm_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
   cudaFree(m->w);
-  cudaFree(m->wq);
-  cudaFree(m->g);
-  cudaFree(m->m);
-  cudaFree(m->v);
-  cudaFree(m->loss);
   delete m;
 }
 
@@ -348,12 +527,12 @@ extern "C" pm_status pm_mlp_create(int device, uint64_t seed, pm_mlp** out) {
   std::unique_ptr<pm_mlp, void (*)(pm_mlp*)> m(new pm_mlp, pm_mlp_free);
   m->device = device;
   CKL(cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, device));
-  CKL(cudaMalloc(&m->w, sizeof(float) * NPARAM));
-  CKL(cudaMalloc(&m->wq, sizeof(__nv_bfloat16) * NPARAM));
-  CKL(cudaMalloc(&m->g, sizeof(float) * NPARAM));
-  CKL(cudaMalloc(&m->m, sizeof(float) * NPARAM));
-  CKL(cudaMalloc(&m->v, sizeof(float) * NPARAM));
-  CKL(cudaMalloc(&m->loss, sizeof(float)));
+  constexpr size_t kPart = (sizeof(float) * (NPARAM + 1) + 255) & ~(size_t)255;
+  CKL(cudaMalloc(&m->w, 5 * kPart));  // one allocation, five 256-byte aligned parts
+  m->g = reinterpret_cast<float*>(reinterpret_cast<char*>(m->w) + kPart);
+  m->m = reinterpret_cast<float*>(reinterpret_cast<char*>(m->w) + 2 * kPart);
+  m->v = reinterpret_cast<float*>(reinterpret_cast<char*>(m->w) + 3 * kPart);
+  m->wq = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(m->w) + 4 * kPart);
   // He-uniform init from the seed (host side, deterministic)
   std::vector<float> h(NPARAM, 0.f);
   Rng r(seed, 77);
@@ -365,8 +544,7 @@ extern "C" pm_status pm_mlp_create(int device, uint64_t seed, pm_mlp** out) {
   fill(OFF_W2, NH, NH * NH);
   fill(OFF_W3, NH, NH * NOUT);
   CKL(cudaMemcpy(m->w, h.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
-  CKL(cudaMemset(m->m, 0, sizeof(float) * NPARAM));
-  CKL(cudaMemset(m->v, 0, sizeof(float) * NPARAM));
+  CKL(cudaMemset(m->m, 0, 2 * kPart));  // and v after it
   PM_CK_PENDING("pm_mlp_create");
   quantize_kernel<<<(NPARAM + 255) / 256, 256>>>(m->w, m->wq);
   CKL(cudaGetLastError());
@@ -400,9 +578,10 @@ extern "C" pm_status pm_mlp_forward(pm_mlp* m, const float* d_x, int64_t n, floa
   if (!m || (n > 0 && (!d_x || !d_y))) return fail(PM_ERR_INVALID, "pm_mlp_forward: bad arguments");
   CKL(cudaSetDevice(m->device));
   if (n == 0) return PM_OK;
-  const int blocks = (int)std::min<int64_t>((n + 127) / 128, 8 * m->nsm);
+  const int blocks = (int)std::min<int64_t>((n + FT - 1) / FT, 3 * m->nsm);  // three fit an SM
   PM_CK_PENDING("MLP kernels");
-  mlp_forward_kernel<<<blocks, 128>>>(m->wq, d_x, n, d_y);
+  CKL(cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ForwardSmem)));
+  mlp_forward_kernel<<<blocks, 256, sizeof(ForwardSmem)>>>(m->wq, d_x, n, d_y);
   CKL(cudaGetLastError());
   CKL(cudaDeviceSynchronize());
   return PM_OK;
@@ -412,17 +591,18 @@ extern "C" pm_status pm_mlp_gradient(pm_mlp* m, const float* d_x, const float* d
                                      float* loss_out) {
   if (!m || n <= 0 || !d_x || !d_t) return fail(PM_ERR_INVALID, "pm_mlp_gradient: bad arguments");
   CKL(cudaSetDevice(m->device));
-  CKL(cudaMemset(m->g, 0, sizeof(float) * NPARAM));
-  CKL(cudaMemset(m->loss, 0, sizeof(float)));
-  const int blocks = (int)std::min<int64_t>((n + TILE - 1) / TILE, 2 * m->nsm);
+  CKL(cudaMemsetAsync(m->g, 0, sizeof(float) * (NPARAM + 1)));
+  const int blocks = (int)std::min<int64_t>((n + TILE - 1) / TILE, m->nsm);
+  PM_CK_PENDING("MLP kernels");
   CKL(cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sizeof(BackwardSmem)));
-  PM_CK_PENDING("MLP kernels");
-  mlp_backward_kernel<<<blocks, 256, sizeof(BackwardSmem)>>>(m->wq, d_x, d_t, n, m->g, m->loss);
+  mlp_backward_kernel<<<blocks, 256, sizeof(BackwardSmem)>>>(m->wq, d_x, d_t, n, m->g);
   CKL(cudaGetLastError());
-  if (host_grad) CKL(cudaMemcpy(host_grad, m->g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
-  if (loss_out) CKL(cudaMemcpy(loss_out, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
-  CKL(cudaDeviceSynchronize());
+  // one copy (which waits for the kernel): the gradients when asked for, and the loss
+  const int first = host_grad ? 0 : NPARAM;
+  CKL(cudaMemcpy(m->h_out + first, m->g + first, sizeof(float) * (NPARAM + 1 - first), cudaMemcpyDeviceToHost));
+  if (host_grad) memcpy(host_grad, m->h_out, sizeof(float) * NPARAM);
+  if (loss_out) *loss_out = m->h_out[NPARAM];
   return PM_OK;
 }
 
