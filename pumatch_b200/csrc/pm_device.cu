@@ -2899,75 +2899,134 @@ __device__ __forceinline__ unsigned long long pair_hash(unsigned lo, unsigned hi
   return Rng::splitmix(x);
 }
 
-__global__ void maxnbrdeg_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n, int32_t* out,
-                                 unsigned long long* asym) {
+__global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n,
+                                                        int32_t* out, unsigned long long* asym) {
+  __shared__ int best[kListWarps];
   const int lane = lane_id();
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long sum = 0;
-  for (long long v = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
-    const uint64_t b = rowptr[v], e = rowptr[v + 1];
+  auto walk = [&](long long v, uint64_t b, uint64_t e) {
     int m = 0;
-    for (uint64_t i = b + lane; i < e; i += 32) {
-      const int u = colidx[i];
-      m = max(m, (int)(rowptr[u + 1] - rowptr[u]));
-      if (u > v) sum += pair_hash((unsigned)v, (unsigned)u);
-      else if (u < v) sum -= pair_hash((unsigned)u, (unsigned)v);
+    for (uint64_t i0 = b; i0 < e; i0 += 128) {
+      int u[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) u[q] = i0 + 32 * q + lane < e ? colidx[i0 + 32 * q + lane] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (u[q] < 0) continue;
+        m = max(m, (int)(rowptr[u[q] + 1] - rowptr[u[q]]));
+        if (u[q] > v) sum += pair_hash((unsigned)v, (unsigned)u[q]);
+        else if (u[q] < v) sum -= pair_hash((unsigned)u[q], (unsigned)v);
+      }
     }
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
-    if (lane == 0) out[v] = m;
-  }
+    return __reduce_max_sync(FULL, m);
+  };
+  for_lists(rowptr, 0, n,
+            [&](long long v, uint64_t b, uint64_t e) {
+              const int m = walk(v, b, e);
+              if (lane == 0) out[v] = m;
+            },
+            [&](long long v, uint64_t, uint64_t, uint64_t b0, uint64_t e0, int k) {
+              const int m = walk(v, b0, e0);
+              if (lane == 0) best[k] = m;
+              __syncthreads();
+              if (threadIdx.x < 32) {
+                const int top = __reduce_max_sync(FULL, lane < kListWarps ? best[lane] : 0);
+                if (lane == 0) out[v] = top;
+              }
+              __syncthreads();
+            });
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
   if (lane == 0 && sum) atomicAdd(asym, sum);
 }
 
 // Regroups each list by label, keeping id order within a label (a stable
-// partition): one warp per vertex, ranks from __match_any_sync.  Vertices
-// [v_begin, v_end); entry i of the adjacency array lands at out[i - out_base].
-__global__ void label_group_kernel(const uint64_t* rowptr, const int32_t* colidx, const uint8_t* labels,
-                                   int64_t v_begin, int64_t v_end, int nl1, int32_t* out, uint64_t out_base,
-                                   int32_t* off) {
-  __shared__ int base_s[16][33];
+// partition), ranks from __match_any_sync; a long list's warps count the
+// labels of their parts first.  Vertices [v_begin, v_end); entry i of the
+// adjacency array lands at out[i - out_base].
+__global__ void __launch_bounds__(512) label_group_kernel(const uint64_t* rowptr, const int32_t* colidx,
+                                                          const uint8_t* labels, int64_t v_begin, int64_t v_end,
+                                                          int nl1, int32_t* out, uint64_t out_base, int32_t* off) {
+  __shared__ int base_s[kListWarps][33];
   const int lane = lane_id();
   const int wib = threadIdx.x >> 5;
   int* base = base_s[wib];
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long v = v_begin + (long long)blockIdx.x * (blockDim.x >> 5) + wib; v < v_end; v += warps) {
-    const uint64_t b = rowptr[v], e = rowptr[v + 1];
-    // per-label counts: lane l counts label l
-    int mine = 0;
-    for (uint64_t i0 = b; i0 < e; i0 += 32) {
-      const uint64_t i = i0 + lane;
-      const int lb = i < e ? labels[colidx[i]] : -1;
-      for (int l = 0; l < nl1 - 1; l++) {
-        const unsigned bal = __ballot_sync(FULL, lb == l);
-        if (lane == l) mine += __popc(bal);
-      }
+  // entries of each label in [b, e) into base[]
+  auto count = [&](uint64_t b, uint64_t e) {
+    base[lane] = 0;
+    __syncwarp();
+    for (uint64_t i0 = b; i0 < e; i0 += 128) {
+      int x[4], lb[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) x[q] = i0 + 32 * q + lane < e ? colidx[i0 + 32 * q + lane] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; q++) lb[q] = x[q] >= 0 ? (int)labels[x[q]] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if ((unsigned)lb[q] < 32u) atomicAdd(&base[lb[q]], 1);
     }
-    // exclusive scan over labels
+    __syncwarp();
+  };
+  auto scan = [&](int mine) {  // exclusive sum over the lanes
     int incl = mine;
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(FULL, incl, o);
       if (lane >= o) incl += t;
     }
-    const int excl = incl - mine;
-    if (lane < nl1 - 1) {
-      off[v * nl1 + lane] = excl;
-      base[lane] = excl;
+    return incl - mine;
+  };
+  // entries [b, e) to their places, base[] the next place of each label in the list at b_list
+  auto place = [&](uint64_t b_list, uint64_t b, uint64_t e) {
+    for (uint64_t i0 = b; i0 < e; i0 += 128) {
+      int x[4], lb[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) x[q] = i0 + 32 * q + lane < e ? colidx[i0 + 32 * q + lane] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        lb[q] = x[q] >= 0 ? (int)labels[x[q]] : 32 + lane;  // none: matches only itself
+        if (lb[q] >= 32) x[q] = -1;                         // (no such label is accepted)
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const unsigned same = __match_any_sync(FULL, lb[q]);
+        if (x[q] >= 0) out[b_list - out_base + base[lb[q]] + __popc(same & lanemask_lt())] = x[q];
+        __syncwarp();
+        if (x[q] >= 0 && (same & lanemask_lt()) == 0) base[lb[q]] += __popc(same);
+        __syncwarp();
+      }
     }
+  };
+  auto offsets = [&](long long v, uint64_t b, uint64_t e, int excl) {
+    if (lane < nl1 - 1) off[v * nl1 + lane] = excl;
     if (lane == 0) off[v * nl1 + nl1 - 1] = (int)(e - b);  // up to 32 labels: entry 32 needs its own store
-    __syncwarp();
-    for (uint64_t i0 = b; i0 < e; i0 += 32) {
-      const uint64_t i = i0 + lane;
-      const bool valid = i < e;
-      const int x = valid ? colidx[i] : 0;
-      const int lb = valid ? (int)labels[x] : 32 + lane;  // invalid lanes match only themselves
-      const unsigned same = __match_any_sync(FULL, lb);
-      if (valid) out[b - out_base + base[lb] + __popc(same & lanemask_lt())] = x;
-      __syncwarp();
-      if (valid && (same & lanemask_lt()) == 0) base[lb] += __popc(same);
-      __syncwarp();
-    }
-  }
+  };
+  for_lists(rowptr, v_begin, v_end,
+            [&](long long v, uint64_t b, uint64_t e) {
+              count(b, e);
+              const int excl = scan(base[lane]);
+              offsets(v, b, e, excl);
+              __syncwarp();
+              base[lane] = excl;
+              __syncwarp();
+              place(b, b, e);
+            },
+            [&](long long v, uint64_t b, uint64_t e, uint64_t b0, uint64_t e0, int k) {
+              count(b0, e0);
+              __syncthreads();
+              if (wib == 0) {  // lane l: label l's entries in the parts before each part
+                int mine = 0;
+                for (int w = 0; w < kListWarps; w++) {
+                  const int c = base_s[w][lane];
+                  base_s[w][lane] = mine;
+                  mine += c;
+                }
+                const int excl = scan(mine);
+                offsets(v, b, e, excl);
+                for (int w = 0; w < kListWarps; w++) base_s[w][lane] += excl;
+              }
+              __syncthreads();
+              place(b, b0, e0);
+              __syncthreads();
+            });
 }
 
 // Vertices per power of two of their degree (bin k: degree in [2^k, 2^(k+1))).
@@ -2984,24 +3043,38 @@ __global__ void degree_bins_kernel(const uint64_t* rowptr, int64_t n, unsigned i
 }
 
 // Gives every vertex of at least min_deg neighbours a bit row and fills it
-// (rows zeroed before), one warp per vertex.
-__global__ void hub_rows_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n, int min_deg, int64_t words,
-                                unsigned int* next, int32_t* slot, unsigned int* bits) {
+// (rows zeroed before).
+__global__ void __launch_bounds__(512) hub_rows_kernel(const uint64_t* rowptr, const int32_t* colidx, int64_t n,
+                                                       int min_deg, int64_t words, unsigned int* next, int32_t* slot,
+                                                       unsigned int* bits) {
+  __shared__ int row;
   const int lane = lane_id();
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long v = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
-    const uint64_t b = rowptr[v], e = rowptr[v + 1];
-    int k = -1;
-    if ((long long)(e - b) >= min_deg) {
-      if (lane == 0) k = (int)atomicAdd(next, 1u);
-      k = __shfl_sync(FULL, k, 0);
-      for (uint64_t i = b + lane; i < e; i += 32) {
-        const int u = colidx[i];
-        if (u >= 0 && u < n) atomicOr(&bits[k * words + (u >> 5)], 1u << (u & 31));
-      }
+  auto fill = [&](int k, uint64_t b, uint64_t e) {
+    for (uint64_t i = b + lane; i < e; i += 32) {
+      const int u = colidx[i];
+      if (u >= 0 && u < n) atomicOr(&bits[k * words + (u >> 5)], 1u << (u & 31));
     }
-    if (lane == 0) slot[v] = k;
-  }
+  };
+  for_lists(rowptr, 0, n,
+            [&](long long v, uint64_t b, uint64_t e) {
+              int k = -1;
+              if ((long long)(e - b) >= min_deg) {
+                if (lane == 0) k = (int)atomicAdd(next, 1u);
+                k = __shfl_sync(FULL, k, 0);
+                fill(k, b, e);
+              }
+              if (lane == 0) slot[v] = k;
+            },
+            [&](long long v, uint64_t b, uint64_t e, uint64_t b0, uint64_t e0, int) {
+              const bool has = (long long)(e - b) >= min_deg;
+              if (threadIdx.x == 0) {
+                row = has ? (int)atomicAdd(next, 1u) : -1;
+                slot[v] = row;
+              }
+              __syncthreads();
+              if (has) fill(row, b0, e0);
+              __syncthreads();
+            });
 }
 
 struct RootFilter {
@@ -3012,32 +3085,63 @@ struct RootFilter {
 };
 
 template <bool WRITE>
-__global__ void roots_kernel(const uint64_t* rowptr, const int32_t* colidx, const uint8_t* labels,
-                             const int32_t* maxnbrdeg, int64_t n, RootFilter f, int32_t* counts,
-                             const int64_t* offsets, int2* out) {
+__global__ void __launch_bounds__(512) roots_kernel(const uint64_t* rowptr, const int32_t* colidx,
+                                                    const uint8_t* labels, const int32_t* maxnbrdeg, int64_t n,
+                                                    RootFilter f, int32_t* counts, const int64_t* offsets, int2* out) {
+  __shared__ int part_total[kListWarps];
   const int lane = lane_id();
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
-    const uint64_t b = rowptr[r], e = rowptr[r + 1];
+  // root edges (r, c) for c in [b, e): counted, or written from out[base] on
+  auto filter = [&](long long r, uint64_t b, uint64_t e, bool write, long long base) {
     int total = 0;
-    const bool rok = (long long)(e - b) >= f.d0 && (!f.labeled || labels[r] == f.lab0);
-    if (rok) {
-      long long base = WRITE ? offsets[r] : 0;
-      for (uint64_t i0 = b; i0 < e; i0 += 32) {
-        const uint64_t i = i0 + lane;
-        bool keep = false;
-        if (i < e) {
-          const int c = colidx[i];
-          keep = (!f.need_gt || r > c) && (!f.labeled || labels[c] == f.lab1) &&
-                 (int)(rowptr[c + 1] - rowptr[c]) >= f.d1 && maxnbrdeg[c] >= f.d2;
-        }
-        const unsigned bal = __ballot_sync(FULL, keep);
-        if (WRITE && keep) out[base + total + __popc(bal & lanemask_lt())] = make_int2((int)r, colidx[i]);
+    for (uint64_t i0 = b; i0 < e; i0 += 128) {
+      int c[4];
+      bool keep[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        c[q] = i0 + 32 * q + lane < e ? colidx[i0 + 32 * q + lane] : -1;
+        keep[q] = c[q] >= 0 && (!f.need_gt || r > c[q]);
+      }
+      if (f.labeled) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) keep[q] = keep[q] && labels[c[q]] == f.lab1;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        keep[q] = keep[q] && (int)(rowptr[c[q] + 1] - rowptr[c[q]]) >= f.d1 && maxnbrdeg[c[q]] >= f.d2;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const unsigned bal = __ballot_sync(FULL, keep[q]);
+        if (write && keep[q]) out[base + total + __popc(bal & lanemask_lt())] = make_int2((int)r, c[q]);
         total += __popc(bal);
       }
     }
-    if (!WRITE && lane == 0) counts[r] = total;
-  }
+    return total;
+  };
+  auto root_ok = [&](long long r, uint64_t b, uint64_t e) {
+    return (long long)(e - b) >= f.d0 && (!f.labeled || labels[r] == f.lab0);
+  };
+  for_lists(rowptr, 0, n,
+            [&](long long r, uint64_t b, uint64_t e) {
+              const int total = root_ok(r, b, e) ? filter(r, b, e, WRITE, WRITE ? offsets[r] : 0) : 0;
+              if (!WRITE && lane == 0) counts[r] = total;
+            },
+            [&](long long r, uint64_t b, uint64_t e, uint64_t b0, uint64_t e0, int k) {
+              if (!root_ok(r, b, e)) {
+                if (!WRITE && threadIdx.x == 0) counts[r] = 0;
+                return;  // the same for all of the block
+              }
+              const int mine = filter(r, b0, e0, false, 0);
+              if (lane == 0) part_total[k] = mine;
+              __syncthreads();
+              int before = 0, all = 0;
+              for (int w = 0; w < kListWarps; w++) {
+                if (w < k) before += part_total[w];
+                all += part_total[w];
+              }
+              if (WRITE) filter(r, b0, e0, true, offsets[r] + before);
+              else if (threadIdx.x == 0) counts[r] = all;
+              __syncthreads();
+            });
 }
 
 // =====================================================================
@@ -3227,7 +3331,7 @@ pm_status compute_maxnbrdeg(pm_graph* g, const int32_t* colidx) {
   if (g->n > 0) {
     PM_CK_PENDING("max neighbour degree");
     CK(cudaMemset(asym_word(g), 0, 8));
-    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, colidx, g->n, g->d_maxnbrdeg, asym_word(g));
+    maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
   }
@@ -3242,7 +3346,7 @@ static pm_status graph_finish(pm_graph* g) {
   if (g->n > 0 && g->residency == PM_RESIDENT_HBM) {
     PM_CK_PENDING("max neighbour degree");
     CK(cudaMemset(asym_word(g), 0, 8));
-    maxnbrdeg_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
+    maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
   }
@@ -3270,7 +3374,7 @@ static pm_status graph_finish(pm_graph* g) {
       if (e == cudaSuccess) e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
       if (e == cudaSuccess) e = cudaMemset(g->d_hub_bits, 0, rows * words * 4);
       if (e == cudaSuccess) {
-        hub_rows_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->n, 1 << k, words, bins + 32, g->d_hub_slot,
+        hub_rows_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, 1 << k, words, bins + 32, g->d_hub_slot,
                                        g->d_hub_bits);
         e = cudaGetLastError();
       }
@@ -3286,7 +3390,7 @@ static pm_status graph_finish(pm_graph* g) {
     CK(cudaMalloc(&g->d_lab_off, sizeof(int32_t) * (size_t)g->n * g->nl1));
     g->device_bytes += sizeof(int32_t) * ((size_t)g->nadj + (size_t)g->n * g->nl1);
     PM_CK_PENDING("label grouping");
-    label_group_kernel<<<2048, 256>>>(g->d_rowptr, g->d_colidx, g->d_labels, 0, g->n, g->nl1, g->d_colidx_lab, 0,
+    label_group_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->d_labels, 0, g->n, g->nl1, g->d_colidx_lab, 0,
                                       g->d_lab_off);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
@@ -3318,7 +3422,7 @@ static pm_status paged_group_labels(pm_graph* g, const uint64_t* h_rowptr, bool 
     int64_t v1 = v0;
     while (v1 < g->n && (int64_t)(h_rowptr[v1 + 1] - h_rowptr[v0]) <= chunk) v1++;
     const uint64_t b0 = h_rowptr[v0], len = h_rowptr[v1] - b0;
-    label_group_kernel<<<2048, 256>>>(g->d_rowptr, g->h_colidx_dev, g->d_labels, v0, v1, g->nl1, tmp, b0,
+    label_group_kernel<<<list_blocks(v1 - v0), 512>>>(g->d_rowptr, g->h_colidx_dev, g->d_labels, v0, v1, g->nl1, tmp, b0,
                                       g->d_lab_off);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && len && keep_copy)
@@ -3560,6 +3664,7 @@ extern "C" void pm_ctx_destroy(pm_ctx* c) {
   free_dev(c->d_ctl);
   if (c->memo) free_dev(c->memo->d);
   delete c->memo;
+  free_dev(c->d_feat);
   free_dev(c->d_roots);
   free_dev(c->d_tmp);
   free_dev(c->d_vcount);
@@ -3597,7 +3702,7 @@ static pm_status build_roots(pm_ctx* c, const pm_graph* g, const Plan& p, size_t
   const RootFilter f = to_filter(p);
   const int32_t* colidx = g->residency == PM_RESIDENT_HBM ? g->d_colidx : g->h_colidx_dev;
   PM_CK_PENDING("root filter");
-  roots_kernel<false><<<4 * c->nsm, 256, 0, c->stream>>>(g->d_rowptr, colidx, g->d_labels, g->d_maxnbrdeg, n, f,
+  roots_kernel<false><<<list_blocks(n), 512, 0, c->stream>>>(g->d_rowptr, colidx, g->d_labels, g->d_maxnbrdeg, n, f,
                                                           c->d_vcount, nullptr, nullptr);
   CK(cudaGetLastError());
   CK(cudaMemsetAsync(c->d_vcount + n, 0, sizeof(int32_t), c->stream));
@@ -3624,7 +3729,7 @@ static pm_status build_roots(pm_ctx* c, const pm_graph* g, const Plan& p, size_t
     *roots_bytes = want + want / 4;
   }
   PM_CK_PENDING("root filter");
-  roots_kernel<true><<<4 * c->nsm, 256, 0, c->stream>>>(g->d_rowptr, colidx, g->d_labels, g->d_maxnbrdeg, n, f,
+  roots_kernel<true><<<list_blocks(n), 512, 0, c->stream>>>(g->d_rowptr, colidx, g->d_labels, g->d_maxnbrdeg, n, f,
                                                          nullptr, c->d_voff, *roots_buf + offset_roots);
   CK(cudaGetLastError());
   return PM_OK;
