@@ -46,7 +46,8 @@ struct DPlan {
   uint8_t clique;                 // the plan is an unlabeled clique's (clique_bits)
   uint8_t pair;                   // PairKind of the last two levels (pair_levels), 0: none
   int8_t pair_h0;                 // the slot its copy or meeting reads
-  int8_t pad_[2];
+  uint8_t copy_next;              // labeled: bit L: level L+1 is all copies (one candidate searched for all)
+  int8_t pad_[1];
   uint8_t hole_ok[16];            // 1: the slot may be read in place, path vertices skipped by its walker
   const int2* roots;              // (v0, v1) root edges, reference order (the whole list)
   int64_t nroots;                 // positions this launch processes

@@ -95,3 +95,27 @@ def test_one_context_many_graphs(ctx):
     for seed, shape, wpb in ((1, "C5", 8), (2, "C5", 8), (1, "C6", 4), (3, "C5", 16), (1, "C5", 8)):
         hg = pm.gen_chung_lu(100 + 30 * seed, 400, seed=seed)
         same(*runs(ctx, hg, shape, None, warps_per_block=wpb))
+
+
+@pytest.mark.parametrize("shape", [P.star(6), P.star(7), P.house_tail(1), P.house_tail(2)])
+@pytest.mark.parametrize("truncate,paged", [(0, False), (4, False), (0, True)])
+def test_levels_of_copies(ctx, shape, truncate, paged):
+    """One candidate searched for all where the next level only copies: against the oracle, also when pieces of the
+    search change hands."""
+    import os
+    import sys
+    sys.path.insert(0, os.path.join(os.path.dirname(__file__), "..", "oracle"))
+    import pm_oracle as orc
+    hg = pm.gen_rmat(300, 1500, seed=2)
+    hg = pm.HostGraph(hg.rowptr, hg.colidx, pm.gen_labels(hg.n, 3, 4))
+    k, e = shape
+    text = P.to_g(k, e, P.seeded_labels(k, 3, 8))
+    og, op = orc.Graph(hg.rowptr, hg.colidx, hg.labels), orc.plan(text, True)
+    want, st0 = orc.count(og, op, orc.roots(og, op), truncate=truncate)
+    kw = dict(paged=True, page_bytes=4096, frame_pool_bytes=64 << 10) if paged else {}
+    g = pm.GraphPreprocessor.from_host(hg, labeled=True, **kw)
+    p = pm.PatternPreprocessor(text=text, labeled=True)
+    for split in (0, 2, -1):
+        c, st = ctx.match(g, [p], truncate=truncate, split_level1=split, timeout_ms=60000)
+        assert (c[0], st["set_ops"], st["alg_bytes"]) == (want, st0["set_ops"], st0["alg_bytes"])
+    g.close()
