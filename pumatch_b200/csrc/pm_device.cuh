@@ -47,8 +47,9 @@ struct DPlan {
   uint8_t pair;                   // PairKind of the last two levels (pair_levels), 0: none
   int8_t pair_h0;                 // the slot its copy or meeting reads
   uint8_t copy_next;              // labeled: bit L: level L+1 is all copies (one candidate searched for all)
-  int8_t pad_[1];
-  uint8_t hole_ok[16];            // 1: the slot may be read in place, path vertices skipped by its walker
+  int8_t chain_from;              // labeled: first of the fresh levels the plan ends in, 0: none (chain_kernel)
+  uint8_t hole_ok[16];
+  const ulonglong4* chain;        // its table, by vertex (null: not used)            // 1: the slot may be read in place, path vertices skipped by its walker
   const int2* roots;              // (v0, v1) root edges, reference order (the whole list)
   int64_t nroots;                 // positions this launch processes
   int64_t rbase;                  // first position: root_begin (0 = all)
@@ -213,6 +214,8 @@ struct pm_ctx {
   int2* d_roots = nullptr;
   size_t roots_bytes = 0;
   MemoTables* memo = nullptr;  // the warps' value tables
+  void* d_chain = nullptr;     // chain tables
+  size_t chain_bytes = 0;
   void* d_feat = nullptr;      // root features: degree counts, per-vertex rows
   size_t feat_bytes = 0;
   void* d_tmp = nullptr;

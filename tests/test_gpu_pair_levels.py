@@ -10,7 +10,7 @@ from pumatch_b200 import patterns as P
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = {"C5": P.cycle(5), "C6": P.cycle(6), "C7": P.cycle(7), "P5": P.path(5), "P6": P.path(6), "house": P.house(),
+SHAPES = {"C5": P.cycle(5), "C6": P.cycle(6), "C7": P.cycle(7), "P4": P.path(4), "P5": P.path(5), "P6": P.path(6), "P7": P.path(7), "house": P.house(),
           "house_tail": P.house_tail(1), "house_tail2": P.house_tail(2), "C4_tail": P.cycle_tail(4, 1),
           "C4_tail2": P.cycle_tail(4, 2), "C5_tail2": P.cycle_tail(5, 2), "C6_tail": P.cycle_tail(6, 1),
           "S5": P.star(5)}
