@@ -211,6 +211,8 @@ struct alignas(16) WarpState {
   int32_t memo_len, memo_ub;
   int32_t queue[64];
   int32_t lcnt[32];
+  unsigned long long prb[32];    // the candidates' lists laid end to end: where each starts
+  int32_t pexcl[33];             // and its offset in the row
   long long next_check;          // SM clock at which to look for waiting warps and at the deadline
   long long began;               // SM clock at the start of the current root or piece
   int32_t checks;                // checks made (the heartbeat is bumped on every 16th)
@@ -1984,7 +1986,11 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
 //               values in a table of its own in device memory (MemoEntry),
 //               tagged with the number of the (h0, bound) they belong to.
 // So no slot of level q is built, and no call is made per candidate of level
-// q: elements come in tiles of 32 (one list each), four tiles in flight.
+// q: the lists of 32 candidates are laid end to end and their elements taken
+// 128 at a time, four per lane in flight (a tile per list left most lanes
+// without one: the 6-cycle's lists have about ten elements below their bound).
+// Each kind is a function of its own: what the loop waited for most was its
+// own instructions (no_instruction 9.2 of 25 stall cycles per issue).
 // Set operations, counts and accounting are those of run_level + leaf_batch.
 //
 // What bounded the search before was instructions, not bytes: about 1,400 per
@@ -2007,7 +2013,7 @@ struct PairSums {
 // label's part, are laid end to end and walked in equal parts, a part at a
 // time per lane, matches added to the owner's counter in shared memory.
 template <bool LABELED>
-__device__ __forceinline__ void meet_values(const MatchArgs& a, WarpState& S, const LeafSet& m, int mode, int group,
+__device__ __noinline__ void meet_values(const MatchArgs& a, WarpState& S, const LeafSet& m, int mode, int group,
                                             int ub, int count, PairSums& r) {
   const int lane = lane_id();
   const int32_t* lists = LABELED ? a.colidx_lab : a.colidx;
@@ -2090,15 +2096,15 @@ __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, c
 }
 
 // Candidates [b, e) (at most 32) of level L = n-4's main slot.
-template <bool LABELED, bool PAGED>
-__device__ __noinline__ unsigned long long pair_levels(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
-                                                       int e, Work* wt) {
+template <bool LABELED, bool PAGED, int KIND, bool MET>
+__device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
+                                                     int e, Work* wt) {
   Work& w = *wt;
   const int lane = lane_id();
   const int q = L + 1;
   const int ms = P.level_begin[q], last = P.last_slot;
-  const int kind = P.pair;
-  const bool meet_main = P.kind[ms] == SLOT_INTERSECT;
+  constexpr int kind = KIND;
+  constexpr bool meet_main = MET;  // the main slot is an intersection
   const int main_group = LABELED ? __ffs(P.slot_labels[ms]) - 1 : -1;
   const int last_group = LABELED ? __ffs(P.slot_labels[last]) - 1 : -1;
   // the parent a main intersection meets, and the set a copy or a meeting reads
@@ -2207,155 +2213,186 @@ __device__ __noinline__ unsigned long long pair_levels(const MatchArgs& a, const
       }
     }
   }
-  // walk: tiles of 32 elements of one list, four in flight
+  // walk
   int queued = 0;
-  unsigned left = __ballot_sync(FULL, len > 0);
-  int j = left ? __ffs(left) - 1 : 0, o = 0;
-  ListRef cur{nullptr, 0, -1};  // PAGED: the current candidate's resolved list
-  while (left) {
-    const int32_t* src[4];
-    int own[4], cnt4[4];
+  int total = len;
+  if (!PAGED) {
+    int incl = len;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, d);
+      if (lane >= d) incl += t;
+    }
+    total = __shfl_sync(FULL, incl, 31);
+    S.prb[lane] = rb;
+    S.pexcl[lane] = incl - len;
+    if (lane == 31) S.pexcl[32] = total;
+    __syncwarp();
+  }
+  const int32_t* lists = LABELED ? a.colidx_lab : a.colidx;
+  // (paged: one resolved list after the other)
+  for (unsigned left = PAGED ? __ballot_sync(FULL, len > 0) : 1u; left; left &= left - 1) {
+    const int one = PAGED ? __ffs(left) - 1 : 0;
+    ListRef cur{nullptr, 0, -1};
+    if (PAGED) {
+      total = __shfl_sync(FULL, len, one);
+      const unsigned long long base = __shfl_sync(FULL, rb, one);
+      if (!gather_room(a, S, S.top[q], total, w)) break;
+      cur = paged_list(a.pg, base, total, S.gather, S.pins, w.pc);
+    }
+    for (int t0 = 0; t0 < total; t0 += 128) {
+      int x[4], own[4];
+      bool in[4];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      src[t] = nullptr;
-      own[t] = 0;
-      cnt4[t] = 0;
-      if (!left) continue;
-      const int n = __shfl_sync(FULL, len, j);
-      const unsigned long long base = __shfl_sync(FULL, rb, j);
-      if (PAGED) {
-        if (t > 0 && o == 0) continue;  // one list at a time: the next one after this round's reads
-        if (o == 0) {
-          if (!gather_room(a, S, S.top[q], n, w)) { left = 0; continue; }
-          cur = paged_list(a.pg, base, n, S.gather, S.pins, w.pc);
+      for (int k = 0; k < 4; k++) {
+        const int t = t0 + 32 * k + lane;
+        in[k] = t < total;
+        if (PAGED) {
+          own[k] = one;
+          x[k] = in[k] ? ld<PAGED>(cur.p + t, cur.cg) : 0;
+        } else {
+          int j = 0;
+#pragma unroll
+          for (int step = 16; step; step >>= 1)
+            if (S.pexcl[j + step] <= t) j += step;
+          own[k] = j;
+          x[k] = in[k] ? __ldg(lists + S.prb[j] + (unsigned)(t - S.pexcl[j])) : 0;
         }
-        src[t] = cur.p + o;
-      } else {
-        src[t] = (LABELED ? a.colidx_lab : a.colidx) + base + o;
       }
-      own[t] = j;
-      cnt4[t] = min(32, n - o);
-      o += 32;
-      if (o >= n) {
-        left &= left - 1;
-        j = left ? __ffs(left) - 1 : 0;
-        o = 0;
-      }
-    }
-    int x[4];
-    bool in[4];
+      if (MET) {
+        if (mode == MEMB_BITMAP) {
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      in[t] = lane < cnt4[t];
-      x[t] = in[t] ? ld<PAGED>(src[t] + lane, cur.cg) : 0;
-    }
-    if (PAGED && o == 0) {
-      __syncwarp();
-      unpin(a.pg, cur);
-      cur.pinned = -1;
-    }
-    if (meet_main) {
+          for (int k = 0; k < 4; k++) in[k] = in[k] && leaf_maybe<MEMB_BITMAP>(set, x[k]);
+        } else {
 #pragma unroll
-      for (int t = 0; t < 4; t++)
-        in[t] = in[t] && (mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(set, x[t]) : leaf_member<MEMB_FILTER>(set, x[t]));
-    } else if (!LABELED) {
-      for (int k = 0; k <= L; k++) {
-        const int p = S.path[k];
-#pragma unroll
-        for (int t = 0; t < 4; t++) in[t] = in[t] && x[t] != p;
-      }
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int vo = __shfl_sync(FULL, v, own[t]);
-        in[t] = in[t] && x[t] != vo;
-      }
-    }
-    if (kind == PAIR_COPY) {
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int h = __shfl_sync(FULL, h_v, own[t]), vo = __shfl_sync(FULL, v, own[t]);
-        if (!in[t]) continue;
-        r.elems++;
-        const int f = LABELED ? h : h - (x[t] != vo && bsearch_in<false>(H0, len0, x[t]) ? 1 : 0);
-        r.cnt += (unsigned long long)f;
-        r.bytes += 4ull * (unsigned long long)(h + f) + (LABELED ? (unsigned long long)h : 0ull);
-      }
-    } else if (kind == PAIR_FRESH) {
-      int deg[4], f[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        deg[t] = f[t] = 0;
-        if (!in[t]) continue;
-        const uint64_t xb = a.rowptr[x[t]];
-        deg[t] = (int)(a.rowptr[x[t] + 1] - xb);
-        if (LABELED) {
-          f[t] = label_range(a, x[t], last_group).y;
-          if (a.T) f[t] = min(f[t], a.T);
+          for (int k = 0; k < 4; k++) in[k] = in[k] && leaf_maybe<MEMB_FILTER>(set, x[k]);
+          if (__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) bsearch4<false>(set.g, set.lenB, x, in, false);
         }
-        else if (ub_last != INT_MAX) deg[t] = lane_lower_bound(a.colidx + xb, deg[t], ub_last);
-      }
-      if (!LABELED) {
+      } else if (!LABELED) {
+        for (int i = 0; i <= L; i++) {
+          const int p = S.path[i];
 #pragma unroll
-        for (int t = 0; t < 4; t++) f[t] = deg[t] - known - (__shfl_sync(FULL, v, own[t]) < ub_last ? 1 : 0);
+          for (int k = 0; k < 4; k++) in[k] = in[k] && x[k] != p;
+        }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          if (k >= n_ask) continue;
-          if (prow[k]) {
+          const int vo = __shfl_sync(FULL, v, own[k]);
+          in[k] = in[k] && x[k] != vo;
+        }
+      }
+      if (MET && !__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) continue;
+      int n_el = 0;
 #pragma unroll
-            for (int t = 0; t < 4; t++)
-              if (in[t]) f[t] -= (__ldg(prow[k] + (x[t] >> 5)) >> (x[t] & 31)) & 1u;
-          } else {
-            const uint64_t pb = a.rowptr[pv[k]];
-            const int pn = (int)(a.rowptr[pv[k] + 1] - pb);
+      for (int k = 0; k < 4; k++) n_el += in[k] ? 1 : 0;
+      r.elems += (unsigned)n_el;
+      if (KIND == PAIR_COPY) {
+        bool hit[4];
+        int h[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          h[k] = __shfl_sync(FULL, h_v, own[k]);
+          hit[k] = false;
+          if (!LABELED) {
+            const int vo = __shfl_sync(FULL, v, own[k]);
+            hit[k] = in[k] && x[k] != vo;
+          }
+        }
+        if (!LABELED) bsearch4<false>(H0, len0, x, hit, false);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (!in[k]) continue;
+          const int f = h[k] - (hit[k] ? 1 : 0);
+          r.cnt += (unsigned)f;
+          r.bytes += 4ull * (unsigned)(h[k] + f) + (LABELED ? (unsigned)h[k] : 0u);
+        }
+      } else if (KIND == PAIR_FRESH) {
+        int deg[4], f[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          deg[k] = f[k] = 0;
+          if (!in[k]) continue;
+          const uint64_t xb = a.rowptr[x[k]];
+          deg[k] = (int)(a.rowptr[x[k] + 1] - xb);
+          if (LABELED) {
+            f[k] = label_range(a, x[k], last_group).y;
+            if (a.T) f[k] = min(f[k], a.T);
+          } else if (ub_last != INT_MAX) {
+            deg[k] = lane_lower_bound(a.colidx + xb, deg[k], ub_last);
+          }
+        }
+        if (!LABELED) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) f[k] = deg[k] - known - (__shfl_sync(FULL, v, own[k]) < ub_last ? 1 : 0);
+          for (int i = 0; i < n_ask; i++) {
+            const int p = i == 0 ? pv[0] : i == 1 ? pv[1] : i == 2 ? pv[2] : pv[3];
+            const unsigned* row = i == 0 ? prow[0] : i == 1 ? prow[1] : i == 2 ? prow[2] : prow[3];
             bool hit[4];
 #pragma unroll
-            for (int t = 0; t < 4; t++) hit[t] = in[t];
-            bsearch4<false>(a.colidx + pb, pn, x, hit, false);
+            for (int k = 0; k < 4; k++) hit[k] = in[k];
+            if (row) {
 #pragma unroll
-            for (int t = 0; t < 4; t++) f[t] -= hit[t] ? 1 : 0;
+              for (int k = 0; k < 4; k++) hit[k] = in[k] && ((__ldg(row + (x[k] >> 5)) >> (x[k] & 31)) & 1u);
+            } else {
+              const uint64_t pb = a.rowptr[p];
+              bsearch4<false>(a.colidx + pb, (int)(a.rowptr[p + 1] - pb), x, hit, false);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) f[k] -= hit[k] ? 1 : 0;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (!in[k]) continue;
+          r.cnt += (unsigned)f[k];
+          r.bytes += 4ull * (unsigned)(deg[k] + f[k]) + (LABELED ? (unsigned)deg[k] : 0u);
+        }
+      } else {
+        int4 en[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          en[k] = in[k] ? *reinterpret_cast<const int4*>(S.memo + (x[k] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
+        int c = 0, by = 0, lw = 0;  // this round's sums (lists are shorter than 2^28)
+        unsigned missing = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int h = __shfl_sync(FULL, h_v, own[k]), l1 = LABELED ? 0 : __shfl_sync(FULL, less, own[k]);
+          const bool hit = in[k] && en[k].x == x[k] && (unsigned)en[k].y == epoch;
+          if (in[k]) {
+            c -= l1;
+            by += h - l1;
+          }
+          if (hit) {
+            c += en[k].z;
+            by += en[k].w + en[k].z;
+            lw += en[k].w;
+          }
+          missing |= in[k] && !hit ? 1u << k : 0u;
+        }
+        r.cnt += (unsigned long long)(long long)c;
+        r.bytes += (unsigned long long)(4ll * by + (LABELED ? lw : 0));
+        if (__any_sync(FULL, missing)) {
+          for (int k = 0; k < 4; k++) {
+            const bool mk = (missing >> k) & 1u;
+            const unsigned miss = __ballot_sync(FULL, mk);
+            if (!miss) continue;
+            const int xk = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
+            if (mk) S.queue[queued + __popc(miss & lanemask_lt())] = xk;
+            queued += __popc(miss);
+            __syncwarp();
+            if (queued >= 32) {
+              meet_values<LABELED>(a, S, set, mode, last_group, ub_last, 32, r);
+              const int rest = lane < queued - 32 ? S.queue[32 + lane] : 0;
+              __syncwarp();
+              queued -= 32;
+              if (lane < queued) S.queue[lane] = rest;
+              __syncwarp();
+            }
           }
         }
       }
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        if (!in[t]) continue;
-        r.elems++;
-        r.cnt += (unsigned long long)f[t];
-        r.bytes += 4ull * (unsigned long long)(deg[t] + f[t]) + (LABELED ? (unsigned long long)deg[t] : 0ull);
-      }
-    } else {
-      int4 en[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        en[t] = in[t] ? *reinterpret_cast<const int4*>(S.memo + (x[t] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int h = __shfl_sync(FULL, h_v, own[t]), l1 = __shfl_sync(FULL, less, own[t]);
-        const bool hit = in[t] && en[t].x == x[t] && (unsigned)en[t].y == epoch;
-        if (in[t]) {  // what does not depend on the value
-          r.elems++;
-          r.cnt -= (unsigned long long)l1;
-          r.bytes += 4ull * (unsigned long long)(h - l1);
-        }
-        if (hit) {
-          r.cnt += (unsigned long long)en[t].z;
-          r.bytes += 4ull * (unsigned long long)(en[t].w + en[t].z) + (LABELED ? (unsigned long long)en[t].w : 0ull);
-        }
-        const unsigned miss = __ballot_sync(FULL, in[t] && !hit);
-        if (miss) {
-          if (in[t] && !hit) S.queue[queued + __popc(miss & lanemask_lt())] = x[t];
-          queued += __popc(miss);
-          __syncwarp();
-          if (queued >= 32) {
-            meet_values<LABELED>(a, S, set, mode, last_group, ub_last, 32, r);
-            const int rest = lane < queued - 32 ? S.queue[32 + lane] : 0;
-            __syncwarp();
-            queued -= 32;
-            if (lane < queued) S.queue[lane] = rest;
-            __syncwarp();
-          }
-        }
-      }
+    }
+    if (PAGED) {
+      __syncwarp();
+      unpin(a.pg, cur);
     }
   }
   if (queued) meet_values<LABELED>(a, S, set, mode, last_group, ub_last, queued, r);
@@ -2470,6 +2507,19 @@ __device__ __forceinline__ unsigned long long chain_sum(const DPlan& P, const in
   w.bytes += bytes;
   w.reads += reads;
   return cnt;
+}
+
+template <bool LABELED, bool PAGED>
+__device__ __forceinline__ unsigned long long pair_levels(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
+                                                          int b, int e, Work* w) {
+  const bool met = P.kind[P.level_begin[L + 1]] == SLOT_INTERSECT;
+  if constexpr (!PAGED)
+    if (P.pair == PAIR_MEET) return pair_pass<LABELED, PAGED, PAIR_MEET, false>(a, P, S, L, b, e, w);
+  if (P.pair == PAIR_COPY)
+    return met ? pair_pass<LABELED, PAGED, PAIR_COPY, true>(a, P, S, L, b, e, w)
+               : pair_pass<LABELED, PAGED, PAIR_COPY, false>(a, P, S, L, b, e, w);
+  return met ? pair_pass<LABELED, PAGED, PAIR_FRESH, true>(a, P, S, L, b, e, w)
+             : pair_pass<LABELED, PAGED, PAIR_FRESH, false>(a, P, S, L, b, e, w);
 }
 
 // A donated piece of a DFS: candidates [begin, end) of level `level`'s main
