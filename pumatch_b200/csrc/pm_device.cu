@@ -141,15 +141,16 @@ struct MatchArgs {
   float* root_reads;
   const int32_t* root_order;
   const int32_t* root_split;      // optional per-root donation threshold of the last-but-one level (plan 0)
-  // work hand-off (publish_pieces, wait_piece): a warp out of work draws a
-  // ticket and waits on the ring slot of that number; a warp with work fills
-  // the oldest tickets' slots with (plan, root, level, begin, end,
-  // path[2..level])
+  // work hand-off (publish_pieces, wait_piece), in don_groups groups of blocks:
+  // a warp out of work draws a ticket of its group and waits on the group's
+  // ring slot of that number; a warp with work fills the oldest tickets' slots
+  // of a group with (plan, root, level, begin, end, path[2..level])
   int4* don_items;                // 3 int4 per slot
   unsigned long long* don_ready;  // per slot: 0 empty, ticket + 1 filled, kQuit no more work
-  unsigned long long* sched;      // (tickets drawn << 32) | pieces handed out
+  unsigned long long* sched;      // per group, kSchedStride apart: (tickets drawn << 32) | pieces handed out
+  unsigned long long* all_sched;  // the same over all groups
   unsigned int* started;          // warps that have begun
-  unsigned int don_mask;
+  unsigned int don_groups;        // a power of two; each has kGroupSlots slots
   unsigned int total_warps;
   unsigned long long* heartbeat;  // bumped by busy warps
   unsigned long long timeout_ns;  // hard limit on the launch; idle warps also give
@@ -2534,6 +2535,9 @@ struct Donation {
 // look costs one L2 read; a piece costs its taker the prefix again, so work
 // that ends sooner than this is not worth handing out.
 #define PM_CHECK_CYCLES 4096
+constexpr unsigned kGroupSlots = 256;   // ring slots of a group
+constexpr unsigned kSchedStride = 16;   // words from one group's sched to the next (a line of its own)
+#define PM_PAIR_PIECE 32  // shortest range of a two-level pass that is cut
 
 __device__ __forceinline__ unsigned long long ld_vol_u64(const unsigned long long* p) {
   return *(const volatile unsigned long long*)p;
@@ -2546,7 +2550,9 @@ __device__ __forceinline__ unsigned long long ld_vol_u64(const unsigned long lon
 // -- so handing out is one CAS by the donor and no contention among the
 // waiting (thousands of idle warps competing for one queue head by CAS cost
 // several microseconds a piece and held every query with few roots at 5 us
-// per donation).  With many waiting for each busy warp the range is cut into
+// per donation).  A donor looks at its own group's word, then at another's,
+// in turn: with one word for all warps 97% of the CAS failed (2.4 million on
+// the labeled 5-cycle with a tail, launch 9.1 -> 4.5 ms).  With many waiting for each busy warp the range is cut into
 // up to 33 pieces at once, one published per lane, so that a single heavy
 // root reaches all warps in two or three rounds.  A range whose candidates
 // head whole subtrees is long enough from 2 candidates on; one whose
@@ -2557,28 +2563,48 @@ __device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, const DPlan&
   const int n = P.nnodes;
   const int lane = lane_id();
   int k = L0, q = 0;
+  unsigned g = 0;
   unsigned long long first = 0;
   if (lane == 0) {
-    const unsigned long long cur = ld_vol_u64(a.sched);
-    const int waiting = (int)((unsigned)(cur >> 32) - (unsigned)cur);
+    const unsigned own = blockIdx.x & (a.don_groups - 1);
+    unsigned long long cur = 0;
+    int waiting = 0;
+    for (int look = 0; look < 2 && waiting <= 0; look++) {
+      g = look == 0 ? own : (own + 1u + (unsigned)S.checks * 5u) & (a.don_groups - 1);
+      cur = ld_vol_u64(a.sched + g * kSchedStride);
+      waiting = (int)((unsigned)(cur >> 32) - (unsigned)cur);
+    }
     if (waiting > 0) {
-      const int busy = max(1, (int)a.total_warps - waiting);
+      const int busy = max(1, (int)(a.total_warps / a.don_groups) - waiting);
       const int want = min(32, (waiting + busy - 1) / busy);
       for (; k <= L; k++) {
         if ((P.copy_next >> k) & 1u) continue;  // one of its candidates is searched for all
         const int len = S.iend[k] - S.iter[k];
-        const int unit = (k + 1 == n - 2) ? max(S.split, 2) : 2;
+        // a candidate before a chain is one table entry: nothing to hand out;
+        // one of a pass over the last two levels is a list, worth more than the
+        // prefix its taker repeats only in numbers
+        if (P.chain && k + 1 == P.chain_from) continue;
+        const int unit = (k + 1 == n - 2) ? max(S.split, 2) : (P.pair && a.pairs && k + 4 == n) ? PM_PAIR_PIECE : 2;
         if (len < unit) continue;
-        q = min(want, 2 * len / unit - 1);  // >= 1
+        q = min(min(want, waiting), 2 * len / unit - 1);  // >= 1
         break;
       }
-      if (q > 0 && atomicCAS(a.sched, cur, cur + (unsigned long long)q) != cur) q = 0;  // look again later
+      if (q > 0) {
+        // counted before they are given (draw_ticket must not see the takers
+        // waiting still), taken back when another donor was first
+        atomicAdd(a.all_sched, (unsigned long long)q);
+        if (atomicCAS(a.sched + g * kSchedStride, cur, cur + (unsigned long long)q) != cur) {
+          atomicAdd(a.all_sched, 0ull - (unsigned long long)q);
+          q = 0;
+        }
+      }
       first = cur & 0xffffffffull;
     }
   }
   q = __shfl_sync(FULL, q, 0);
   if (q == 0) return 0;
   k = __shfl_sync(FULL, k, 0);
+  g = __shfl_sync(FULL, g, 0);
   first = __shfl_sync(FULL, first, 0);
   const int it = S.iter[k], len = S.iend[k] - it;
   // part 0 of q + 1 stays here, part lane + 1 goes out
@@ -2587,12 +2613,13 @@ __device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, const DPlan&
     const int b = it + (int)((long long)len * (lane + 1) / (q + 1));
     const int e = it + (int)((long long)len * (lane + 2) / (q + 1));
     const unsigned long long slot = first + (unsigned long long)lane;
-    unsigned long long* ready = &a.don_ready[slot & a.don_mask];
+    const unsigned at = g * kGroupSlots + (unsigned)(slot & (kGroupSlots - 1));
+    unsigned long long* ready = &a.don_ready[at];
     // the slot's holder of one lap ago is reading it: a bounded wait
     int spin = 0;
     while (ld_acquire(ready) != 0ull && spin < (1 << 20)) { __nanosleep(64); spin++; }
     if (spin == (1 << 20)) err = DEV_TIMEOUT;
-    int4* dst = a.don_items + 3 * (slot & a.don_mask);
+    int4* dst = a.don_items + 3 * at;
     dst[0] = make_int4(plan_id, root_id, k, b);
     dst[1] = make_int4(e, S.path[2], S.path[3], S.path[4]);
     dst[2] = make_int4(S.path[5], S.path[6], (int)(unsigned)S.mul[k], (int)(unsigned)(S.mul[k] >> 32));
@@ -2815,23 +2842,24 @@ constexpr unsigned long long kQuit = ~0ull;
 __device__ unsigned long long draw_ticket(const MatchArgs& a, unsigned& seen) {
   const int lane = lane_id();
   unsigned long long old = 0;
+  unsigned ticket = 0;
   __syncwarp();
-  if (lane == 0) old = atomicAdd(a.sched, 1ull << 32);
+  if (lane == 0) {
+    ticket = (unsigned)(atomicAdd(a.sched + (blockIdx.x & (a.don_groups - 1)) * kSchedStride, 1ull << 32) >> 32);
+    old = atomicAdd(a.all_sched, 1ull << 32);
+  }
+  ticket = __shfl_sync(FULL, ticket, 0);
   old = __shfl_sync(FULL, old, 0);
-  const unsigned tickets = (unsigned)(old >> 32), pieces = (unsigned)old;
-  const unsigned waiting = tickets + 1u - pieces;
-  if (waiting < seen) return tickets;
+  const int waiting = (int)((unsigned)(old >> 32) + 1u - (unsigned)old);
+  if (waiting < (int)seen) return ticket;
   if (lane == 0) {
     __threadfence();  // after the pop that found the queue empty
     seen = atomicAdd(a.started, 0u);
   }
   seen = __shfl_sync(FULL, seen, 0);
-  if (waiting != seen) return tickets;
-  const unsigned long long last = min((unsigned long long)a.total_warps, (unsigned long long)a.don_mask + 1ull);
-  for (unsigned long long i = lane; i < last; i += 32) {
-    const unsigned long long slot = (unsigned long long)pieces + i;
-    *(volatile unsigned long long*)&a.don_ready[slot & a.don_mask] = kQuit;
-  }
+  if (waiting != (int)seen) return ticket;
+  for (unsigned i = lane; i < a.don_groups * kGroupSlots; i += 32)
+    *(volatile unsigned long long*)&a.don_ready[i] = kQuit;
   return kQuit;
 }
 
@@ -2841,14 +2869,16 @@ __device__ int wait_piece(const MatchArgs& a, unsigned long long ticket, Donatio
   int got = 0;
   int v[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (lane_id() == 0) {
-    unsigned long long* ready = &a.don_ready[ticket & a.don_mask];
+    const unsigned at =
+        (blockIdx.x & (a.don_groups - 1)) * kGroupSlots + (unsigned)(ticket & (kGroupSlots - 1));
+    unsigned long long* ready = &a.don_ready[at];
     // polled with plain volatile reads: an acquire read drops the SM's L1
     // contents, which the busy warps beside this one live on
     const unsigned long long r = ld_vol_u64(ready);
     if (r == kQuit) got = -1;
     else if (r == ticket + 1 && ld_acquire(ready) == r) {
       got = 1;
-      const volatile int* src = (const volatile int*)(a.don_items + 3 * (ticket & a.don_mask));
+      const volatile int* src = (const volatile int*)(a.don_items + 3 * at);
       for (int i = 0; i < 12; i++) v[i] = src[i];
       st_release(ready, 0ull);  // read: the slot is free for the ticket one lap on
     }
@@ -4020,7 +4050,7 @@ struct Launch {
   const pm_graph* g = nullptr;
 };
 
-static constexpr unsigned kDonSlots = 1u << 13;  // a launch has at most a few thousand warps
+static constexpr unsigned kDonSlots = 64 * kGroupSlots;  // 64 groups of some 50 warps
 // a warp's own arena: at most this many slot words and gather words
 static constexpr int64_t kOwnSlotWords = 1 << 16;
 static constexpr int64_t kOwnGatherWords = 1 << 15;
@@ -4157,7 +4187,7 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   L->big_bytes = big_bytes;
   // control block: cursors[32] counts[32] stats[] status sched heartbeat,
   // hand-off ready[] and items[]
-  L->ctl_words = 32 + 32 + kStatWords + 8 + kDonSlots + 6 * kDonSlots;
+  L->ctl_words = 32 + 32 + kStatWords + 24 + (kDonSlots / kGroupSlots) * kSchedStride + kDonSlots + 6 * kDonSlots;
   st = ensure((void**)ctl, ctl_bytes, L->ctl_words * 8);
   if (st != PM_OK) return st;
 
@@ -4263,12 +4293,13 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.counts = w; w += 32;
   a.stats = w; w += kStatWords;
   a.status = (unsigned int*)w; w += 1;
-  a.sched = w; w += 1;
+  a.all_sched = w; w += 1;
   a.started = (unsigned int*)w; w += 1;
-  a.heartbeat = w; w += 5;
+  a.heartbeat = w; w += 21;
+  a.don_groups = kDonSlots / kGroupSlots;
+  a.sched = w; w += a.don_groups * kSchedStride;
   a.don_ready = w; w += kDonSlots;
   a.don_items = (int4*)w; w += 6 * kDonSlots;
-  a.don_mask = kDonSlots - 1;
   a.total_warps = (unsigned int)L->warps;
   a.arena = *arena;
   a.arena_words = arena_words;
@@ -4525,8 +4556,11 @@ extern "C" pm_status pm_query_run(pm_query* q, uint64_t* counts_out, pm_stats* s
 static __device__ __align__(256) unsigned char g_static_scratch[PM_STATIC_SCRATCH_BYTES];
 
 namespace {
-constexpr unsigned kStaticRing = 4096;  // donation slots inside the static scratch
-constexpr size_t kStaticCtlWords = 32 + 32 + kStatWords + 8 + kStaticRing + 6 * kStaticRing;
+// Donation slots inside the static scratch (with the groups' words no more
+// than 4,096 slots and one set of words took before).
+constexpr unsigned kStaticRing = 8 * kGroupSlots;
+constexpr size_t kStaticCtlWords =
+    32 + 32 + kStatWords + 24 + (kStaticRing / kGroupSlots) * kSchedStride + kStaticRing + 6 * kStaticRing;
 
 struct StaticScratch {
   bool ready = false;
@@ -4694,12 +4728,13 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.counts = w; w += 32;
   a.stats = w; w += kStatWords;
   a.status = (unsigned int*)w; w += 1;
-  a.sched = w; w += 1;
+  a.all_sched = w; w += 1;
   a.started = (unsigned int*)w; w += 1;
-  a.heartbeat = w; w += 5;
+  a.heartbeat = w; w += 21;
+  a.don_groups = kStaticRing / kGroupSlots;
+  a.sched = w; w += a.don_groups * kSchedStride;
   a.don_ready = w; w += kStaticRing;
   a.don_items = (int4*)w; w += 6 * kStaticRing;
-  a.don_mask = kStaticRing - 1;
   const int64_t warps = blocks * wpb;
   a.total_warps = (unsigned int)warps;
   a.arena = arena;
