@@ -210,7 +210,6 @@ struct alignas(16) WarpState {
   unsigned long long memo_id;
   uint32_t memo_epoch;
   int32_t memo_len, memo_ub;
-  int32_t queue[64];
   int32_t lcnt[32];
   unsigned long long prb[32];    // the candidates' lists laid end to end: where each starts
   int32_t pexcl[33];             // and its offset in the row
@@ -225,7 +224,13 @@ struct alignas(16) WarpState {
   unsigned long long mul[8];     // per level: how many equal subtrees the search below it stands for
   int32_t big;                   // borrowed arena, or -1
   int32_t split;                 // donation threshold of the last-but-one level for the current root
-  int32_t pins[PM_MAX_LIST_PAGES];  // paged mode: frames pinned for a gather
+  // Paged mode: frames pinned for a gather; in HBM: elements whose value is not
+  // in the table (pair_levels).  (State for a block of eight warps is kept under
+  // a third of 100 KB, so that three blocks leave 156 KB of the SM to L1.)
+  union {
+    int32_t pins[PM_MAX_LIST_PAGES];
+    int32_t queue[64];
+  };
   alignas(16) int32_t sb[PM_SB_MAX + 4];  // the common operand (bitmap, hash table or sorted copy); +4 for a
                                          // bulk copy that starts up to 3 words before it
   unsigned long long mbar;               // completion barrier of the warp's bulk copies
@@ -233,6 +238,8 @@ struct alignas(16) WarpState {
   unsigned long long lrb[32];       // leaf batches: start of each candidate's first operand in colidx
   int32_t lexcl[33];                // leaf batches: offset of each candidate's operand in the flat layout
 };
+
+static_assert(3 * (8 * sizeof(WarpState) + 1024 + 256) <= 100 * 1024, "shared memory of three blocks");
 
 // Per-warp work counters (registers; flushed once at kernel exit).
 struct Work {
@@ -2910,6 +2917,19 @@ __device__ int wait_piece(const MatchArgs& a, unsigned long long ticket, Donatio
 template <bool LABELED, bool PAGED, int MINB>
 __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(const __grid_constant__ MatchArgs a) {
   extern __shared__ WarpState smem_state[];
+  // What the block's warps have in common: thousands of warps adding their
+  // counters to the same few words, one atomic after the other, took longer
+  // than a small query's search (the 4-clique on 400 vertices: launch 57 ->
+  // 48 us).
+  __shared__ unsigned long long blk_stats[kStatWords];
+  __shared__ unsigned blk_empty, blk_ended;  // plans whose queue was found empty; warps that have ended
+  if (threadIdx.x < kStatWords) blk_stats[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    blk_empty = blk_ended = 0;
+    atomicAdd(a.started, blockDim.x >> 5);  // before the first pop (draw_ticket)
+    __threadfence();
+  }
+  __syncthreads();
   const int lane = lane_id();
   const int wib = threadIdx.x >> 5;
   WarpState& S = smem_state[wib];
@@ -2936,8 +2956,6 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
     S.mphase = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.mbar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    atomicAdd(a.started, 1u);  // before the first pop (draw_ticket)
-    __threadfence();
   }
   __syncwarp();
   Work w;
@@ -2976,13 +2994,19 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
       // a unit, and the last unit, may be shorter)
       const unsigned long long per = (unsigned long long)((a.chunk + a.pop - 1) / a.pop);
       const unsigned long long nchunks = (unsigned long long)((P.nroots + a.chunk - 1) / a.chunk);
-      unsigned long long c = 0;
-      if (lane == 0) c = atomicAdd(&a.cursors[p], 1ull);
+      unsigned long long c = ~0ull;
+      if (lane == 0 && !((*(volatile unsigned*)&blk_empty >> p) & 1u)) c = atomicAdd(&a.cursors[p], 1ull);
       c = __shfl_sync(FULL, c, 0);
+      if (c == ~0ull) {
+        p = (p + 1 == np) ? 0 : p + 1;
+        exhausted++;
+        continue;
+      }
       const unsigned long long gc = c / per * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
       plan = p;
       p = (p + 1 == np) ? 0 : p + 1;
       if (gc >= nchunks) {
+        if (lane == 0) atomicOr(&blk_empty, 1u << plan);
         exhausted++;
         continue;
       }
@@ -3090,26 +3114,36 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   if (lane == 0) {
     if (a.memo) S.memo[a.memo_entries].x = (int32_t)S.memo_epoch;
     const unsigned long long t_end = global_ns();
-    atomicAdd(&a.stats[ST_WARP_NS], t_end - S.t_start);
-    if (t_drain) atomicAdd(&a.stats[ST_IDLE_NS], t_end - t_drain - min(busy_ns, t_end - t_drain));
-    atomicAdd(&a.stats[ST_SETOPS], w.setops);
-    atomicAdd(&a.stats[ST_BYTES], w.bytes + 8ull * roots);
-    atomicAdd(&a.stats[ST_ROOTS], roots);
-    if (w.borrows) atomicAdd(&a.stats[ST_BORROWS], w.borrows);
-    atomicAdd(&a.stats[ST_LEAF_CYC], w.leaf_cyc);
-    atomicAdd(&a.stats[ST_LEVEL_CYC], w.level_cyc);
-    atomicAdd(&a.stats[ST_PREFIX_CYC], w.prefix_cyc);
-    if (w.prefetched) atomicAdd(&a.stats[ST_PREFETCH], w.prefetched);
+    auto add = [&](int k, unsigned long long v) {
+      if (v) atomicAdd(&blk_stats[k], v);
+    };
+    add(ST_WARP_NS, t_end - S.t_start);
+    if (t_drain) add(ST_IDLE_NS, t_end - t_drain - min(busy_ns, t_end - t_drain));
+    add(ST_SETOPS, w.setops);
+    add(ST_BYTES, w.bytes + 8ull * roots);
+    add(ST_ROOTS, roots);
+    add(ST_BORROWS, w.borrows);
+    add(ST_LEAF_CYC, w.leaf_cyc);
+    add(ST_LEVEL_CYC, w.level_cyc);
+    add(ST_PREFIX_CYC, w.prefix_cyc);
+    add(ST_PREFETCH, w.prefetched);
     if (PAGED) {
-      atomicAdd(&a.stats[ST_HITS], w.pc.hits);
-      atomicAdd(&a.stats[ST_MISSES], w.pc.misses);
-      atomicAdd(&a.stats[ST_ZC_BYTES], w.pc.zc_bytes);
-      atomicAdd(&a.stats[ST_REQUESTS], w.pc.requests);
-      atomicAdd(&a.stats[ST_EVICTIONS], w.pc.evictions);
-      atomicAdd(&a.stats[ST_DROPPED], w.pc.dropped);
-      if (w.pc.dev_loads) {
-        atomicAdd(&a.stats[ST_DEV_LOADS], w.pc.dev_loads);
-        atomicAdd(&a.stats[ST_DEV_BYTES], w.pc.dev_bytes);
+      add(ST_HITS, w.pc.hits);
+      add(ST_MISSES, w.pc.misses);
+      add(ST_ZC_BYTES, w.pc.zc_bytes);
+      add(ST_REQUESTS, w.pc.requests);
+      add(ST_EVICTIONS, w.pc.evictions);
+      add(ST_DROPPED, w.pc.dropped);
+      add(ST_DEV_LOADS, w.pc.dev_loads);
+      add(ST_DEV_BYTES, w.pc.dev_bytes);
+    }
+    // the block's last warp takes the sums out
+    __threadfence_block();
+    if (atomicAdd(&blk_ended, 1u) == (blockDim.x >> 5) - 1) {
+      __threadfence_block();
+      for (int k = 0; k < kStatWords; k++) {
+        const unsigned long long v = *(volatile unsigned long long*)&blk_stats[k];
+        if (v) atomicAdd(&a.stats[k], v);
       }
     }
   }
@@ -4057,6 +4091,14 @@ static constexpr int64_t kOwnGatherWords = 1 << 15;
 static constexpr size_t kBigPoolMaxBytes = 48ull << 30;
 static constexpr int kCtlRead = 32 + 32 + kStatWords + 1;  // cursors, counts, stats, status word
 
+// Entries of a warp's value table for a graph of n vertices: one each up to
+// 16,384 (a warp's lookups go to the surroundings of a few roots).
+static int memo_entries_for(int64_t n) {
+  int e = 256;
+  while (e < 16384 && e < n) e <<= 1;
+  return e;
+}
+
 static MemoTables* memo_of(pm_ctx* c) {
   if (!c->memo) c->memo = new MemoTables;
   return c->memo;
@@ -4160,10 +4202,18 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   L->blocks = c->nsm * per_sm;
   L->warps = (int64_t)L->blocks * wpb;
   // keep the arenas within half of the free memory by trimming resident warps
+  // (what the buffers of an earlier call hold needs no look at free memory: a
+  // query of 50 us spends as much again on asking)
+  bool meets = false;
+  for (int i = 0; i < nplans; i++) meets = meets || (L->dp[i].pair == PAIR_MEET && !L->paged && o.leaf_per_lane == 0);
   size_t free_b = 0, total_b = 0;
-  CK(cudaMemGetInfo(&free_b, &total_b));
-  free_b += *arena_bytes;
-  while (L->blocks > c->nsm && (size_t)(L->warps * arena_words * 4) > free_b / 2) {
+  const bool fits = !borrowing && (size_t)(L->warps * arena_words * 4) + 256 <= *arena_bytes && *arena &&
+                    (!meets || (mt->d && mt->warps == L->warps && mt->entries == memo_entries_for(g->n)));
+  if (!fits) {
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    free_b += *arena_bytes;
+  }
+  while (!fits && L->blocks > c->nsm && (size_t)(L->warps * arena_words * 4) > free_b / 2) {
     L->blocks -= c->nsm;
     L->warps = (int64_t)L->blocks * wpb;
   }
@@ -4234,14 +4284,11 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   // surroundings, not to the whole graph), within an eighth of free memory
   MemoEntry* none = nullptr;
   MemoEntry** memo = &none;
-  bool meets = false;
-  for (int i = 0; i < nplans; i++) meets = meets || L->dp[i].pair == PAIR_MEET;
-  if (meets && !L->paged && o.leaf_per_lane == 0) {
-    int entries = 256;
-    while (entries < 16384 && entries < g->n) entries <<= 1;
+  if (meets) {
+    int entries = memo_entries_for(g->n);
     auto need = [&]() { return (size_t)L->warps * (size_t)(entries + 1) * sizeof(MemoEntry); };
-    while (entries > 256 && need() > (free_b + mt->bytes) / 8) entries >>= 1;
-    if (need() <= (free_b + mt->bytes) / 8) {
+    while (!fits && entries > 256 && need() > (free_b + mt->bytes) / 8) entries >>= 1;
+    if (fits || need() <= (free_b + mt->bytes) / 8) {
       const bool fresh = mt->bytes < need() || !mt->d;
       st = ensure((void**)&mt->d, &mt->bytes, need());
       if (st != PM_OK) return st;
