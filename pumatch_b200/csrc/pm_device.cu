@@ -1993,6 +1993,12 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
 //               only, and the same x is met under many v: each warp keeps the
 //               values in a table of its own in device memory (MemoEntry),
 //               tagged with the number of the (h0, bound) they belong to.
+//   PAIR_SHARED the main slot itself is a copy of a set s of level q-1, less v,
+//               and the last level fresh (unlabeled): the elements are the same
+//               for every v but for v itself and its neighbours in s, so the
+//               sum over s is taken once, and of each v's list only its members
+//               of s are counted -- by the list or, when v has a bit row and s
+//               is shorter, by looking s up in the row.
 // So no slot of level q is built, and no call is made per candidate of level
 // q: the lists of 32 candidates are laid end to end and their elements taken
 // 128 at a time, four per lane in flight (a tile per list left most lanes
@@ -2090,13 +2096,13 @@ template <bool LABELED, bool PAGED>
 __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, const WarpState& S) {
   // (truncated: an unlabeled list's first T elements less the path vertices
   // among them is not its length less them)
-  if (!P.pair || !a.pairs || (!LABELED && a.T && P.pair == PAIR_FRESH) || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
+  if (!P.pair || !a.pairs || (!LABELED && a.T && (P.pair == PAIR_FRESH || P.pair == PAIR_SHARED)) || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
   if (P.pair == PAIR_MEET) {
     if (PAGED || !a.memo) return false;
     const int n0 = S.size[P.pair_h0];
     return n0 <= PM_FILTER_MAX || (n0 > 0 && S.ptr[P.pair_h0][n0 - 1] < 32 * PM_SB_MAX);
   }
-  if (P.kind[P.level_begin[P.nnodes - 3]] == SLOT_INTERSECT) {
+  if (P.kind[P.level_begin[P.nnodes - 3]] == SLOT_INTERSECT || P.pair == PAIR_SHARED) {
     const int par = P.parent[P.level_begin[P.nnodes - 3]], n0 = S.size[par];
     return (n0 <= PM_FILTER_MAX || (n0 > 0 && S.ptr[par][n0 - 1] < 32 * PM_SB_MAX));
   }
@@ -2125,8 +2131,9 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
     mode = leaf_build(S, S.ptr[par], lenBm, S.id[par], set);
   }
   const int h0 = P.pair_h0;
-  const int32_t* H0 = kind != PAIR_FRESH ? S.ptr[h0] : nullptr;
-  const int len0 = kind != PAIR_FRESH ? S.size[h0] : 0;
+  constexpr bool has_h = KIND == PAIR_COPY || KIND == PAIR_MEET;
+  const int32_t* H0 = has_h ? S.ptr[h0] : nullptr;
+  const int len0 = has_h ? S.size[h0] : 0;
   // the last slot's bound (a main slot: the smallest constrained path vertex; up to L only in these plans)
   int ub_last = INT_MAX;
   if (!LABELED)
@@ -2186,8 +2193,9 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
     // no longer than they are
     if (a.T && !meet_main) len = min(len, a.T);
     ops = 1;
-    r.bytes += 4ull * (unsigned long long)(lenA + lenBm) + (LABELED ? (unsigned long long)lenA : 0ull);
-    if (kind != PAIR_FRESH) {
+    if (KIND != PAIR_SHARED)
+      r.bytes += 4ull * (unsigned long long)(lenA + lenBm) + (LABELED ? (unsigned long long)lenA : 0ull);
+    if (has_h) {
       // h: h0 without v (labeled: h0 itself), below h's bound
       bool in0 = false;
       if (!LABELED) {
@@ -2201,12 +2209,12 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       r.bytes += 4ull * (unsigned long long)(len_h + h_v) + (LABELED ? (unsigned long long)len_h : 0ull);
     }
   }
-  w.reads += __popc(__ballot_sync(FULL, mine));
+  if (KIND != PAIR_SHARED) w.reads += __popc(__ballot_sync(FULL, mine));
   // PAIR_FRESH: path vertices whose adjacency to x has to be looked up
   int pv[4];
   const unsigned* prow[4];
   int known = 0, n_ask = 0;  // neighbours of every x, below the bound
-  if (!LABELED && kind == PAIR_FRESH) {
+  if (!LABELED && (kind == PAIR_FRESH || kind == PAIR_SHARED)) {
 #pragma unroll
     for (int j = 0; j < 4; j++) { pv[j] = -1; prow[j] = nullptr; }
     for (int j = 0; j <= L; j++) {
@@ -2219,6 +2227,57 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
           if (k == n_ask) { pv[k] = p; prow[k] = hub_row(a, p); }
         n_ask++;
       }
+    }
+  }
+  if constexpr (KIND == PAIR_SHARED) {
+    // f(x) without v: x's degree less the path vertices next to it
+    const int32_t* shared = S.ptr[P.parent[ms]];
+    auto value = [&](int x, int& deg) {
+      deg = (int)(a.rowptr[x + 1] - a.rowptr[x]);
+      int f = deg - known;
+      for (int i = 0; i < n_ask; i++) {
+        const int p = i == 0 ? pv[0] : i == 1 ? pv[1] : i == 2 ? pv[2] : pv[3];
+        const unsigned* row = i == 0 ? prow[0] : i == 1 ? prow[1] : i == 2 ? prow[2] : prow[3];
+        const uint64_t pb = a.rowptr[p];
+        f -= (row ? (__ldg(row + (x >> 5)) >> (x & 31)) & 1u
+                  : bsearch_in<false>(a.colidx + pb, (int)(a.rowptr[p + 1] - pb), x)) ? 1 : 0;
+      }
+      return f;
+    };
+    unsigned long long sum_f = 0, sum_deg = 0;
+    for (int i = lane; i < lenBm; i += 32) {
+      int deg;
+      sum_f += (unsigned)value(shared[i], deg);
+      sum_deg += (unsigned)deg;
+    }
+    for (int d = 16; d; d >>= 1) {
+      sum_f += __shfl_xor_sync(FULL, sum_f, d);
+      sum_deg += __shfl_xor_sync(FULL, sum_deg, d);
+    }
+    if (mine) {
+      const bool in_s = mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(set, v) : leaf_member<MEMB_FILTER>(set, v);
+      unsigned long long f = sum_f, deg = sum_deg;
+      if (in_s) {
+        int dv;
+        f -= (unsigned)value(v, dv);
+        deg -= (unsigned)dv;
+      }
+      const unsigned long long k = (unsigned long long)(lenBm - (in_s ? 1 : 0));  // the main slot
+      // members of s next to v, v aside: taken off below (each counts one, and
+      // its bytes)
+      int near = 0;
+      const unsigned* row = hub_row(a, v);
+      if (row && lenBm <= len) {
+        for (int i = 0; i < lenBm; i++) {
+          const int x = shared[i];
+          near += x != v ? (__ldg(row + (x >> 5)) >> (x & 31)) & 1u : 0u;
+        }
+        len = 0;
+      }
+      f -= (unsigned)near;
+      ops += k;
+      r.cnt += f;
+      r.bytes += 4ull * ((unsigned long long)lenBm + k) + 4ull * (deg + f);
     }
   }
   // walk
@@ -2289,6 +2348,16 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       }
       if (MET && !__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) continue;
       int n_el = 0;
+      if (KIND == PAIR_SHARED) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int vo = __shfl_sync(FULL, v, own[k]);
+          n_el += in[k] && x[k] != vo ? 1 : 0;
+        }
+        r.cnt -= (unsigned)n_el;
+        r.bytes -= 4ull * (unsigned)n_el;
+        continue;
+      }
 #pragma unroll
       for (int k = 0; k < 4; k++) n_el += in[k] ? 1 : 0;
       r.elems += (unsigned)n_el;
@@ -2523,6 +2592,8 @@ __device__ __forceinline__ unsigned long long pair_levels(const MatchArgs& a, co
   const bool met = P.kind[P.level_begin[L + 1]] == SLOT_INTERSECT;
   if constexpr (!PAGED)
     if (P.pair == PAIR_MEET) return pair_pass<LABELED, PAGED, PAIR_MEET, false>(a, P, S, L, b, e, w);
+  if constexpr (!LABELED && !PAGED)
+    if (P.pair == PAIR_SHARED) return pair_pass<LABELED, PAGED, PAIR_SHARED, true>(a, P, S, L, b, e, w);
   if (P.pair == PAIR_COPY)
     return met ? pair_pass<LABELED, PAGED, PAIR_COPY, true>(a, P, S, L, b, e, w)
                : pair_pass<LABELED, PAGED, PAIR_COPY, false>(a, P, S, L, b, e, w);
@@ -3528,6 +3599,9 @@ DPlan to_dplan(const Plan& p) {
     const bool met = d.kind[b] == SLOT_INTERSECT;
     bool ok = (d.kind[b] == SLOT_FRESH || met) && d.alias[b] < 0;
     if (p.labeled) ok = ok && __builtin_popcount(p.slot_labels[b]) == 1 && __builtin_popcount(p.slot_labels[last]) == 1;
+    if (!p.labeled && k == 1 && d.kind[b] == SLOT_COPY && d.alias[b] < 0 && !p.partial[b] && d.kind[last] == SLOT_FRESH &&
+        !p.partial[last])
+      d.pair = PAIR_SHARED;
     auto within = [&](int small, int large) { return (p.slot_labels[small] & ~p.slot_labels[large]) == 0; };
     if (ok && k == 1) {
       if (d.kind[last] == SLOT_FRESH && !(p.partial[last] & ~early)) d.pair = PAIR_FRESH;

@@ -21,7 +21,7 @@ enum : uint32_t {
 };
 
 // What the last level adds per element of level n-3's main slot (pair_levels).
-enum PairKind : uint8_t { PAIR_NONE = 0, PAIR_COPY = 1, PAIR_FRESH = 2, PAIR_MEET = 3 };
+enum PairKind : uint8_t { PAIR_NONE = 0, PAIR_COPY = 1, PAIR_FRESH = 2, PAIR_MEET = 3, PAIR_SHARED = 4 };
 
 // One plan as the kernel reads it (constant memory).
 struct DPlan {
