@@ -5,22 +5,23 @@
 //   * one persistent grid, sized to the SM count times the resident blocks
 //     per SM; every warp runs its own depth-first search;
 //   * work = root edges (v0, v1) of one or more plans, handed out in chunks
-//     by 64-bit atomic cursors (one per plan, warps start on different plans
-//     so a batch of patterns interleaves);
-//   * a warp that still holds a candidate range (at any DFS level) when the
-//     queue has run dry donates the upper half of its shallowest splittable
-//     range, with the path prefix, to a global donation ring that idle warps
-//     drain (replaces the reference's disabled stealing,
-//     src/gpu_match.cu:21-148, 818-853);
-//   * each level's candidate sets ("slots") are computed by a warp-cooperative
-//     sorted-set operation -- 32 candidates per step, per-lane membership
-//     search, __ballot_sync/__popc compaction -- and stored in a per-warp
-//     arena in HBM sized to the plan's worst case, so nothing is truncated
-//     (the reference caps every set at GRAPH_DEGREE=4096; that cap is kept
-//     only as an explicit emulation switch);
-//   * the last level is counted, never materialised: work-balanced across
-//     the warp (leaf_flat), one candidate per lane (leaf_batch), or, for
-//     clique-like plans, the last two levels one candidate per lane
+//     by 64-bit atomic cursors (one per plan, plan after plan);
+//   * a warp that still holds a candidate range (at any DFS level) when others
+//     have run out of roots cuts its shallowest splittable range and hands the
+//     pieces, with the path prefix, to waiting warps by ticket (replaces the
+//     reference's disabled stealing, src/gpu_match.cu:21-148, 818-853);
+//   * each level's candidate sets ("slots") are read in place where they are
+//     an adjacency list or their parent, else computed by a warp-cooperative
+//     sorted-set operation -- 128 elements per step, __ballot_sync/__popc
+//     compaction -- and stored in a per-warp arena in HBM sized to the plan's
+//     worst case, so nothing is truncated (the reference caps every set at
+//     GRAPH_DEGREE=4096; that cap is kept only as an explicit emulation
+//     switch);
+//   * the last level is counted, never materialised: with the level before it
+//     in one pass where the plan allows (pair_levels), cliques in bit sets
+//     (clique_bits), labeled tails from tables per vertex (chain_kernel), else
+//     work-balanced across the warp (leaf_flat), one candidate per lane
+//     (leaf_batch) or the last two levels one candidate per lane
 //     (lane_subtree).
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
@@ -104,7 +105,7 @@ struct MatchArgs {
   int32_t pairs;                // last two levels in one pass where the plan allows (pair_levels)
   int32_t memo_entries;         // entries of a warp's value table (a power of two), and the tables: each
   MemoEntry* memo;              // warp's entries, then one that holds the last epoch it used (null: none)
-  const unsigned long long* asym;  // 0 when every adjacency entry has its reverse
+  const unsigned long long* asym;  // two words, 0 when every adjacency entry has its reverse and none comes twice
   const int32_t* hub_slot;      // unlabeled, HBM: [n] bit row of a vertex with a long list, or -1 (null: none)
   const unsigned* hub_bits;     // bit rows of hub_words words: bit u of v's row = u is in v's list
   int32_t hub_words;
@@ -645,13 +646,14 @@ __device__ __forceinline__ int compact(const int32_t* A, int n, bool cg, int32_t
   return cnt;
 }
 
-// Whether u in N(v) says v in N(u): an undirected graph, as the interface
-// asks for.  What is taken from one list about the other asks first.
-__device__ __forceinline__ bool symmetric(const MatchArgs& a) { return a.asym && *a.asym == 0ull; }
+// Whether u in N(v) says v in N(u), and each list holds an element once: an
+// undirected simple graph, as the interface asks for.  What is taken from one
+// list about the other, or from a bit about an element, asks first.
+__device__ __forceinline__ bool symmetric(const MatchArgs& a) { return a.asym && (a.asym[0] | a.asym[1]) == 0ull; }
 
 // v's bit row (pm_graph::d_hub_bits), or null when its list is short.
 __device__ __forceinline__ const unsigned* hub_row(const MatchArgs& a, int v) {
-  if (!a.hub_slot) return nullptr;
+  if (!a.hub_slot || !symmetric(a)) return nullptr;
   const int k = a.hub_slot[v];
   return k < 0 ? nullptr : a.hub_bits + (long long)k * a.hub_words;
 }
@@ -767,6 +769,9 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
   const bool cgA = RA.cg, cgB = RB.cg;
   // elements that stay where they are: device memory that outlives the slot
   const bool in_place = !PAGED || (kind == SLOT_COPY && L > 1);
+  // each element once, so that leaving a vertex out leaves one element out and
+  // an intersection has its elements from either operand
+  const bool simple = symmetric(a);
 
   // symmetry-breaking upper bound (unlabeled only, src/gpu_match.cu:426-458)
   // and, for fresh sets and copies, the path vertices to leave out
@@ -789,7 +794,17 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
     const int scan = (kind == SLOT_FRESH && T && lenA > T) ? T : lenA;
     const int holes = __popc(__ballot_sync(FULL, hole && (lane & 3) == 0 && pos < scan));
     cnt = scan - holes;
-    if (T && cnt > T) {  // a copy longer than T: its first T survivors
+    if (!simple) {
+      if (last) {
+        cnt = compact<PAGED>(A, scan, cgA, nullptr, 0, [&](const int (&v)[4], bool (&in)[4]) {
+          for (int k = first; k <= L; k++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] != S.path[k];
+        });
+        if (T && cnt > T) cnt = T;
+        done = true;
+      }
+    } else if (T && cnt > T) {  // a copy longer than T: its first T survivors
       cnt = T;
       done = last;
       if (in_place && !holes && !last) {
@@ -803,16 +818,18 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
       done = true;
     }
     if (!done) {
+      if (!simple) cnt = T && scan > T ? T : scan;  // room for all of them
       if (slot_room(a, S, top, cnt, w)) {
         int32_t* out = S.arena + top;
-        const int want = cnt;
-        compact<PAGED>(A, scan, cgA, out, want, [&](const int (&v)[4], bool (&in)[4]) {
+        const int want = simple ? cnt : T;
+        const int got = compact<PAGED>(A, scan, cgA, out, want, [&](const int (&v)[4], bool (&in)[4]) {
           for (int k = first; k <= L; k++) {
             const int pk = S.path[k];
 #pragma unroll
             for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] != pk;
           }
         });
+        if (!simple) cnt = T && got > T ? T : got;
       } else {
         cnt = 0;
       }
@@ -866,7 +883,7 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
 #pragma unroll
         for (int q = 0; q < 4; q++) in[q] = in[q] && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
       });
-    } else if ((long long)lenB * 16 < lenA) {
+    } else if ((long long)lenB * 16 < lenA && simple) {
       cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[4], bool (&in)[4]) {
         bsearch4<PAGED>(A, lenA, v, in, cgA);
         labelled(v, in);
@@ -2819,7 +2836,10 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
     bool subtree = false, bits = false;
     if constexpr (!LABELED && !PAGED) {
       const int hs = P.level_begin[L] + 1;
-      bits = a.clique_bits && P.clique && L + 4 <= n && it < iend && S.size[hs] <= PM_CLIQUE_MAX &&
+      // (seven vertices: two levels between a candidate and the last make one
+      // candidate of a large set too long a stretch without a look at the
+      // deadline; the level below takes over there)
+      bits = a.clique_bits && P.clique && L + 4 <= n && (L + 6 > n || S.size[hs] <= 128) && symmetric(a) && it < iend && S.size[hs] <= PM_CLIQUE_MAX &&
              S.top[L + 1] + clique_words(S.size[hs]) <= S.cap;
       subtree = !bits && P.l2_x >= 0 && L + 4 == n && it < iend && a.lane_subtree_max > 0 &&
                 S.size[P.parent[P.l2_x]] <= a.lane_subtree_max &&
@@ -3033,7 +3053,7 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
   memset(&w, 0, sizeof(w));
   unsigned long long roots = 0;
   const int np = a.nplans;
-  int p = (int)(gw % np);
+  int p = 0;
   int exhausted = 0;
   long long r = 0, re = 0;        // phase 1: roots [r, re) of the last pop
   unsigned long long local = 0;   // matches of plan `plan` not yet in a.counts
@@ -3057,7 +3077,10 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
       r++;
       roots++;
     } else if (exhausted < np) {
-      // phase 1: root chunks from the per-plan cursors, plans in turn
+      // phase 1: root chunks from the per-plan cursors, one plan after the
+      // other: warps on twenty plans at once empty each other's instruction
+      // cache and their own value tables (20 patterns on 65,536 vertices, each
+      // warp starting on another plan 21.4 ms, so 19.2 ms)
       if (lane == 0 && local) atomicAdd(&a.counts[plan], local);
       local = 0;
       const DPlan& P = a.plans[p];
@@ -3075,9 +3098,9 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
       }
       const unsigned long long gc = c / per * (unsigned long long)a.shard_count + (unsigned long long)a.shard_rank;
       plan = p;
-      p = (p + 1 == np) ? 0 : p + 1;
       if (gc >= nchunks) {
         if (lane == 0) atomicOr(&blk_empty, 1u << plan);
+        p = (p + 1 == np) ? 0 : p + 1;
         exhausted++;
         continue;
       }
@@ -3227,9 +3250,9 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
 // adjacency order), so root ids match the reference's Job[] indices.
 // =====================================================================
 
-// Also sums a hash of every entry's vertex pair into *asym, with the sign of
+// Also sums a hash of every entry's vertex pair into asym[0], with the sign of
 // the entry's direction: 0 when each entry has its reverse (and, but for one
-// graph in 2^64 or so, only then).
+// graph in 2^64 or so, only then).  asym[1]: a list holds an element twice.
 __device__ __forceinline__ unsigned long long pair_hash(unsigned lo, unsigned hi) {
   uint64_t x = ((uint64_t)hi << 32 | lo) + 0x9E3779B97F4A7C15ull;
   return Rng::splitmix(x);
@@ -3240,7 +3263,8 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
   __shared__ int best[kListWarps];
   const int lane = lane_id();
   unsigned long long sum = 0;
-  auto walk = [&](long long v, uint64_t b, uint64_t e) {
+  bool twice = false;
+  auto walk = [&](long long v, uint64_t b, uint64_t e, uint64_t e_list) {
     int m = 0;
     for (uint64_t i0 = b; i0 < e; i0 += 128) {
       int u[4];
@@ -3249,6 +3273,8 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         if (u[q] < 0) continue;
+        const uint64_t next = i0 + 32 * q + lane + 1;
+        twice = twice || (next < e_list && colidx[next] == u[q]);
         m = max(m, (int)(rowptr[u[q] + 1] - rowptr[u[q]]));
         if (u[q] > v) sum += pair_hash((unsigned)v, (unsigned)u[q]);
         else if (u[q] < v) sum -= pair_hash((unsigned)u[q], (unsigned)v);
@@ -3258,11 +3284,11 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
   };
   for_lists(rowptr, 0, n,
             [&](long long v, uint64_t b, uint64_t e) {
-              const int m = walk(v, b, e);
+              const int m = walk(v, b, e, e);
               if (lane == 0) out[v] = m;
             },
-            [&](long long v, uint64_t, uint64_t, uint64_t b0, uint64_t e0, int k) {
-              const int m = walk(v, b0, e0);
+            [&](long long v, uint64_t, uint64_t e, uint64_t b0, uint64_t e0, int k) {
+              const int m = walk(v, b0, e0, e);
               if (lane == 0) best[k] = m;
               __syncthreads();
               if (threadIdx.x < 32) {
@@ -3273,6 +3299,7 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
             });
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
   if (lane == 0 && sum) atomicAdd(asym, sum);
+  if (__any_sync(FULL, twice) && lane == 0) atomicOr(asym + 1, 1ull);
 }
 
 // Regroups each list by label, keeping id order within a label (a stable
@@ -3679,9 +3706,9 @@ int64_t arena_words_for(const Plan& p, int32_t maxdeg, int T) {
 
 }  // namespace
 
-// d_maxnbrdeg: n entries and, after them, the 64-bit word maxnbrdeg_kernel sums
-// the entries' directions into.
-static size_t maxnbrdeg_bytes(int64_t n) { return sizeof(int32_t) * (size_t)((n + 1) & ~1ll) + 8; }
+// d_maxnbrdeg: n entries and, after them, the two 64-bit words in which
+// maxnbrdeg_kernel notes what the lists are like.
+static size_t maxnbrdeg_bytes(int64_t n) { return sizeof(int32_t) * (size_t)((n + 1) & ~1ll) + 16; }
 static unsigned long long* asym_word(const pm_graph* g) {
   return reinterpret_cast<unsigned long long*>(g->d_maxnbrdeg + ((g->n + 1) & ~1ll));
 }
@@ -3692,7 +3719,7 @@ namespace pm {
 pm_status compute_maxnbrdeg(pm_graph* g, const int32_t* colidx) {
   if (g->n > 0) {
     PM_CK_PENDING("max neighbour degree");
-    CK(cudaMemset(asym_word(g), 0, 8));
+    CK(cudaMemset(asym_word(g), 0, 16));
     maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
@@ -3707,7 +3734,7 @@ static pm_status graph_finish(pm_graph* g) {
   g->device_bytes += sizeof(int32_t) * g->n;
   if (g->n > 0 && g->residency == PM_RESIDENT_HBM) {
     PM_CK_PENDING("max neighbour degree");
-    CK(cudaMemset(asym_word(g), 0, 8));
+    CK(cudaMemset(asym_word(g), 0, 16));
     maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
@@ -3734,14 +3761,22 @@ static pm_status graph_finish(pm_graph* g) {
     if (e == cudaSuccess && rows) {
       e = cudaMalloc(&g->d_hub_slot, sizeof(int32_t) * g->n);
       if (e == cudaSuccess) e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
-      if (e == cudaSuccess) e = cudaMemset(g->d_hub_bits, 0, rows * words * 4);
-      if (e == cudaSuccess) {
+      if (e == cudaErrorMemoryAllocation) {  // no room: the graph does without
+        (void)cudaGetLastError();
+        free_dev(g->d_hub_slot);
+        g->d_hub_slot = nullptr;
+        g->d_hub_bits = nullptr;
+        rows = 0;
+        e = cudaSuccess;
+      }
+      if (e == cudaSuccess && rows) e = cudaMemset(g->d_hub_bits, 0, rows * words * 4);
+      if (e == cudaSuccess && rows) {
         hub_rows_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, 1 << k, words, bins + 32, g->d_hub_slot,
                                        g->d_hub_bits);
         e = cudaGetLastError();
       }
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
-      g->device_bytes += sizeof(int32_t) * g->n + rows * words * 4;
+      if (rows) g->device_bytes += sizeof(int32_t) * g->n + rows * words * 4;
     }
     cudaFree(bins);
     CK(e);
@@ -4326,8 +4361,10 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
       if (need + levels * table > (1ull << 30)) L->dp[i].chain_from = 0;
       else need += levels * table;
     }
-    st = ensure(chain, chain_bytes, need);
-    if (st != PM_OK) return st;
+    if (ensure(chain, chain_bytes, need) != PM_OK) {  // no room: the tails are searched
+      (void)cudaGetLastError();
+      for (int i = 0; i < nplans; i++) L->dp[i].chain_from = 0;
+    }
     ulonglong4* at = (ulonglong4*)*chain;
     for (int i = 0; i < nplans; i++) {
       DPlan& d = L->dp[i];
@@ -4364,14 +4401,17 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
     while (!fits && entries > 256 && need() > (free_b + mt->bytes) / 8) entries >>= 1;
     if (fits || need() <= (free_b + mt->bytes) / 8) {
       const bool fresh = mt->bytes < need() || !mt->d;
-      st = ensure((void**)&mt->d, &mt->bytes, need());
-      if (st != PM_OK) return st;
-      if (fresh || mt->warps != L->warps || mt->entries != entries)
-        CK(cudaMemsetAsync(mt->d, 0, need(), c->stream));
-      mt->warps = L->warps;
-      mt->entries = entries;
-      L->memo_entries = entries;
-      memo = &mt->d;
+      if (ensure((void**)&mt->d, &mt->bytes, need()) != PM_OK) {  // no room: lists are walked each time
+        (void)cudaGetLastError();
+        mt->warps = 0;
+      } else {
+        if (fresh || mt->warps != L->warps || mt->entries != entries)
+          CK(cudaMemsetAsync(mt->d, 0, need(), c->stream));
+        mt->warps = L->warps;
+        mt->entries = entries;
+        L->memo_entries = entries;
+        memo = &mt->d;
+      }
     }
   }
 

@@ -119,3 +119,16 @@ def test_levels_of_copies(ctx, shape, truncate, paged):
         c, st = ctx.match(g, [p], truncate=truncate, split_level1=split, timeout_ms=60000)
         assert (c[0], st["set_ops"], st["alg_bytes"]) == (want, st0["set_ops"], st0["alg_bytes"])
     g.close()
+
+
+@pytest.mark.parametrize("shape", ["C5", "house", "C4_tail", "house_tail"])
+def test_elements_that_come_twice(ctx, shape):
+    """A list that holds an element twice is no simple graph's: bit rows and what one list says of another are not
+    used, and both ways count alike."""
+    hg = pm.gen_chung_lu(120, 500, seed=9)
+    src = np.repeat(np.arange(hg.n), np.diff(hg.rowptr.astype(np.int64)))
+    e = [(int(a), int(b)) for a, b in zip(src, hg.colidx)]
+    e += [x for a, b in e if a < b and (a + b) % 7 == 0 for x in ((a, b), (b, a))]
+    e.sort()
+    rp = np.concatenate([[0], np.cumsum(np.bincount([a for a, _ in e], minlength=hg.n))])
+    same(*runs(ctx, pm.HostGraph(rp.astype(np.uint64), np.array([b for _, b in e], dtype=np.int32)), shape, None))
