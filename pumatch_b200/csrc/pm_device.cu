@@ -595,45 +595,48 @@ __device__ __forceinline__ int group_lower_bound(const int32_t* A, int len, int 
 // Four searches at once: whether each x[q] is in sorted B[0, len).  The steps
 // do not depend on what is found, so the four loads of a step are in flight
 // together.
-template <bool CG>
-__device__ __forceinline__ void bsearch4(const int32_t* B, int len, const int (&x)[4], bool (&in)[4], bool cg) {
-  int p[4] = {0, 0, 0, 0};
+template <bool CG, int N>
+__device__ __forceinline__ void bsearch4(const int32_t* B, int len, const int (&x)[N], bool (&in)[N], bool cg) {
+  int p[N] = {};
   if (len <= 0) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) in[q] = false;
+    for (int q = 0; q < N; q++) in[q] = false;
     return;
   }
   for (int n = len; n > 1;) {
     const int h = n >> 1;
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+    for (int q = 0; q < N; q++)
       if (ld<CG>(B + p[q] + h, cg) <= x[q]) p[q] += h;
     n -= h;
   }
 #pragma unroll
-  for (int q = 0; q < 4; q++) in[q] = in[q] && ld<CG>(B + p[q], cg) == x[q];
+  for (int q = 0; q < N; q++) in[q] = in[q] && ld<CG>(B + p[q], cg) == x[q];
 }
 
 // The elements of A[0, n) that `keep` leaves (keep(x, in): in[q] comes in as
 // "x[q] is an element"), in order: counted, and written to out (unless null)
-// up to T of them (T 0: all).  Four loads in flight per lane: one tile of 32
-// per step left the warp waiting a load's latency for every tile.
+// up to T of them (T 0: all).  Two loads in flight per lane: with one the warp
+// waits a load's latency for every tile of 32, with four the code is so long
+// that it waits for its instructions (labeled 5-cycle with a tail on 131,072
+// vertices: 4.5 ms with four, 3.8 ms with two).
 template <bool CG, class Keep>
 __device__ __forceinline__ int compact(const int32_t* A, int n, bool cg, int32_t* out, int T, Keep keep) {
   const int lane = lane_id();
+  constexpr int U = 2;
   int cnt = 0;
-  for (int base = 0; base < n; base += 128) {
-    int x[4];
-    bool in[4];
+  for (int base = 0; base < n; base += 32 * U) {
+    int x[U];
+    bool in[U];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < U; q++) {
       const int i = base + 32 * q + lane;
       in[q] = i < n;
       x[q] = in[q] ? ld<CG>(A + i, cg) : 0;
     }
     keep(x, in);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < U; q++) {
       const unsigned bal = __ballot_sync(FULL, in[q]);
       if (out && in[q]) {
         const int pos = cnt + __popc(bal & lanemask_lt());
@@ -796,10 +799,10 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
     cnt = scan - holes;
     if (!simple) {
       if (last) {
-        cnt = compact<PAGED>(A, scan, cgA, nullptr, 0, [&](const int (&v)[4], bool (&in)[4]) {
+        cnt = compact<PAGED>(A, scan, cgA, nullptr, 0, [&](const int (&v)[2], bool (&in)[2]) {
           for (int k = first; k <= L; k++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] != S.path[k];
+            for (int q = 0; q < 2; q++) in[q] = in[q] && v[q] != S.path[k];
         });
         if (T && cnt > T) cnt = T;
         done = true;
@@ -822,11 +825,11 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
       if (slot_room(a, S, top, cnt, w)) {
         int32_t* out = S.arena + top;
         const int want = simple ? cnt : T;
-        const int got = compact<PAGED>(A, scan, cgA, out, want, [&](const int (&v)[4], bool (&in)[4]) {
+        const int got = compact<PAGED>(A, scan, cgA, out, want, [&](const int (&v)[2], bool (&in)[2]) {
           for (int k = first; k <= L; k++) {
             const int pk = S.path[k];
 #pragma unroll
-            for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] != pk;
+            for (int q = 0; q < 2; q++) in[q] = in[q] && v[q] != pk;
           }
         });
         if (!simple) cnt = T && got > T ? T : got;
@@ -843,7 +846,7 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
         done = true;
       } else {
         if (slot_room(a, S, top, cnt, w))
-          compact<PAGED>(A, cnt, cgA, S.arena + top, 0, [](const int (&)[4], bool (&)[4]) {});
+          compact<PAGED>(A, cnt, cgA, S.arena + top, 0, [](const int (&)[2], bool (&)[2]) {});
         else
           cnt = 0;
         used = cnt;
@@ -853,10 +856,10 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
     // labeled by mask, or an intersection
     if (ub != INT_MAX) lenA = warp_lower_bound<PAGED>(A, lenA, ub, cgA);
     const bool check = LABELED && !by_label;
-    auto labelled = [&](const int (&v)[4], bool (&in)[4]) {
+    auto labelled = [&](const int (&v)[2], bool (&in)[2]) {
       if (check) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) in[q] = in[q] && ((mask >> a.labels[v[q]]) & 1u);
+        for (int q = 0; q < 2; q++) in[q] = in[q] && ((mask >> a.labels[v[q]]) & 1u);
       }
     };
     const unsigned* row = nullptr;
@@ -874,38 +877,38 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
       cnt = compact<PAGED>(A, lenA, cgA, out, T, labelled);
     } else if (!LABELED && !PAGED && lenB <= lenA && (row = hub_row(a, vL))) {
       // the newest vertex has a bit row: one load per element of the parent
-      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[2], bool (&in)[2]) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) in[q] = in[q] && v[q] < ub && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
+        for (int q = 0; q < 2; q++) in[q] = in[q] && v[q] < ub && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
       });
     } else if (!LABELED && !PAGED && L == 1 && (row = hub_row(a, S.path[0]))) {
-      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[2], bool (&in)[2]) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) in[q] = in[q] && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
+        for (int q = 0; q < 2; q++) in[q] = in[q] && ((__ldg(row + (v[q] >> 5)) >> (v[q] & 31)) & 1u);
       });
     } else if ((long long)lenB * 16 < lenA && simple) {
-      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+      cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[2], bool (&in)[2]) {
         bsearch4<PAGED>(A, lenA, v, in, cgA);
         labelled(v, in);
       });
     } else if ((long long)lenA * 16 < lenB && !(idB && idB == S.sb_id && lenB == S.sb_len)) {
-      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[2], bool (&in)[2]) {
         bsearch4<PAGED>(B, lenB, v, in, cgB);
         labelled(v, in);
       });
     } else {
       LeafSet m;
       const int mode = leaf_build<PAGED>(S, B, lenB, idB, m, cgB);
-      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[4], bool (&in)[4]) {
+      cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[2], bool (&in)[2]) {
         if (mode == MEMB_BITMAP) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) in[q] = in[q] && leaf_maybe<MEMB_BITMAP>(m, v[q]);
+          for (int q = 0; q < 2; q++) in[q] = in[q] && leaf_maybe<MEMB_BITMAP>(m, v[q]);
         } else {
           if (mode == MEMB_FILTER) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) in[q] = in[q] && leaf_maybe<MEMB_FILTER>(m, v[q]);
+            for (int q = 0; q < 2; q++) in[q] = in[q] && leaf_maybe<MEMB_FILTER>(m, v[q]);
           }
-          if (__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) bsearch4<PAGED>(B, lenB, v, in, cgB);
+          if (__any_sync(FULL, in[0] || in[1])) bsearch4<PAGED>(B, lenB, v, in, cgB);
         }
         labelled(v, in);
       });
@@ -2018,10 +2021,12 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
 //               is shorter, by looking s up in the row.
 // So no slot of level q is built, and no call is made per candidate of level
 // q: the lists of 32 candidates are laid end to end and their elements taken
-// 128 at a time, four per lane in flight (a tile per list left most lanes
+// 64 at a time, two per lane in flight (a tile per list left most lanes
 // without one: the 6-cycle's lists have about ten elements below their bound).
-// Each kind is a function of its own: what the loop waited for most was its
-// own instructions (no_instruction 9.2 of 25 stall cycles per issue).
+// Each kind is a function of its own: what the loop waits for most is its own
+// instructions (no_instruction 9.2 of 25 stall cycles per issue; four elements
+// per lane in flight: 6-cycle shard 40 ms, 20-pattern batch 19.2 ms; two: 36.6
+// and 16.0; one: 40.9 and 14.9, but the 7-cycle 74 ms for 66).
 // Set operations, counts and accounting are those of run_level + leaf_batch.
 //
 // What bounded the search before was instructions, not bytes: about 1,400 per
@@ -2075,10 +2080,10 @@ __device__ __noinline__ void meet_values(const MatchArgs& a, WarpState& S, const
   if (lane == 31) S.lexcl[32] = total;
   S.lcnt[lane] = 0;
   __syncwarp();
-  for (int t0 = 0; t0 < total; t0 += 128) {
-    int y[4], own[4];
+  for (int t0 = 0; t0 < total; t0 += 64) {
+    int y[2], own[2];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < 2; q++) {
       const int t = t0 + 32 * q + lane;
       int j = 0;
 #pragma unroll
@@ -2088,7 +2093,7 @@ __device__ __noinline__ void meet_values(const MatchArgs& a, WarpState& S, const
       y[q] = t < total ? __ldg(lists + S.lrb[j] + (unsigned long long)(t - S.lexcl[j])) : -1;
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < 2; q++) {
       const bool hit = y[q] >= 0 && (mode == MEMB_BITMAP ? leaf_member<MEMB_BITMAP>(m, y[q])
                                                           : leaf_member<MEMB_FILTER>(m, y[q]));
       if (hit) atomicAdd(&S.lcnt[own[q]], 1);
@@ -2127,6 +2132,14 @@ __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, c
 }
 
 // Candidates [b, e) (at most 32) of level L = n-4's main slot.
+template <int N>
+__device__ __forceinline__ bool any_of(const bool (&in)[N]) {
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < N; q++) any = any || in[q];
+  return any;
+}
+
 template <bool LABELED, bool PAGED, int KIND, bool MET>
 __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
                                                      int e, Work* wt) {
@@ -2313,6 +2326,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
     __syncwarp();
   }
   const int32_t* lists = LABELED ? a.colidx_lab : a.colidx;
+  constexpr int U = 2;  // elements per lane in flight
   // (paged: one resolved list after the other)
   for (unsigned left = PAGED ? __ballot_sync(FULL, len > 0) : 1u; left; left &= left - 1) {
     const int one = PAGED ? __ffs(left) - 1 : 0;
@@ -2323,11 +2337,11 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       if (!gather_room(a, S, S.top[q], total, w)) break;
       cur = paged_list(a.pg, base, total, S.gather, S.pins, w.pc);
     }
-    for (int t0 = 0; t0 < total; t0 += 128) {
-      int x[4], own[4];
-      bool in[4];
+    for (int t0 = 0; t0 < total; t0 += 32 * U) {
+      int x[U], own[U];
+      bool in[U];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
+      for (int k = 0; k < U; k++) {
         const int t = t0 + 32 * k + lane;
         in[k] = t < total;
         if (PAGED) {
@@ -2345,29 +2359,29 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       if (MET) {
         if (mode == MEMB_BITMAP) {
 #pragma unroll
-          for (int k = 0; k < 4; k++) in[k] = in[k] && leaf_maybe<MEMB_BITMAP>(set, x[k]);
+          for (int k = 0; k < U; k++) in[k] = in[k] && leaf_maybe<MEMB_BITMAP>(set, x[k]);
         } else {
 #pragma unroll
-          for (int k = 0; k < 4; k++) in[k] = in[k] && leaf_maybe<MEMB_FILTER>(set, x[k]);
-          if (__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) bsearch4<false>(set.g, set.lenB, x, in, false);
+          for (int k = 0; k < U; k++) in[k] = in[k] && leaf_maybe<MEMB_FILTER>(set, x[k]);
+          if (__any_sync(FULL, any_of(in))) bsearch4<false>(set.g, set.lenB, x, in, false);
         }
       } else if (!LABELED) {
         for (int i = 0; i <= L; i++) {
           const int p = S.path[i];
 #pragma unroll
-          for (int k = 0; k < 4; k++) in[k] = in[k] && x[k] != p;
+          for (int k = 0; k < U; k++) in[k] = in[k] && x[k] != p;
         }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           const int vo = __shfl_sync(FULL, v, own[k]);
           in[k] = in[k] && x[k] != vo;
         }
       }
-      if (MET && !__any_sync(FULL, in[0] || in[1] || in[2] || in[3])) continue;
+      if (MET && !__any_sync(FULL, any_of(in))) continue;
       int n_el = 0;
       if (KIND == PAIR_SHARED) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           const int vo = __shfl_sync(FULL, v, own[k]);
           n_el += in[k] && x[k] != vo ? 1 : 0;
         }
@@ -2376,13 +2390,13 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
         continue;
       }
 #pragma unroll
-      for (int k = 0; k < 4; k++) n_el += in[k] ? 1 : 0;
+      for (int k = 0; k < U; k++) n_el += in[k] ? 1 : 0;
       r.elems += (unsigned)n_el;
       if (KIND == PAIR_COPY) {
-        bool hit[4];
-        int h[4];
+        bool hit[U];
+        int h[U];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           h[k] = __shfl_sync(FULL, h_v, own[k]);
           hit[k] = false;
           if (!LABELED) {
@@ -2392,16 +2406,16 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
         }
         if (!LABELED) bsearch4<false>(H0, len0, x, hit, false);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           if (!in[k]) continue;
           const int f = h[k] - (hit[k] ? 1 : 0);
           r.cnt += (unsigned)f;
           r.bytes += 4ull * (unsigned)(h[k] + f) + (LABELED ? (unsigned)h[k] : 0u);
         }
       } else if (KIND == PAIR_FRESH) {
-        int deg[4], f[4];
+        int deg[U], f[U];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           deg[k] = f[k] = 0;
           if (!in[k]) continue;
           const uint64_t xb = a.rowptr[x[k]];
@@ -2415,39 +2429,39 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
         }
         if (!LABELED) {
 #pragma unroll
-          for (int k = 0; k < 4; k++) f[k] = deg[k] - known - (__shfl_sync(FULL, v, own[k]) < ub_last ? 1 : 0);
+          for (int k = 0; k < U; k++) f[k] = deg[k] - known - (__shfl_sync(FULL, v, own[k]) < ub_last ? 1 : 0);
           for (int i = 0; i < n_ask; i++) {
             const int p = i == 0 ? pv[0] : i == 1 ? pv[1] : i == 2 ? pv[2] : pv[3];
             const unsigned* row = i == 0 ? prow[0] : i == 1 ? prow[1] : i == 2 ? prow[2] : prow[3];
-            bool hit[4];
+            bool hit[U];
 #pragma unroll
-            for (int k = 0; k < 4; k++) hit[k] = in[k];
+            for (int k = 0; k < U; k++) hit[k] = in[k];
             if (row) {
 #pragma unroll
-              for (int k = 0; k < 4; k++) hit[k] = in[k] && ((__ldg(row + (x[k] >> 5)) >> (x[k] & 31)) & 1u);
+              for (int k = 0; k < U; k++) hit[k] = in[k] && ((__ldg(row + (x[k] >> 5)) >> (x[k] & 31)) & 1u);
             } else {
               const uint64_t pb = a.rowptr[p];
               bsearch4<false>(a.colidx + pb, (int)(a.rowptr[p + 1] - pb), x, hit, false);
             }
 #pragma unroll
-            for (int k = 0; k < 4; k++) f[k] -= hit[k] ? 1 : 0;
+            for (int k = 0; k < U; k++) f[k] -= hit[k] ? 1 : 0;
           }
         }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           if (!in[k]) continue;
           r.cnt += (unsigned)f[k];
           r.bytes += 4ull * (unsigned)(deg[k] + f[k]) + (LABELED ? (unsigned)deg[k] : 0u);
         }
       } else {
-        int4 en[4];
+        int4 en[U];
 #pragma unroll
-        for (int k = 0; k < 4; k++)
+        for (int k = 0; k < U; k++)
           en[k] = in[k] ? *reinterpret_cast<const int4*>(S.memo + (x[k] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
         int c = 0, by = 0, lw = 0;  // this round's sums (lists are shorter than 2^28)
         unsigned missing = 0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < U; k++) {
           const int h = __shfl_sync(FULL, h_v, own[k]), l1 = LABELED ? 0 : __shfl_sync(FULL, less, own[k]);
           const bool hit = in[k] && en[k].x == x[k] && (unsigned)en[k].y == epoch;
           if (in[k]) {
@@ -2464,11 +2478,13 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
         r.cnt += (unsigned long long)(long long)c;
         r.bytes += (unsigned long long)(4ll * by + (LABELED ? lw : 0));
         if (__any_sync(FULL, missing)) {
-          for (int k = 0; k < 4; k++) {
+          for (int k = 0; k < U; k++) {
             const bool mk = (missing >> k) & 1u;
             const unsigned miss = __ballot_sync(FULL, mk);
             if (!miss) continue;
-            const int xk = k == 0 ? x[0] : k == 1 ? x[1] : k == 2 ? x[2] : x[3];
+            int xk = x[0];
+#pragma unroll
+            for (int i = 1; i < U; i++) xk = k == i ? x[i] : xk;
             if (mk) S.queue[queued + __popc(miss & lanemask_lt())] = xk;
             queued += __popc(miss);
             __syncwarp();
