@@ -2458,7 +2458,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
 #pragma unroll
         for (int k = 0; k < U; k++)
           en[k] = in[k] ? *reinterpret_cast<const int4*>(S.memo + (x[k] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
-        int c = 0, by = 0, lw = 0;  // this round's sums (lists are shorter than 2^28)
+        int c = 0, by = 0, lw = 0;  // sums of these elements (lists are shorter than 2^28)
         unsigned missing = 0;
 #pragma unroll
         for (int k = 0; k < U; k++) {
