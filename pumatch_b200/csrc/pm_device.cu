@@ -105,7 +105,8 @@ struct MatchArgs {
   int32_t pairs;                // last two levels in one pass where the plan allows (pair_levels)
   int32_t memo_entries;         // entries of a warp's value table (a power of two), and the tables: each
   MemoEntry* memo;              // warp's entries, then one that holds the last epoch it used (null: none)
-  const unsigned long long* asym;  // two words, 0 when every adjacency entry has its reverse and none comes twice
+  const unsigned long long* asym;  // two words, 0 when every adjacency entry has its reverse, none comes twice and
+                                   // none is its own vertex (maxnbrdeg_kernel)
   const int32_t* hub_slot;      // unlabeled, HBM: [n] bit row of a vertex with a long list, or -1 (null: none)
   const unsigned* hub_bits;     // bit rows of hub_words words: bit u of v's row = u is in v's list
   int32_t hub_words;
@@ -649,9 +650,10 @@ __device__ __forceinline__ int compact(const int32_t* A, int n, bool cg, int32_t
   return cnt;
 }
 
-// Whether u in N(v) says v in N(u), and each list holds an element once: an
-// undirected simple graph, as the interface asks for.  What is taken from one
-// list about the other, or from a bit about an element, asks first.
+// Whether u in N(v) says v in N(u), and each list holds an element once and
+// not its own vertex: an undirected simple graph, as the interface asks for.
+// What is taken from one list about the other, from a bit about an element, or
+// from a vertex's own list being without it, asks first.
 __device__ __forceinline__ bool symmetric(const MatchArgs& a) { return a.asym && (a.asym[0] | a.asym[1]) == 0ull; }
 
 // v's bit row (pm_graph::d_hub_bits), or null when its list is short.
@@ -3268,7 +3270,8 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
 
 // Also sums a hash of every entry's vertex pair into asym[0], with the sign of
 // the entry's direction: 0 when each entry has its reverse (and, but for one
-// graph in 2^64 or so, only then).  asym[1]: a list holds an element twice.
+// graph in 2^64 or so, only then).  asym[1]: bit 0 a list holds an element
+// twice, bit 1 a list holds its own vertex.
 __device__ __forceinline__ unsigned long long pair_hash(unsigned lo, unsigned hi) {
   uint64_t x = ((uint64_t)hi << 32 | lo) + 0x9E3779B97F4A7C15ull;
   return Rng::splitmix(x);
@@ -3279,7 +3282,7 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
   __shared__ int best[kListWarps];
   const int lane = lane_id();
   unsigned long long sum = 0;
-  bool twice = false;
+  bool twice = false, loop = false;
   auto walk = [&](long long v, uint64_t b, uint64_t e, uint64_t e_list) {
     int m = 0;
     for (uint64_t i0 = b; i0 < e; i0 += 128) {
@@ -3294,6 +3297,7 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
         m = max(m, (int)(rowptr[u[q] + 1] - rowptr[u[q]]));
         if (u[q] > v) sum += pair_hash((unsigned)v, (unsigned)u[q]);
         else if (u[q] < v) sum -= pair_hash((unsigned)u[q], (unsigned)v);
+        else loop = true;
       }
     }
     return __reduce_max_sync(FULL, m);
@@ -3315,7 +3319,8 @@ __global__ void __launch_bounds__(512) maxnbrdeg_kernel(const uint64_t* rowptr, 
             });
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
   if (lane == 0 && sum) atomicAdd(asym, sum);
-  if (__any_sync(FULL, twice) && lane == 0) atomicOr(asym + 1, 1ull);
+  const unsigned odd = (__any_sync(FULL, twice) ? 1u : 0u) | (__any_sync(FULL, loop) ? 2u : 0u);
+  if (odd && lane == 0) atomicOr(asym + 1, (unsigned long long)odd);
 }
 
 // Regroups each list by label, keeping id order within a label (a stable
