@@ -656,6 +656,10 @@ __device__ __forceinline__ int compact(const int32_t* A, int n, bool cg, int32_t
 // from a vertex's own list being without it, asks first.
 __device__ __forceinline__ bool symmetric(const MatchArgs& a) { return a.asym && (a.asym[0] | a.asym[1]) == 0ull; }
 
+// Whether each list holds an element once: then a list met with a slot of at
+// most T elements has at most T of them.
+__device__ __forceinline__ bool distinct(const MatchArgs& a) { return a.asym && (a.asym[1] & 1ull) == 0ull; }
+
 // v's bit row (pm_graph::d_hub_bits), or null when its list is short.
 __device__ __forceinline__ const unsigned* hub_row(const MatchArgs& a, int v) {
   if (!a.hub_slot || !symmetric(a)) return nullptr;
@@ -1154,7 +1158,8 @@ __device__ __forceinline__ bool on_path(const WarpState& S, int L, int v) {
 // per lane.  A lane finds the candidate owning its part's start once and
 // walks on through the following lists, four 128-bit loads in flight, testing
 // each element against B's structure in shared memory (leaf_build).  Counts
-// only.  Truncation needs no care here: B is a slot, at most T long already.
+// only.  Truncation needs no care here: B is a slot, at most T long already,
+// and the lists hold an element once (the caller asks: distinct).
 // Same set operations, counts and accounting as lane_intersect per candidate.
 // Batches averaging under 16 elements per lane, and a.leaf_flat == 2, use
 // the strided layout instead (element t0 + lane, owner found per element by
@@ -1297,7 +1302,7 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
       if (P.partial[s] & (1u << j)) common_ub = min(common_ub, S.path[j]);
     self_ub = (P.partial[s] >> Lf) & 1u;
   }
-  if (!PAGED && kind == SLOT_INTERSECT && a.leaf_flat) {
+  if (!PAGED && kind == SLOT_INTERSECT && a.leaf_flat && (!T || distinct(a))) {
     const int group = (LABELED && a.lab_off && __popc(mask) == 1) ? __ffs(mask) - 1 : -1;
     unsigned long long k;
     if (leaf_flat<LABELED>(a, S, L, holes, cand, b, e, B, lenB, S.id[par], mask, group, common_ub, self_ub, w, &k))
@@ -2119,8 +2124,10 @@ __device__ __noinline__ void meet_values(const MatchArgs& a, WarpState& S, const
 template <bool LABELED, bool PAGED>
 __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, const WarpState& S) {
   // (truncated: an unlabeled list's first T elements less the path vertices
-  // among them is not its length less them)
-  if (!P.pair || !a.pairs || (!LABELED && a.T && (P.pair == PAIR_FRESH || P.pair == PAIR_SHARED)) || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
+  // among them is not its length less them, and a labeled list that holds an
+  // element twice may meet a slot in more than T elements)
+  if (!P.pair || !a.pairs || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
+  if (a.T && (LABELED ? !distinct(a) : P.pair == PAIR_FRESH || P.pair == PAIR_SHARED)) return false;
   if (P.pair == PAIR_MEET) {
     if (PAGED || !a.memo) return false;
     const int n0 = S.size[P.pair_h0];

@@ -10,7 +10,7 @@ from pumatch_b200 import patterns as P
 pytestmark = pytest.mark.gpu
 
 SHAPES = {"P4": P.path(4), "house": P.house(), "house_tail": P.house_tail(1), "C4_tail": P.cycle_tail(4, 1),
-          "C5": P.cycle(5), "K4": P.clique(4), "K5": P.clique(5)}
+          "C4": P.cycle(4), "C5": P.cycle(5), "K4": P.clique(4), "K5": P.clique(5)}
 
 
 def entries(n, per, seed):
@@ -98,10 +98,11 @@ def ctx():
     c.close()
 
 
-def check(ctx, hg, shape, labeled, truncate, **kw):
+def check(ctx, hg, shape, labeled, truncate, paged=False, **kw):
     k, e = SHAPES[shape]
     p = pm.PatternPreprocessor(text=P.to_g(k, e, P.seeded_labels(k, 3, 5) if labeled else None), labeled=labeled)
-    g = pm.GraphPreprocessor.from_host(hg, labeled=labeled)
+    pool = dict(paged=True, page_bytes=4096, frame_pool_bytes=64 << 10) if paged else {}
+    g = pm.GraphPreprocessor.from_host(hg, labeled=labeled, **pool)
     try:
         got, st = ctx.match(g, [p], truncate=truncate, timeout_ms=60000, **kw)
         want = Search(hg, p, truncate).run(ctx.roots(g, p))
@@ -118,3 +119,14 @@ def test_vertices_in_their_own_lists(ctx, shape, step, truncate):
     e, n = entries(90, 4, 1)
     loops = [(v, v) for v in (range(0, n - 2, step) if step else [])] + [(n - 2, n - 2), (n - 1, n - 1)]
     check(ctx, host_graph(e + loops, n), shape, False, truncate)
+
+
+@pytest.mark.parametrize("truncate", [0, 5])
+@pytest.mark.parametrize("shape", ["P4", "C4", "C5", "house", "house_tail", "C4_tail", "K5"])
+@pytest.mark.parametrize("paged", [False, True])
+def test_labeled_elements_that_come_twice(ctx, shape, truncate, paged):
+    """A list that holds an element twice can meet a set of at most T elements in more than T."""
+    e, n = entries(90, 4, 1)
+    e += [x for a, b in e if a < b and (a * 7 + b) % 5 == 0 for x in ((a, b), (b, a))]
+    labels = (np.arange(n) * 7 % 5 % 3).astype(np.uint32)
+    check(ctx, host_graph(e, n, labels), shape, True, truncate, paged)
