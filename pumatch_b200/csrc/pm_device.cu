@@ -1538,10 +1538,14 @@ __device__ unsigned long long leaf_batch(const MatchArgs& a, const DPlan& P, War
 // counts the last level over X/Y's candidates -- the small sets of light
 // subtrees, where warp-wide set operations leave most lanes idle.  Same set
 // operations, counts and accounting as run_level + leaf_batch; unlabeled
-// plans of the shape DPlan.l2_x describes, no truncation, X's parent at most
-// lane_subtree_max long (it is staged in shared memory).
-__device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b, int e,
-                                           Work& w) {
+// plans of the shape DPlan.l2_x describes, X's parent at most lane_subtree_max
+// long (it is staged in shared memory); truncation needs no care where the
+// lists hold an element once (the caller asks: distinct).  Returns false,
+// having counted nothing, when a list that holds an element twice meets the
+// parent in more elements than the parent has: a lane's part holds no more.
+__device__ bool lane_subtree(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b, int e, Work& w,
+                             unsigned long long* total_cnt) {
+  const long long c0 = clock64();
   int32_t* arena = S.arena;
   const int lane = lane_id();
   const int Lq = L + 1;
@@ -1554,6 +1558,7 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
   const int32_t* cand = S.ptr[P.level_begin[L]];
   const bool holes = S.raw[P.level_begin[L]] != S.size[P.level_begin[L]];
   unsigned long long cnt = 0, bytes = 0, ops = 0;
+  bool over = false;
   const int i = b + lane;
   if (i < e && !(holes && on_path(S, L, cand[i]))) {
     const int v = cand[i];
@@ -1578,7 +1583,7 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
     const int lenAX = (ubX == INT_MAX) ? deg : lane_lower_bound(A, deg, ubX);
     int32_t* buf = arena + S.top[Lq] + lane * lenB1;
     int sizeX = 0, p = 0;
-    for (int x = 0; x < lenAX && p < lenB1; x++) {
+    for (int x = 0; x < lenAX && p < lenB1 && !over; x++) {
       const int val = A[x];
       int lo = p, step = 1;
       while (lo + step < lenB1 && Bs[lo + step] < val) { lo += step; step <<= 1; }
@@ -1588,11 +1593,13 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
         if (Bs[mid] < val) lo = mid + 1; else hi = mid;
       }
       p = lo;
-      if (p < lenB1 && Bs[p] == val) buf[sizeX++] = val;
+      if (p < lenB1 && Bs[p] == val) {
+        over = sizeX == lenB1;
+        if (!over) buf[sizeX++] = val;
+      }
     }
     bytes += 4ull * (unsigned long long)(lenAX + lenB1 + sizeX);
     ops++;
-    w.reads++;
     // Y: X itself or its prefix below Y's bound, charged as its own operation
     int sizeY = sizeX;
     if (Y >= 0) {
@@ -1622,6 +1629,8 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
       ops++;
     }
   }
+  if (__any_sync(FULL, over)) return false;
+  w.reads++;
   for (int o = 16; o; o >>= 1) {
     cnt += __shfl_xor_sync(FULL, cnt, o);
     bytes += __shfl_xor_sync(FULL, bytes, o);
@@ -1629,7 +1638,9 @@ __device__ unsigned long long lane_subtree(const MatchArgs& a, const DPlan& P, W
   }
   w.setops += ops;
   w.bytes += bytes;
-  return cnt;
+  *total_cnt = cnt;
+  w.leaf_cyc += (unsigned long long)(clock64() - c0);
+  return true;
 }
 
 // The rest of a clique search below one node of level L, in bit sets: the
@@ -2859,6 +2870,7 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
     // (labeled plans with levels of copies: what is searched here, for how many)
     const unsigned long long mul = LABELED && P.copy_next ? S.mul[L] : 1ull;
     bool subtree = false, bits = false;
+    unsigned long long lanes_cnt = 0;
     if constexpr (!LABELED && !PAGED) {
       const int hs = P.level_begin[L] + 1;
       // (seven vertices: two levels between a candidate and the last make one
@@ -2866,7 +2878,7 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
       // deadline; the level below takes over there)
       bits = a.clique_bits && P.clique && L + 4 <= n && (L + 6 > n || S.size[hs] <= 128) && symmetric(a) && it < iend && S.size[hs] <= PM_CLIQUE_MAX &&
              S.top[L + 1] + clique_words(S.size[hs]) <= S.cap;
-      subtree = !bits && P.l2_x >= 0 && L + 4 == n && it < iend && a.lane_subtree_max > 0 &&
+      subtree = !bits && P.l2_x >= 0 && L + 4 == n && it < iend && a.lane_subtree_max > 0 && (!a.T || distinct(a)) &&
                 S.size[P.parent[P.l2_x]] <= a.lane_subtree_max &&
                 S.top[L + 1] + 32ll * S.size[P.parent[P.l2_x]] <= S.cap;
     }
@@ -2910,12 +2922,9 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
       w.leaf_cyc += (unsigned long long)(clock64() - c0);
       if (lane == 0) S.iter[L] = e2;
       __syncwarp();
-    } else if (subtree) {
-      const int e2 = min(iend, it + 32);
-      const long long c0 = clock64();
-      cnt += lane_subtree(a, P, S, L, it, e2, w);
-      w.leaf_cyc += (unsigned long long)(clock64() - c0);
-      if (lane == 0) S.iter[L] = e2;
+    } else if (subtree && lane_subtree(a, P, S, L, it, min(iend, it + 32), w, &lanes_cnt)) {
+      cnt += lanes_cnt;
+      if (lane == 0) S.iter[L] = min(iend, it + 32);
       __syncwarp();
     } else if (it < iend && L + 1 == n - 2) {
       const int e2 = min(iend, it + PM_LEAF_BATCH);

@@ -10,7 +10,7 @@ from pumatch_b200 import patterns as P
 pytestmark = pytest.mark.gpu
 
 SHAPES = {"P4": P.path(4), "house": P.house(), "house_tail": P.house_tail(1), "C4_tail": P.cycle_tail(4, 1),
-          "C4": P.cycle(4), "C5": P.cycle(5), "K4": P.clique(4), "K5": P.clique(5)}
+          "C4": P.cycle(4), "C5": P.cycle(5), "K4": P.clique(4), "K5": P.clique(5), "K6": P.clique(6)}
 
 
 def entries(n, per, seed):
@@ -130,3 +130,14 @@ def test_labeled_elements_that_come_twice(ctx, shape, truncate, paged):
     e += [x for a, b in e if a < b and (a * 7 + b) % 5 == 0 for x in ((a, b), (b, a))]
     labels = (np.arange(n) * 7 % 5 % 3).astype(np.uint32)
     check(ctx, host_graph(e, n, labels), shape, True, truncate, paged)
+
+
+@pytest.mark.parametrize("truncate", [0, 5])
+@pytest.mark.parametrize("shape", ["K5", "K6"])
+@pytest.mark.parametrize("lane", [0, 512])
+def test_cliques_of_elements_that_come_twice(ctx, shape, truncate, lane):
+    """More of a doubled list is in the parent set than the set has elements: the scheme of one candidate per lane,
+    whose lanes have room for the set, leaves the node to the search."""
+    e, n = entries(70, 12, 3)
+    e += [x for a, b in e if a < b and (a + b) % 3 for x in ((a, b), (b, a))]
+    check(ctx, host_graph(e, n), shape, False, truncate, lane_subtree_max=lane)
