@@ -869,7 +869,8 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
       }
     };
     const unsigned* row = nullptr;
-    int room = kind == SLOT_INTERSECT ? min(lenA, lenB) : lenA;
+    // (a list that holds an element twice may meet B in more than lenB elements)
+    int room = kind == SLOT_INTERSECT && distinct(a) ? min(lenA, lenB) : lenA;
     if (T && room > T) room = T;
     int32_t* out = nullptr;
     bool fits = true;

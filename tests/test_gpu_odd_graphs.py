@@ -141,3 +141,14 @@ def test_cliques_of_elements_that_come_twice(ctx, shape, truncate, lane):
     e, n = entries(70, 12, 3)
     e += [x for a, b in e if a < b and (a + b) % 3 for x in ((a, b), (b, a))]
     check(ctx, host_graph(e, n), shape, False, truncate, lane_subtree_max=lane)
+
+
+@pytest.mark.parametrize("shape,labeled", [("K5", False), ("K6", False), ("house_tail", False), ("house", True), ("K5", True)])
+@pytest.mark.parametrize("words", [1, 80, 200])
+def test_small_arenas_and_elements_that_come_twice(ctx, shape, labeled, words):
+    """A doubled list can meet a set in more elements than the set has: the arena is asked for room for all of them
+    (a warp whose own is too small borrows a larger one)."""
+    e, n = entries(70, 12, 3)
+    e += [x for a, b in e if a < b and (a + b) % 3 for x in ((a, b), (b, a))]
+    labels = (np.arange(n) * 7 % 5 % 3).astype(np.uint32) if labeled else None
+    check(ctx, host_graph(e, n, labels), shape, labeled, 0, lane_subtree_max=-1, own_arena_words=words)
