@@ -148,7 +148,7 @@ struct MatchArgs {
   // ring slot of that number; a warp with work fills the oldest tickets' slots
   // of a group with (plan, root, level, begin, end, path[2..level])
   int4* don_items;                // 3 int4 per slot
-  unsigned long long* don_ready;  // per slot: 0 empty, ticket + 1 filled, kQuit no more work
+  unsigned long long* don_ready;  // per slot: 0 empty, kClaimed being filled, ticket + 1 filled, kQuit no more work
   unsigned long long* sched;      // per group, kSchedStride apart: (tickets drawn << 32) | pieces handed out
   unsigned long long* all_sched;  // the same over all groups
   unsigned int* started;          // warps that have begun
@@ -2668,6 +2668,8 @@ struct Donation {
 // that ends sooner than this is not worth handing out.
 #define PM_CHECK_CYCLES 4096
 constexpr unsigned kGroupSlots = 256;   // ring slots of a group
+constexpr unsigned long long kQuit = ~0ull;         // a slot's mark: no more work
+constexpr unsigned long long kClaimed = ~0ull - 1;  // a slot's mark: a piece is being written
 constexpr unsigned kSchedStride = 16;   // words from one group's sched to the next (a line of its own)
 #define PM_PAIR_PIECE 32  // shortest range of a two-level pass that is cut
 
@@ -2740,22 +2742,27 @@ __device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, const DPlan&
   first = __shfl_sync(FULL, first, 0);
   const int it = S.iter[k], len = S.iend[k] - it;
   // part 0 of q + 1 stays here, part lane + 1 goes out
-  unsigned err = 0;
-  if (lane < q) {
-    const int b = it + (int)((long long)len * (lane + 1) / (q + 1));
-    const int e = it + (int)((long long)len * (lane + 2) / (q + 1));
-    const unsigned long long slot = first + (unsigned long long)lane;
-    const unsigned at = g * kGroupSlots + (unsigned)(slot & (kGroupSlots - 1));
-    unsigned long long* ready = &a.don_ready[at];
-    // the slot's holder of one lap ago is reading it: a bounded wait
-    int spin = 0;
-    while (ld_acquire(ready) != 0ull && spin < (1 << 20)) { __nanosleep(64); spin++; }
-    if (spin == (1 << 20)) err = DEV_TIMEOUT;
-    int4* dst = a.don_items + 3 * at;
-    dst[0] = make_int4(plan_id, root_id, k, b);
-    dst[1] = make_int4(e, S.path[2], S.path[3], S.path[4]);
-    dst[2] = make_int4(S.path[5], S.path[6], (int)(unsigned)S.mul[k], (int)(unsigned)(S.mul[k] >> 32));
-    st_release(ready, slot + 1);
+  const int b = it + (int)((long long)len * (lane + 1) / (q + 1));
+  const int e = it + (int)((long long)len * (lane + 2) / (q + 1));
+  const unsigned long long slot = first + (unsigned long long)lane;
+  const unsigned at = g * kGroupSlots + (unsigned)(slot & (kGroupSlots - 1));
+  // A slot is claimed before it is written: it may hold the piece of a ticket a
+  // lap older or younger, which its taker is about to read, or another donor
+  // may be writing one (a group with more warps than slots).  Each is gone when
+  // its taker has read it: a bounded wait, in which no lane holds a claim.
+  bool done = lane >= q;
+  for (int spin = 0; spin < (1 << 20); spin++) {
+    if (!done && atomicCAS(&a.don_ready[at], 0ull, kClaimed) == 0ull) {
+      __threadfence();  // after the last taker's reads
+      int4* dst = a.don_items + 3 * at;
+      dst[0] = make_int4(plan_id, root_id, k, b);
+      dst[1] = make_int4(e, S.path[2], S.path[3], S.path[4]);
+      dst[2] = make_int4(S.path[5], S.path[6], (int)(unsigned)S.mul[k], (int)(unsigned)(S.mul[k] >> 32));
+      st_release(&a.don_ready[at], slot + 1);
+      done = true;
+    }
+    if (__all_sync(FULL, done)) break;
+    __nanosleep(64);
   }
   __syncwarp();
   if (lane == 0) {
@@ -2763,7 +2770,7 @@ __device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, const DPlan&
     atomicAdd(&a.stats[ST_SPLITS], (unsigned long long)q);
   }
   __syncwarp();
-  return __any_sync(FULL, err != 0) ? DEV_TIMEOUT : 0u;
+  return __all_sync(FULL, done) ? 0u : DEV_TIMEOUT;
 }
 
 // What was counted since (ops, bytes, reads) stands for m equal subtrees.
@@ -2958,8 +2965,6 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
   }
   return cnt;
 }
-
-constexpr unsigned long long kQuit = ~0ull;
 
 // Draws a ticket: the warp is out of work and will take the piece that lands
 // in the ticket's slot.  The warp whose ticket leaves none of the started
