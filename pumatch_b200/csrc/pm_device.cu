@@ -1561,7 +1561,8 @@ __device__ bool lane_subtree(const MatchArgs& a, const DPlan& P, WarpState& S, i
   unsigned long long cnt = 0, bytes = 0, ops = 0;
   bool over = false;
   const int i = b + lane;
-  if (i < e && !(holes && on_path(S, L, cand[i]))) {
+  const bool mine = i < e && !(holes && on_path(S, L, cand[i]));
+  if (mine) {
     const int v = cand[i];
     // slot bounds with path[Lq] = v: main slots take the smallest constrained
     // path vertex, helpers the largest (slot_bound)
@@ -1631,7 +1632,7 @@ __device__ bool lane_subtree(const MatchArgs& a, const DPlan& P, WarpState& S, i
     }
   }
   if (__any_sync(FULL, over)) return false;
-  w.reads++;
+  w.reads += __popc(__ballot_sync(FULL, mine));  // X's list for each candidate
   for (int o = 16; o; o >>= 1) {
     cnt += __shfl_xor_sync(FULL, cnt, o);
     bytes += __shfl_xor_sync(FULL, bytes, o);
@@ -1839,7 +1840,8 @@ __device__ __noinline__ void clique_rows(const MatchArgs& a, WarpState& S, const
 // slot's): matches below them.
 __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
                                                        int e, unsigned long long* ops_out,
-                                                       unsigned long long* bytes_out) {
+                                                       unsigned long long* bytes_out,
+                                                       unsigned long long* reads_out) {
   const int lane = lane_id();
   const int hs = P.level_begin[L] + 1;
   const int32_t* nb = S.ptr[hs];
@@ -1865,6 +1867,7 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
   }
   const int depth = P.nnodes - 4 - L;  // levels between the candidates' and the last
   unsigned long long cnt = 0, ops = 0, bytes = 0;  // per lane
+  unsigned reads = 0;  // nodes entered: the level-by-level search reads a list for each
   if (m <= 32) {
     // one candidate per lane, every set one word
     unsigned* rs = (unsigned*)S.sb;
@@ -1886,6 +1889,7 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
       auto node = [&](int v, int size_up, unsigned h, unsigned mm) {  // the two set operations of a level
         const int nh = __popc(h), nm = __popc(mm);
         ops += 2;
+        reads++;
         bytes += 4ull * (unsigned long long)(lm[v] + lh[v] + 2 * size_up + nh + nm);
       };
       node(i, m, H[0], M[0]);
@@ -1943,6 +1947,7 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
           else { H[2] = h; M[2] = mm; size[2] = nh; }
           if (lane == 0) {
             ops += 2;
+            reads++;
             bytes += 4ull * (unsigned long long)(len_m[v] + len_h[v] + 2 * size_up + nh + nm);
           }
           fresh = false;
@@ -2016,6 +2021,7 @@ __device__ __noinline__ unsigned long long clique_bits(const MatchArgs& a, const
   }
   *ops_out = ops;
   *bytes_out = bytes;
+  *reads_out = __reduce_add_sync(FULL, reads);
   return cnt;
 }
 
@@ -2922,11 +2928,11 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
       // may be long, the more so with levels between it and the last)
       const int e2 = min(iend, it + (S.size[P.level_begin[L] + 1] <= 32 ? 32 : L + 4 == n ? 8 : 1));
       const long long c0 = clock64();
-      unsigned long long ops, bytes;
-      cnt += clique_bits(a, P, S, L, it, e2, &ops, &bytes);
+      unsigned long long ops, bytes, reads;
+      cnt += clique_bits(a, P, S, L, it, e2, &ops, &bytes, &reads);
       w.setops += ops;
       w.bytes += bytes;
-      w.reads++;
+      w.reads += reads;
       w.leaf_cyc += (unsigned long long)(clock64() - c0);
       if (lane == 0) S.iter[L] = e2;
       __syncwarp();
