@@ -102,7 +102,6 @@ struct MatchArgs {
   int32_t leaf_flat;            // last level: 0 one candidate per lane, 1 flat in lane-contiguous parts,
                                 // 2 flat strided (leaf_flat)
   int32_t clique_bits;          // cliques in bit sets
-  int32_t pairs;                // last two levels in one pass where the plan allows (pair_levels)
   int32_t memo_entries;         // entries of a warp's value table (a power of two), and the tables: each
   MemoEntry* memo;              // warp's entries, then one that holds the last epoch it used (null: none)
   const unsigned long long* asym;  // two words, 0 when every adjacency entry has its reverse, none comes twice and
@@ -212,6 +211,8 @@ struct alignas(16) WarpState {
   unsigned long long memo_id;
   uint32_t memo_epoch;
   int32_t memo_len, memo_ub;
+  int32_t pair_take;             // candidates the last pass could take, by their lists' lengths (pair_pass)
+  int32_t pair_off;              // elements of the first candidate's list that passes have walked already
   int32_t lcnt[32];
   unsigned long long prb[32];    // the candidates' lists laid end to end: where each starts
   int32_t pexcl[33];             // and its offset in the row
@@ -2138,16 +2139,14 @@ __device__ __noinline__ void meet_values(const MatchArgs& a, WarpState& S, const
   __syncwarp();
 }
 
-// True when this node's last two levels can be taken in one pass.
+// True when this node's last two levels can be taken in one pass (DPlan.pair:
+// the launch's part of the answer).
 template <bool LABELED, bool PAGED>
 __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, const WarpState& S) {
-  // (truncated: an unlabeled list's first T elements less the path vertices
-  // among them is not its length less them, and a labeled list that holds an
-  // element twice may meet a slot in more than T elements)
-  if (!P.pair || !a.pairs || (LABELED ? !a.lab_off : PAGED || !symmetric(a))) return false;
-  if (a.T && (LABELED ? !distinct(a) : P.pair == PAIR_FRESH || P.pair == PAIR_SHARED)) return false;
+  // (a labeled list that holds an element twice may meet a truncated slot in
+  // more than T elements)
+  if (!P.pair || (LABELED ? a.T && !distinct(a) : !symmetric(a))) return false;
   if (P.pair == PAIR_MEET) {
-    if (PAGED || !a.memo) return false;
     const int n0 = S.size[P.pair_h0];
     return n0 <= PM_FILTER_MAX || (n0 > 0 && S.ptr[P.pair_h0][n0 - 1] < 32 * PM_SB_MAX);
   }
@@ -2158,7 +2157,16 @@ __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, c
   return true;
 }
 
-// Candidates [b, e) (at most 32) of level L = n-4's main slot.
+// Elements a pass walks at most: the lists of as many of its 32 candidates as
+// have this many together, or this much of one list.  A warp looks for waiting
+// warps and at the deadline between passes; with no such bound one over 32
+// hubs' lists took 19 ms (a 5-path on an R-MAT graph of 262,144 vertices), or
+// 136 ms where each element's list is walked in turn (the 5-cycle with 4
+// labels); with it 3 and 25 ms.  Half as many cost the 6-cycle shard 8% (38.1
+// -> 41 ms), a look from inside the walks the 20-pattern batch 5%; this costs
+// the batch 3.5% (19.0 -> 19.7 ms).
+constexpr int kPairRow = 4096;
+
 template <int N>
 __device__ __forceinline__ bool any_of(const bool (&in)[N]) {
   bool any = false;
@@ -2167,9 +2175,13 @@ __device__ __forceinline__ bool any_of(const bool (&in)[N]) {
   return any;
 }
 
+// Candidates [b, e) (at most 32) of level L = n-4's main slot, or the first of
+// them, or a part of the first one's list; with off > 0 the rest of b's list
+// from there, b's own operations counted before.  S.iter[L] and S.pair_off say
+// where the next pass goes on.
 template <bool LABELED, bool PAGED, int KIND, bool MET>
 __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const DPlan& P, WarpState& S, int L, int b,
-                                                     int e, Work* wt) {
+                                                     int e, int off, Work* wt) {
   Work& w = *wt;
   const int lane = lane_id();
   const int q = L + 1;
@@ -2223,7 +2235,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
   const int32_t* cand = S.ptr[P.level_begin[L]];
   const bool holes = !LABELED && S.raw[P.level_begin[L]] != S.size[P.level_begin[L]];
   const int v = b + lane < e ? cand[b + lane] : -1;
-  const bool mine = v >= 0 && !(holes && on_path(S, L, v));
+  bool mine = v >= 0 && !(holes && on_path(S, L, v));
   unsigned long long rb = 0;
   int len = 0;     // elements of v's list to look at
   int h_v = 0;     // |h| under v (a copy's or a meeting's second operand)
@@ -2266,7 +2278,6 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       r.bytes += 4ull * (unsigned long long)(len_h + h_v) + (LABELED ? (unsigned long long)len_h : 0ull);
     }
   }
-  if (KIND != PAIR_SHARED) w.reads += __popc(__ballot_sync(FULL, mine));
   // PAIR_FRESH: path vertices whose adjacency to x has to be looked up
   int pv[4];
   const unsigned* prow[4];
@@ -2337,21 +2348,50 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       r.bytes += 4ull * ((unsigned long long)lenBm + k) + 4ull * (deg + f);
     }
   }
+  if (off) {  // the rest of a list whose operations are counted
+    r = PairSums{0, 0, 0};
+    ops = 0;
+    rb += (unsigned)off;
+    len -= mine ? off : 0;
+    mine = false;
+  }
   // walk
   int queued = 0;
-  int total = len;
+  int total = len, next = e, next_off = 0, pair_take = 32;
   if (!PAGED) {
-    int incl = len;
+    int incl = min(len, 1 << 25);  // (the sum of 32 is an int; as long a list is taken by itself, in parts)
     for (int d = 1; d < 32; d <<= 1) {
       const int t = __shfl_up_sync(FULL, incl, d);
       if (lane >= d) incl += t;
     }
     total = __shfl_sync(FULL, incl, 31);
+    if (total > kPairRow) {
+      const int whole = __popc(__ballot_sync(FULL, incl <= kPairRow));  // candidates whose lists fit
+      const int take = max(1, whole);
+      if (lane >= take) {
+        mine = false;
+        r = PairSums{0, 0, 0};
+        ops = 0;
+      }
+      if (lane >= whole) len = incl = 0;
+      next = b + whole;
+      next_off = whole ? 0 : off + kPairRow;
+      pair_take = take;
+      if (whole == 0 && lane == 0) len = kPairRow;
+      total = __shfl_sync(FULL, whole ? incl : kPairRow, take - 1);
+      incl = lane < whole ? incl : total;
+    }
     S.prb[lane] = rb;
     S.pexcl[lane] = incl - len;
     if (lane == 31) S.pexcl[32] = total;
     __syncwarp();
   }
+  if (lane == 0) {
+    S.iter[L] = next;
+    S.pair_off = next_off;
+    S.pair_take = pair_take;
+  }
+  if (KIND != PAIR_SHARED) w.reads += __popc(__ballot_sync(FULL, mine));
   const int32_t* lists = LABELED ? a.colidx_lab : a.colidx;
   constexpr int U = 2;  // elements per lane in flight
   // (paged: one resolved list after the other)
@@ -2648,17 +2688,17 @@ __device__ __forceinline__ unsigned long long chain_sum(const DPlan& P, const in
 
 template <bool LABELED, bool PAGED>
 __device__ __forceinline__ unsigned long long pair_levels(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
-                                                          int b, int e, Work* w) {
+                                                          int b, int e, int off, Work* w) {
   const bool met = P.kind[P.level_begin[L + 1]] == SLOT_INTERSECT;
   if constexpr (!PAGED)
-    if (P.pair == PAIR_MEET) return pair_pass<LABELED, PAGED, PAIR_MEET, false>(a, P, S, L, b, e, w);
+    if (P.pair == PAIR_MEET) return pair_pass<LABELED, PAGED, PAIR_MEET, false>(a, P, S, L, b, e, off, w);
   if constexpr (!LABELED && !PAGED)
-    if (P.pair == PAIR_SHARED) return pair_pass<LABELED, PAGED, PAIR_SHARED, true>(a, P, S, L, b, e, w);
+    if (P.pair == PAIR_SHARED) return pair_pass<LABELED, PAGED, PAIR_SHARED, true>(a, P, S, L, b, e, off, w);
   if (P.pair == PAIR_COPY)
-    return met ? pair_pass<LABELED, PAGED, PAIR_COPY, true>(a, P, S, L, b, e, w)
-               : pair_pass<LABELED, PAGED, PAIR_COPY, false>(a, P, S, L, b, e, w);
-  return met ? pair_pass<LABELED, PAGED, PAIR_FRESH, true>(a, P, S, L, b, e, w)
-             : pair_pass<LABELED, PAGED, PAIR_FRESH, false>(a, P, S, L, b, e, w);
+    return met ? pair_pass<LABELED, PAGED, PAIR_COPY, true>(a, P, S, L, b, e, off, w)
+               : pair_pass<LABELED, PAGED, PAIR_COPY, false>(a, P, S, L, b, e, off, w);
+  return met ? pair_pass<LABELED, PAGED, PAIR_FRESH, true>(a, P, S, L, b, e, off, w)
+             : pair_pass<LABELED, PAGED, PAIR_FRESH, false>(a, P, S, L, b, e, off, w);
 }
 
 // A donated piece of a DFS: candidates [begin, end) of level `level`'s main
@@ -2677,7 +2717,6 @@ constexpr unsigned kGroupSlots = 256;   // ring slots of a group
 constexpr unsigned long long kQuit = ~0ull;         // a slot's mark: no more work
 constexpr unsigned long long kClaimed = ~0ull - 1;  // a slot's mark: a piece is being written
 constexpr unsigned kSchedStride = 16;   // words from one group's sched to the next (a line of its own)
-#define PM_PAIR_PIECE 32  // shortest range of a two-level pass that is cut
 
 __device__ __forceinline__ unsigned long long ld_vol_u64(const unsigned long long* p) {
   return *(const volatile unsigned long long*)p;
@@ -2721,10 +2760,13 @@ __device__ __noinline__ unsigned publish_pieces(const MatchArgs& a, const DPlan&
         if ((P.copy_next >> k) & 1u) continue;  // one of its candidates is searched for all
         const int len = S.iend[k] - S.iter[k];
         // a candidate before a chain is one table entry: nothing to hand out;
-        // one of a pass over the last two levels is a list, worth more than the
-        // prefix its taker repeats only in numbers
+        // those of a pass over the last two levels are lists, worth the prefix
+        // their taker repeats in the number that a pass takes; where each warp
+        // keeps values of its own (PAIR_MEET), in fewer than 32 they are worked
+        // out again too often
         if (P.chain && k + 1 == P.chain_from) continue;
-        const int unit = (k + 1 == n - 2) ? max(S.split, 2) : (P.pair && a.pairs && k + 4 == n) ? PM_PAIR_PIECE : 2;
+        const int unit = (k + 1 == n - 2) ? max(S.split, 2)
+                         : !P.pair || k + 4 != n ? 2 : P.pair == PAIR_MEET ? 32 : max(2, S.pair_take);
         if (len < unit) continue;
         q = min(min(want, waiting), 2 * len / unit - 1);  // >= 1
         break;
@@ -2912,16 +2954,16 @@ __device__ unsigned long long dfs_from(const MatchArgs& a, const DPlan& P, WarpS
     if (chain) {
       // done above
     } else if (!bits && it < iend && L + 4 == n && pair_ready<LABELED, PAGED>(a, P, S)) {
-      const int e2 = min(iend, it + 32);
+      const int off = S.pair_off;
+      const int e2 = off ? it + 1 : min(iend, it + 32);
       const long long c0 = clock64();
       Work t;
       memset(&t, 0, sizeof(t));
-      cnt += mul * pair_levels<LABELED, PAGED>(a, P, S, L, it, e2, &t);
+      cnt += mul * pair_levels<LABELED, PAGED>(a, P, S, L, it, e2, off, &t);
       add_work(w, t);
       if (LABELED && P.copy_next) scale_work(w, ops0, bytes0, reads0, mul);
       w.leaf_cyc += (unsigned long long)(clock64() - c0);
-      if (lane == 0) S.iter[L] = e2;
-      __syncwarp();
+      __syncwarp();  // (where to go on: pair_pass wrote it)
       if (w.err) return 0;
     } else if (bits) {
       // (a look for waiting warps between: every candidate below a large set
@@ -3083,6 +3125,8 @@ __global__ void __launch_bounds__(MINB == 1 ? 512 : 256, MINB) match_kernel(cons
     S.memo_id = 0;
     S.memo_len = -1;
     S.memo_ub = 0;
+    S.pair_take = 32;
+    S.pair_off = 0;
     for (int k = 0; k < 16; k++) S.ptr[k] = nullptr;
     S.t_start = global_ns();
     S.arena = own;
@@ -4471,7 +4515,15 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.labels = g->d_labels;
   a.colidx_lab = g->d_colidx_lab;
   a.lab_off = g->d_lab_off;
-  a.pairs = o.leaf_per_lane == 0;
+  // plans whose last two levels this launch does not take in one pass
+  // (truncated: an unlabeled list's first T elements less the path vertices
+  // among them is not its length less them)
+  for (int i = 0; i < nplans; i++) {
+    uint8_t& pair = L->dp[i].pair;
+    if (o.leaf_per_lane != 0 || (L->labeled ? !g->d_lab_off : L->paged) ||
+        (!L->labeled && T && (pair == PAIR_FRESH || pair == PAIR_SHARED)) || (pair == PAIR_MEET && (L->paged || !*memo)))
+      pair = PAIR_NONE;
+  }
   a.asym = g->n > 0 ? asym_word(g) : nullptr;
   a.memo = *memo;
   a.memo_entries = L->memo_entries;
@@ -4912,6 +4964,7 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   if (blocks < 1) return fail(PM_ERR_INTERNAL, "pm_match_static: no room for a block of arenas");
 
   DPlan dp = to_dplan(p);
+  dp.pair = PAIR_NONE;  // (no symmetry words, label groups or value tables here)
   dp.roots = roots;
   dp.nroots = (int64_t)nroots;
   MatchArgs a;

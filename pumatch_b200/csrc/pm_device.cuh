@@ -44,7 +44,7 @@ struct DPlan {
   int8_t l2_x, l2_y;
   uint8_t leaf_adj;               // path vertices adjacent to every candidate for vertex nnodes-2 (bit j: v_j)
   uint8_t clique;                 // the plan is an unlabeled clique's (clique_bits)
-  uint8_t pair;                   // PairKind of the last two levels (pair_levels), 0: none
+  uint8_t pair;                   // PairKind of the last two levels (pair_levels), 0: none, or not in this launch
   int8_t pair_h0;                 // the slot its copy or meeting reads
   uint8_t copy_next;              // labeled: bit L: level L+1 is all copies (one candidate searched for all)
   int8_t chain_from;              // labeled: first of the fresh levels the plan ends in, 0: none (chain_kernel)
