@@ -18,6 +18,14 @@
 
 namespace pm {
 
+// Longest list of a graph whose lists are walked 32 to a row, laid end to end:
+// positions in the row are ints, and so are the sums over two elements of
+// three lengths each (pair_pass).  Graphs with longer lists take them one by
+// one (leaf_batch), in 64-bit sums.
+constexpr int32_t kRowListMax = (1 << 26) - 1;
+static_assert(32ll * kRowListMax <= INT32_MAX && 2ll * 3 * kRowListMax <= INT32_MAX, "row positions and sums");
+constexpr bool rows_of_lists(int32_t maxdeg) { return maxdeg <= kRowListMax; }
+
 // ---------------------------------------------------------------- errors
 // Sets the calling thread's last-error message and returns the status.
 pm_status fail(pm_status s, const char* fmt, ...);

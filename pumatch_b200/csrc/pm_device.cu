@@ -2525,7 +2525,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
 #pragma unroll
         for (int k = 0; k < U; k++)
           en[k] = in[k] ? *reinterpret_cast<const int4*>(S.memo + (x[k] & (a.memo_entries - 1))) : make_int4(-1, 0, 0, 0);
-        int c = 0, by = 0, lw = 0;  // sums of these elements (lists are shorter than 2^28)
+        int c = 0, by = 0, lw = 0;  // sums of these elements (an int holds them: kRowListMax)
         unsigned missing = 0;
 #pragma unroll
         for (int k = 0; k < U; k++) {
@@ -4407,7 +4407,8 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   // (what the buffers of an earlier call hold needs no look at free memory: a
   // query of 50 us spends as much again on asking)
   bool meets = false;
-  for (int i = 0; i < nplans; i++) meets = meets || (L->dp[i].pair == PAIR_MEET && !L->paged && o.leaf_per_lane == 0);
+  for (int i = 0; i < nplans; i++)
+    meets = meets || (L->dp[i].pair == PAIR_MEET && !L->paged && o.leaf_per_lane == 0 && rows_of_lists(g->maxdeg));
   size_t free_b = 0, total_b = 0;
   const bool fits = !borrowing && (size_t)(L->warps * arena_words * 4) + 256 <= *arena_bytes && *arena &&
                     (!meets || (mt->d && mt->warps == L->warps && mt->entries == memo_entries_for(g->n)));
@@ -4531,7 +4532,7 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.hub_bits = g->d_hub_bits;
   a.hub_words = (int32_t)((g->n + 31) / 32);
   a.host_sorted = (g->residency == PM_RESIDENT_PAGED && g->d_lab_off) ? g->h_colidx_dev : nullptr;
-  a.leaf_flat = o.leaf_per_lane == 1 ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
+  a.leaf_flat = o.leaf_per_lane == 1 || !rows_of_lists(g->maxdeg) ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
   a.clique_bits = o.lane_subtree_max == 0;
   a.nl1 = g->nl1;
@@ -4973,7 +4974,7 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.rowptr = d_rowptr;
   a.colidx = d_colidx;
   a.labels = d_labels;
-  a.leaf_flat = o.leaf_per_lane == 1 ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
+  a.leaf_flat = o.leaf_per_lane == 1 || !rows_of_lists(max_degree) ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
   a.clique_bits = o.lane_subtree_max == 0;
   a.n = (int32_t)n;
