@@ -779,16 +779,24 @@ extern "C" pm_status pm_root_features(pm_ctx* c, const pm_graph* g, const pm_pla
   if (cap < n) return fail(PM_ERR_INVALID, "pm_root_features: feature buffer holds %lld roots, need %lld",
                            (long long)cap, (long long)n);
   const Plan* pl = plan_of(p);
-  // a row per vertex, unless the graph is so large that they would not pay
-  const bool by_vertex = pl->labeled && (size_t)g->n * NIN * sizeof(float) <= (1ull << 30);
-  const size_t want = 1024 + (by_vertex ? (size_t)g->n * NIN * sizeof(float) : 0);
-  if (c->feat_bytes < want) {
+  // a row per vertex, unless the graph is so large that they would not pay or
+  // there is no room for them: then the features of each root by itself
+  const size_t rows_bytes = pl->labeled ? (size_t)g->n * NIN * sizeof(float) : 0;
+  bool by_vertex = rows_bytes > 0 && rows_bytes <= (1ull << 30);
+  auto grow = [&](size_t want) {
+    if (c->feat_bytes >= want) return cudaSuccess;
     cudaFree(c->d_feat);
     c->d_feat = nullptr;
     c->feat_bytes = 0;
-    CKL(cudaMalloc(&c->d_feat, want));
-    c->feat_bytes = want;
+    const cudaError_t e = cudaMalloc(&c->d_feat, want);
+    if (e == cudaSuccess) c->feat_bytes = want;
+    return e;
+  };
+  if (by_vertex && grow(1024 + rows_bytes) == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    by_vertex = false;
   }
+  CKL(grow(1024));
   unsigned int* cdf = (unsigned int*)c->d_feat;
   float* rows = (float*)((char*)c->d_feat + 1024);
   const int32_t* colidx = g->residency == PM_RESIDENT_HBM ? g->d_colidx : g->h_colidx_dev;
