@@ -3789,6 +3789,26 @@ int lane_subtree_limit(const pm_run_opts& o) {
   return o.lane_subtree_max < 0 ? 0 : (o.lane_subtree_max == 0 ? 64 : std::min(o.lane_subtree_max, PM_SB_MAX));
 }
 
+// Whether the tables of a plan's chain (chain_kernel), which are worked out for
+// every vertex of a label in each launch, take less time than searching the
+// chain below this launch's roots.  How often a root reaches the chain and how
+// much is below it grows with the fresh levels of either; measured (B200,
+// kernel ms with tables / without, R-MAT, at the start and in the middle of the
+// root list), a table costs as much as searching 1 root for every 8 vertices of
+// the label where the chain is all and one table deep (4-path: 64M edges on 4M
+// vertices, 8 labels, 65,536 roots 1.07 / 0.67 and 1.06 / 0.88, 256 roots 1.03 /
+// 0.18 and 1.02 / 0.16; 32 labels, 4,096 roots 0.12 / 0.10); with one such
+// level more a single root is worth some 30,000 (4-cycle with a two-vertex
+// tail, 8 labels: 1 root 1.57 / 2.64 and 1.05 / 0.33, 16 roots 2.1 / 8.5); with
+// two more tables always pay where it matters (5-cycle with the same tail, 1
+// root 6.2 / 141 and 1.09 / 0.22).
+bool chain_pays(const Plan& p, const DPlan& d, int64_t roots, int64_t label_vertices) {
+  if (!d.chain_from) return false;
+  int fresh = d.nnodes - 3 - d.chain_from;  // tables but one, then the fresh main slots before the chain
+  for (int l = 1; l < d.chain_from; l++) fresh += d.kind[p.level_begin[l]] == SLOT_FRESH;
+  return fresh > 1 || roots * (fresh ? 32768 : 8) >= label_vertices;
+}
+
 // Worst-case arena words one warp needs for a plan: every materialised slot
 // is at most its first operand, itself at most a max-degree list.
 int64_t arena_words_for(const Plan& p, int32_t maxdeg, int T) {
@@ -4451,6 +4471,8 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
     const size_t table = sizeof(ulonglong4) * (size_t)g->n;
     size_t need = 0;
     for (int i = 0; i < nplans; i++) {
+      if (!chain_pays(*L->plans[i], L->dp[i], L->dp[i].nroots / shard_count, g->n / std::max(1, g->nlabels)))
+        L->dp[i].chain_from = 0;
       const size_t levels = L->dp[i].chain_from ? (size_t)(L->dp[i].nnodes - 2 - L->dp[i].chain_from) : 0;
       if (need + levels * table > (1ull << 30)) L->dp[i].chain_from = 0;
       else need += levels * table;
