@@ -316,18 +316,25 @@ typedef struct {
                                capped at 64 registers (four 256-thread
                                blocks per SM); 2 capped at 85 (three blocks
                                per SM); 3 uncapped (up to 128, no spills)    */
-  int32_t leaf_per_lane;    /* 1: last-level intersections one candidate per
-                               lane (long lists go to the warp); 0 (default):
-                               work-balanced across the warp when the common
-                               operand fits in shared memory, each lane
-                               walking a contiguous part of the candidates'
-                               lists; 2: the same, strided (lane l takes
-                               every 32nd element)                           */
+  int32_t leaf_per_lane;    /* 0 (default): the last two levels in one pass
+                               where the plan allows, with values kept per
+                               warp; labeled tails from tables per vertex
+                               where the launch has the roots for them; else
+                               the last level work-balanced across the warp,
+                               each lane walking a contiguous part of the
+                               candidates' lists.  1: level by level, the last
+                               level's intersections one candidate per lane
+                               (long lists go to the warp).  2: level by
+                               level, the last one work-balanced, strided
+                               (lane l takes every 32nd element)             */
   int32_t lane_subtree_max; /* unlabeled plans ending in a chain of
                                intersections (cliques): the last two levels
                                run one candidate per lane when the parent set
-                               is at most this long; 0 = default (64), -1 =
-                               never                                          */
+                               is at most this long.  0 or 64 = default:
+                               cliques of five vertices and more in bit sets
+                               first (simple undirected graphs in device
+                               memory).  Other values, and -1 = never, leave
+                               the bit sets out too                           */
   uint64_t* root_counts;    /* optional device ptr: per-root counts (plan 0) */
   float* root_cost;         /* optional device ptr: per-root set-op bytes    */
   const int32_t* root_order;/* optional device ptr: process roots in this

@@ -3784,9 +3784,12 @@ RootFilter to_filter(const Plan& p) {
 }
 
 // Parent-set limit of the two-level lane scheme from the run options: 0 =
-// default (64), negative = never, else capped at the shared staging size.
+// default, negative = never, else capped at the shared staging size.  The
+// default takes cliques in bit sets first.
+constexpr int kLaneSubtreeDefault = 64;
 int lane_subtree_limit(const pm_run_opts& o) {
-  return o.lane_subtree_max < 0 ? 0 : (o.lane_subtree_max == 0 ? 64 : std::min(o.lane_subtree_max, PM_SB_MAX));
+  if (o.lane_subtree_max < 0) return 0;
+  return o.lane_subtree_max == 0 ? kLaneSubtreeDefault : std::min(o.lane_subtree_max, PM_SB_MAX);
 }
 
 // Whether the tables of a plan's chain (chain_kernel), which are worked out for
@@ -4556,7 +4559,7 @@ static pm_status setup_launch(pm_ctx* c, const pm_graph* g, const pm_plan* const
   a.host_sorted = (g->residency == PM_RESIDENT_PAGED && g->d_lab_off) ? g->h_colidx_dev : nullptr;
   a.leaf_flat = o.leaf_per_lane == 1 || !rows_of_lists(g->maxdeg) ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
-  a.clique_bits = o.lane_subtree_max == 0;
+  a.clique_bits = a.lane_subtree_max == kLaneSubtreeDefault;
   a.nl1 = g->nl1;
   a.n = (int32_t)g->n;
   a.nplans = nplans;
@@ -4998,7 +5001,7 @@ extern "C" pm_status pm_match_static(const uint64_t* d_rowptr, const int32_t* d_
   a.labels = d_labels;
   a.leaf_flat = o.leaf_per_lane == 1 || !rows_of_lists(max_degree) ? 0 : (o.leaf_per_lane == 2 ? 2 : 1);
   a.lane_subtree_max = lane_subtree_limit(o);
-  a.clique_bits = o.lane_subtree_max == 0;
+  a.clique_bits = a.lane_subtree_max == kLaneSubtreeDefault;
   a.n = (int32_t)n;
   a.nplans = 1;
   a.T = T;
