@@ -3822,9 +3822,16 @@ int64_t arena_words_for(const Plan& p, int32_t maxdeg, int T) {
 
 }  // namespace
 
-// d_maxnbrdeg: n entries and, after them, the two 64-bit words in which
-// maxnbrdeg_kernel notes what the lists are like.
+// What a graph keeps per vertex besides its rows, in one allocation (from the
+// host: at the end of the rows' own, place_rows -- an allocation and its release
+// take longer than the passes that fill it): d_maxnbrdeg, n entries; the two
+// 64-bit words in which maxnbrdeg_kernel notes what the lists are like;
+// unlabeled in HBM, 33 degree counts (36 words) and d_hub_slot.
 static size_t maxnbrdeg_bytes(int64_t n) { return sizeof(int32_t) * (size_t)((n + 1) & ~1ll) + 16; }
+static bool takes_hub_rows(const pm_graph* g) { return !g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0; }
+static size_t aux_bytes(const pm_graph* g) {
+  return maxnbrdeg_bytes(g->n) + (takes_hub_rows(g) ? sizeof(int32_t) * (size_t)(36 + g->n) : 0);
+}
 static unsigned long long* asym_word(const pm_graph* g) {
   return reinterpret_cast<unsigned long long*>(g->d_maxnbrdeg + ((g->n + 1) & ~1ll));
 }
@@ -3846,28 +3853,25 @@ pm_status compute_maxnbrdeg(pm_graph* g, const int32_t* colidx) {
 
 static pm_status graph_finish(pm_graph* g) {
   // per-vertex max neighbour degree, used by the root filter
-  CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
+  if (!g->d_maxnbrdeg) CK(cudaMalloc(&g->d_maxnbrdeg, aux_bytes(g)));
   g->device_bytes += sizeof(int32_t) * g->n;
+  const bool rows_wanted = takes_hub_rows(g) && g->nadj > 0;
+  unsigned int* bins = reinterpret_cast<unsigned int*>(asym_word(g) + 2);
   if (g->n > 0 && g->residency == PM_RESIDENT_HBM) {
     PM_CK_PENDING("max neighbour degree");
-    CK(cudaMemset(asym_word(g), 0, 16));
+    CK(cudaMemset(asym_word(g), 0, 16 + (rows_wanted ? 33 * sizeof(unsigned int) : 0)));
     maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
-    CK(cudaDeviceSynchronize());
+    if (!rows_wanted) CK(cudaDeviceSynchronize());  // (else the degree counts' copy waits)
   }
-  if (!g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0 && g->nadj > 0) {
+  if (rows_wanted) {
     // Bit rows for the vertices with the longest lists: the lowest power of
     // two of a degree from 64 on (shorter lists are read as fast as a row)
     // from which all rows fit as many bytes as the adjacency array, or 64 MB
     // if that is more, and 256 MB at most -- half of them stay in L2.
-    unsigned int* bins = nullptr;
     unsigned int h[33];
-    CK(cudaMalloc(&bins, sizeof(h)));
-    cudaError_t e = cudaMemset(bins, 0, sizeof(h));
-    if (e == cudaSuccess) {
-      degree_bins_kernel<<<256, 256>>>(g->d_rowptr, g->n, bins);
-      e = cudaGetLastError();
-    }
+    degree_bins_kernel<<<256, 256>>>(g->d_rowptr, g->n, bins);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(h, bins, sizeof(h), cudaMemcpyDeviceToHost);
     const int64_t words = (g->n + 31) / 32;
     const size_t budget = std::min<size_t>(256ull << 20, std::max<size_t>(64ull << 20, 4 * (size_t)g->nadj));
@@ -3875,11 +3879,10 @@ static pm_status graph_finish(pm_graph* g) {
     int k = 31;
     for (; e == cudaSuccess && k > 6 && (rows + h[k - 1]) * words * 4 <= budget; k--) rows += h[k - 1];
     if (e == cudaSuccess && rows) {
-      e = cudaMalloc(&g->d_hub_slot, sizeof(int32_t) * g->n);
-      if (e == cudaSuccess) e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
+      g->d_hub_slot = reinterpret_cast<int32_t*>(bins + 36);
+      e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
       if (e == cudaErrorMemoryAllocation) {  // no room: the graph does without
         (void)cudaGetLastError();
-        free_dev(g->d_hub_slot);
         g->d_hub_slot = nullptr;
         g->d_hub_bits = nullptr;
         rows = 0;
@@ -3894,7 +3897,6 @@ static pm_status graph_finish(pm_graph* g) {
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
       if (rows) g->device_bytes += sizeof(int32_t) * g->n + rows * words * 4;
     }
-    cudaFree(bins);
     CK(e);
   }
   if (g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0) {
@@ -3985,7 +3987,8 @@ static pm_status place_rows(pm_graph* g, int64_t n, int64_t nadj, const uint64_t
   int32_t maxd = 0;
   for (int64_t v = 0; v < n; v++) maxd = std::max<int32_t>(maxd, (int32_t)(rowptr[v + 1] - rowptr[v]));
   g->maxdeg = maxd;
-  CK(cudaMalloc(&g->d_rowptr, sizeof(uint64_t) * (n + 1)));
+  CK(cudaMalloc(&g->d_rowptr, sizeof(uint64_t) * (n + 1) + aux_bytes(g)));
+  g->d_maxnbrdeg = reinterpret_cast<int32_t*>(g->d_rowptr + n + 1);
   CK(cudaMemcpy(g->d_rowptr, rowptr, sizeof(uint64_t) * (n + 1), cudaMemcpyHostToDevice));
   g->device_bytes += sizeof(uint64_t) * (n + 1);
   if (g->labeled) {
@@ -4020,7 +4023,6 @@ extern "C" pm_status pm_graph_from_host(int64_t n, int64_t nadj, const uint64_t*
   if (o.residency == PM_RESIDENT_PAGED) {
     st = paged_place(g.get(), colidx, &o, nullptr);
     if (st != PM_OK) return st;
-    CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
     g->device_bytes += sizeof(int32_t) * g->n;
     st = paged_maxnbrdeg(g.get());
     if (st != PM_OK) return st;
@@ -4065,7 +4067,6 @@ extern "C" pm_status pm_graph_from_paged_source(int64_t n, int64_t nadj, const u
   // the id-sorted lists: root filter, features, and a labeled graph's whole
   // lists (read in place)
   g->h_colidx_dev = const_cast<int32_t*>(sorted);
-  CK(cudaMalloc(&g->d_maxnbrdeg, maxnbrdeg_bytes(g->n)));
   g->device_bytes += sizeof(int32_t) * g->n;
   st = paged_maxnbrdeg(g.get());
   if (st != PM_OK) return st;
@@ -4143,10 +4144,9 @@ extern "C" void pm_graph_close(pm_graph* g) {
     free_dev(g->d_colidx);
     free_dev(g->d_labels);
   }
-  free_dev(g->d_maxnbrdeg);
+  if (!g->owns) free_dev(g->d_maxnbrdeg);  // else a part of the rows' allocation
   free_dev(g->d_colidx_lab);
   free_dev(g->d_lab_off);
-  free_dev(g->d_hub_slot);
   free_dev(g->d_hub_bits);
   paged_release(g);
   delete g;
