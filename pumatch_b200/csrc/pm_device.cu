@@ -3826,7 +3826,8 @@ int64_t arena_words_for(const Plan& p, int32_t maxdeg, int T) {
 // host: at the end of the rows' own, place_rows -- an allocation and its release
 // take longer than the passes that fill it): d_maxnbrdeg, n entries; the two
 // 64-bit words in which maxnbrdeg_kernel notes what the lists are like;
-// unlabeled in HBM, 33 degree counts (36 words) and d_hub_slot.
+// unlabeled in HBM, 33 counts (36 words: of degrees, of rows given out) and
+// d_hub_slot.
 static size_t maxnbrdeg_bytes(int64_t n) { return sizeof(int32_t) * (size_t)((n + 1) & ~1ll) + 16; }
 static bool takes_hub_rows(const pm_graph* g) { return !g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0; }
 static size_t aux_bytes(const pm_graph* g) {
@@ -3835,6 +3836,21 @@ static size_t aux_bytes(const pm_graph* g) {
 static unsigned long long* asym_word(const pm_graph* g) {
   return reinterpret_cast<unsigned long long*>(g->d_maxnbrdeg + ((g->n + 1) & ~1ll));
 }
+
+// Bit rows for the vertices with the longest lists: the lowest power of two of a
+// degree from 64 on (shorter lists are read as fast as a row) from which all
+// rows fit as many bytes as the adjacency array, or 64 MB if that is more, and
+// 256 MB at most -- half of them stay in L2.  h[k]: vertices of [2^k, 2^(k+1))
+// neighbours.
+static void choose_hub_rows(pm_graph* g, const unsigned int* h) {
+  const int64_t words = (g->n + 31) / 32;
+  const size_t budget = std::min<size_t>(256ull << 20, std::max<size_t>(64ull << 20, 4 * (size_t)g->nadj));
+  g->hub_rows = 0;
+  g->hub_log = 31;
+  for (; g->hub_log > 6 && (g->hub_rows + h[g->hub_log - 1]) * words * 4 <= budget; g->hub_log--)
+    g->hub_rows += h[g->hub_log - 1];
+}
+static size_t hub_bytes(const pm_graph* g) { return g->hub_rows * (size_t)((g->n + 31) / 32) * 4; }
 
 namespace pm {
 // Fills g->d_maxnbrdeg from an adjacency array the device can read (HBM or
@@ -3862,41 +3878,35 @@ static pm_status graph_finish(pm_graph* g) {
     CK(cudaMemset(asym_word(g), 0, 16 + (rows_wanted ? 33 * sizeof(unsigned int) : 0)));
     maxnbrdeg_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, g->d_maxnbrdeg, asym_word(g));
     CK(cudaGetLastError());
-    if (!rows_wanted) CK(cudaDeviceSynchronize());  // (else the degree counts' copy waits)
+    if (!rows_wanted) CK(cudaDeviceSynchronize());  // (else after the bit rows)
   }
   if (rows_wanted) {
-    // Bit rows for the vertices with the longest lists: the lowest power of
-    // two of a degree from 64 on (shorter lists are read as fast as a row)
-    // from which all rows fit as many bytes as the adjacency array, or 64 MB
-    // if that is more, and 256 MB at most -- half of them stay in L2.
-    unsigned int h[33];
-    degree_bins_kernel<<<256, 256>>>(g->d_rowptr, g->n, bins);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpy(h, bins, sizeof(h), cudaMemcpyDeviceToHost);
     const int64_t words = (g->n + 31) / 32;
-    const size_t budget = std::min<size_t>(256ull << 20, std::max<size_t>(64ull << 20, 4 * (size_t)g->nadj));
-    size_t rows = 0;
-    int k = 31;
-    for (; e == cudaSuccess && k > 6 && (rows + h[k - 1]) * words * 4 <= budget; k--) rows += h[k - 1];
-    if (e == cudaSuccess && rows) {
-      g->d_hub_slot = reinterpret_cast<int32_t*>(bins + 36);
-      e = cudaMalloc(&g->d_hub_bits, rows * words * 4);
+    cudaError_t e = cudaSuccess;
+    if (g->hub_log < 0) {  // device arrays: how many rows is not known yet
+      unsigned int h[33];
+      degree_bins_kernel<<<256, 256>>>(g->d_rowptr, g->n, bins);
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaMemcpy(h, bins, sizeof(h), cudaMemcpyDeviceToHost);
+      if (e == cudaSuccess) choose_hub_rows(g, h);
+      if (e == cudaSuccess && g->hub_rows) e = cudaMalloc(&g->d_hub_bits, hub_bytes(g));
       if (e == cudaErrorMemoryAllocation) {  // no room: the graph does without
         (void)cudaGetLastError();
-        g->d_hub_slot = nullptr;
         g->d_hub_bits = nullptr;
-        rows = 0;
         e = cudaSuccess;
       }
-      if (e == cudaSuccess && rows) e = cudaMemset(g->d_hub_bits, 0, rows * words * 4);
-      if (e == cudaSuccess && rows) {
-        hub_rows_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, 1 << k, words, bins + 32, g->d_hub_slot,
-                                       g->d_hub_bits);
+    }
+    if (e == cudaSuccess && g->d_hub_bits) {
+      g->d_hub_slot = reinterpret_cast<int32_t*>(bins + 36);
+      e = cudaMemset(g->d_hub_bits, 0, hub_bytes(g));
+      if (e == cudaSuccess) {
+        hub_rows_kernel<<<list_blocks(g->n), 512>>>(g->d_rowptr, g->d_colidx, g->n, 1 << g->hub_log, words, bins + 32,
+                                                    g->d_hub_slot, g->d_hub_bits);
         e = cudaGetLastError();
       }
-      if (e == cudaSuccess) e = cudaDeviceSynchronize();
-      if (rows) g->device_bytes += sizeof(int32_t) * g->n + rows * words * 4;
+      g->device_bytes += sizeof(int32_t) * g->n + hub_bytes(g);
     }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     CK(e);
   }
   if (g->labeled && g->residency == PM_RESIDENT_HBM && g->n > 0) {
@@ -3985,7 +3995,18 @@ static pm_status place_rows(pm_graph* g, int64_t n, int64_t nadj, const uint64_t
   g->labeled = o.labeled ? 1 : 0;
   g->residency = o.residency;
   int32_t maxd = 0;
-  for (int64_t v = 0; v < n; v++) maxd = std::max<int32_t>(maxd, (int32_t)(rowptr[v + 1] - rowptr[v]));
+  if (takes_hub_rows(g)) {
+    unsigned int h[4][32] = {};  // (four of them: neighbours in the array often share a bin)
+    for (int64_t v = 0; v < n; v++) {
+      const uint32_t d = (uint32_t)(rowptr[v + 1] - rowptr[v]);
+      maxd = std::max<int32_t>(maxd, (int32_t)d);
+      h[v & 3][31 - __builtin_clz(d | 1u)]++;
+    }
+    for (int k = 0; k < 32; k++) h[0][k] += h[1][k] + h[2][k] + h[3][k];
+    choose_hub_rows(g, h[0]);
+  } else {
+    for (int64_t v = 0; v < n; v++) maxd = std::max<int32_t>(maxd, (int32_t)(rowptr[v + 1] - rowptr[v]));
+  }
   g->maxdeg = maxd;
   CK(cudaMalloc(&g->d_rowptr, sizeof(uint64_t) * (n + 1) + aux_bytes(g)));
   g->d_maxnbrdeg = reinterpret_cast<int32_t*>(g->d_rowptr + n + 1);
@@ -4031,7 +4052,16 @@ extern "C" pm_status pm_graph_from_host(int64_t n, int64_t nadj, const uint64_t*
       if (st != PM_OK) return st;
     }
   } else {
-    CK(cudaMalloc(&g->d_colidx, sizeof(int32_t) * std::max<int64_t>(nadj, 1)));
+    // the adjacency array and, after it, the bit rows (none when memory is short)
+    const size_t adj_bytes = (sizeof(int32_t) * (size_t)std::max<int64_t>(nadj, 1) + 255) & ~(size_t)255;
+    cudaError_t e = cudaMalloc(&g->d_colidx, adj_bytes + hub_bytes(g.get()));
+    if (e == cudaErrorMemoryAllocation && g->hub_rows) {
+      (void)cudaGetLastError();
+      g->hub_rows = 0;
+      e = cudaMalloc(&g->d_colidx, adj_bytes);
+    }
+    CK(e);
+    if (g->hub_rows) g->d_hub_bits = reinterpret_cast<uint32_t*>(g->d_colidx) + adj_bytes / 4;
     if (nadj) CK(cudaMemcpy(g->d_colidx, colidx, sizeof(int32_t) * nadj, cudaMemcpyHostToDevice));
     g->device_bytes += sizeof(int32_t) * nadj;
     st = graph_finish(g.get());
@@ -4144,10 +4174,12 @@ extern "C" void pm_graph_close(pm_graph* g) {
     free_dev(g->d_colidx);
     free_dev(g->d_labels);
   }
-  if (!g->owns) free_dev(g->d_maxnbrdeg);  // else a part of the rows' allocation
+  if (!g->owns) {  // else parts of the rows' and the adjacency array's allocations
+    free_dev(g->d_maxnbrdeg);
+    free_dev(g->d_hub_bits);
+  }
   free_dev(g->d_colidx_lab);
   free_dev(g->d_lab_off);
-  free_dev(g->d_hub_bits);
   paged_release(g);
   delete g;
 }

@@ -182,7 +182,9 @@ struct pm_graph {
   // unlabeled graphs in HBM: a bit row over all vertices for each vertex with
   // a long list, and which row is whose
   int32_t* d_hub_slot = nullptr;   // [n], -1: none
-  uint32_t* d_hub_bits = nullptr;  // [rows][(n + 31) / 32]
+  uint32_t* d_hub_bits = nullptr;  // [hub_rows][(n + 31) / 32]
+  size_t hub_rows = 0;
+  int hub_log = -1;                // rows for lists of 2^hub_log elements on; -1: not chosen yet
   uint64_t device_bytes = 0;
   // paged residency (pm_paging.cu)
   int32_t* h_colidx = nullptr;     // pinned, mapped copy of the adjacency array
