@@ -30,8 +30,8 @@ def host_graph(e, n, labels=None):
 class Search:
     """A plan's search, one set operation after the other: N(v_L) (fresh), N(v_L) met with the parent slot, or the
     parent slot (copy), the first operand cut at the plan's bound, less the path vertices (fresh) or v_L (copy) when
-    unlabeled, by label else, at most T long.  Of the last level's fresh set only the size counts, less one for each of
-    v_0 .. v_{n-3} in it."""
+    unlabeled, by label else, at most T long.  Of the last level's fresh set or copy only the size counts, less one for
+    each of v_0 .. v_{n-3} (fresh) or for v_{n-2} (copy) in it, however often it is there."""
 
     def __init__(self, hg, p, truncate):
         self.d, self.T = p.describe(), truncate
@@ -64,9 +64,12 @@ class Search:
             size = len(out) - sum(v in out for v in path[:L])
         elif fresh:
             out = [x for x in (A[:T] if T else A) if x not in path]
+        elif last:
+            out, size = A, len(A) - (path[L] in A)
+            size = min(size, T) if T else size
         else:
             out = [x for x in A if x != path[L]]
-        if not (fresh and last and not labeled):
+        if labeled or meet or not last:
             out = out[:T] if T else out
             size = len(out)
         self.ops += 1
@@ -152,3 +155,21 @@ def test_small_arenas_and_elements_that_come_twice(ctx, shape, labeled, words):
     e += [x for a, b in e if a < b and (a + b) % 3 for x in ((a, b), (b, a))]
     labels = (np.arange(n) * 7 % 5 % 3).astype(np.uint32) if labeled else None
     check(ctx, host_graph(e, n, labels), shape, labeled, 0, lane_subtree_max=-1, own_arena_words=words)
+
+
+@pytest.mark.parametrize("truncate", [0, 5])
+@pytest.mark.parametrize("shape", ["P4", "house", "house_tail", "C4_tail", "C5"])
+def test_elements_that_come_twice(ctx, shape, truncate):
+    e, n = entries(90, 4, 1)
+    e += [x for a, b in e if a < b and (a * 7 + b) % 5 == 0 for x in ((a, b), (b, a))]
+    check(ctx, host_graph(e, n), shape, False, truncate)
+
+
+@pytest.mark.parametrize("truncate", [0, 5])
+@pytest.mark.parametrize("shape", ["P4", "house", "house_tail", "C4_tail", "C5", "K4", "K5"])
+@pytest.mark.parametrize("labeled", [False, True])
+def test_entries_without_their_reverse(ctx, shape, labeled, truncate):
+    e, n = entries(90, 4, 1)
+    e = [x for x in e if (x[0] * 31 + x[1] * 17) % 9]
+    labels = (np.arange(n) * 7 % 5 % 3).astype(np.uint32) if labeled else None
+    check(ctx, host_graph(e, n, labels), shape, labeled, truncate)
