@@ -386,7 +386,15 @@ typedef struct {
   float roots_ms;           /* device time of the root filter               */
   int32_t grid_blocks;
   int32_t block_threads;
-  uint64_t arena_bytes;
+  uint64_t arena_bytes;     /* the launch's candidate-set arenas (own and
+                               borrowed).  Besides them a context, and each
+                               prepared query, may hold value tables (plans
+                               with a cycle of five or more: at most 16 B x
+                               16,385 a warp, 931 MB on 148 SMs), tables for
+                               labeled tails (at most 1 GiB) and, the context,
+                               feature rows (64 B a vertex, at most 1 GiB);
+                               none of them is needed: without room for them
+                               the search does without.  Freed with it       */
   uint32_t device_status;   /* 0 ok; else PM_DEV_* flags                     */
   uint32_t pad_;
   uint64_t warp_ns;         /* sum over warps of their time in the launch    */

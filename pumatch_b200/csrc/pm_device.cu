@@ -12,7 +12,7 @@
 //     reference's disabled stealing, src/gpu_match.cu:21-148, 818-853);
 //   * each level's candidate sets ("slots") are read in place where they are
 //     an adjacency list or their parent, else computed by a warp-cooperative
-//     sorted-set operation -- 128 elements per step, __ballot_sync/__popc
+//     sorted-set operation -- 64 elements per step, __ballot_sync/__popc
 //     compaction -- and stored in a per-warp arena in HBM sized to the plan's
 //     worst case, so nothing is truncated (the reference caps every set at
 //     GRAPH_DEGREE=4096; that cap is kept only as an explicit emulation
@@ -234,7 +234,7 @@ struct alignas(16) WarpState {
     int32_t pins[PM_MAX_LIST_PAGES];
     int32_t queue[64];
   };
-  alignas(16) int32_t sb[PM_SB_MAX + 4];  // the common operand (bitmap, hash table or sorted copy); +4 for a
+  alignas(16) int32_t sb[PM_SB_MAX + 4];  // the common operand (bitmap, filter or sorted copy); +4 for a
                                          // bulk copy that starts up to 3 words before it
   unsigned long long mbar;               // completion barrier of the warp's bulk copies
   uint32_t mphase;                       // its current phase
@@ -594,11 +594,11 @@ __device__ __forceinline__ int group_lower_bound(const int32_t* A, int len, int 
   return lo;
 }
 
-// Four searches at once: whether each x[q] is in sorted B[0, len).  The steps
-// do not depend on what is found, so the four loads of a step are in flight
+// N searches at once: whether each x[q] is in sorted B[0, len).  The steps
+// do not depend on what is found, so the loads of a step are in flight
 // together.
 template <bool CG, int N>
-__device__ __forceinline__ void bsearch4(const int32_t* B, int len, const int (&x)[N], bool (&in)[N], bool cg) {
+__device__ __forceinline__ void bsearch_n(const int32_t* B, int len, const int (&x)[N], bool (&in)[N], bool cg) {
   int p[N] = {};
   if (len <= 0) {
 #pragma unroll
@@ -697,7 +697,7 @@ __device__ __forceinline__ unsigned long long list_id(const int32_t* p) {
 // adjacency list itself, cut at its bound, with the path vertices in it
 // skipped by whoever walks it (DPlan.hole_ok: only where nothing else reads
 // the slot); a copy that removes nothing is its parent.  Intersections test
-// four elements per lane at a time against a structure in shared memory that
+// two elements per lane at a time against a structure in shared memory that
 // the candidates of a level share (leaf_build), or look the shorter operand
 // up in the longer when that is 16 times as long.
 // Measured (B200), cycles of all warps in levels above the last, the 20-pattern
@@ -896,12 +896,12 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
       });
     } else if ((long long)lenB * 16 < lenA && simple) {
       cnt = compact<PAGED>(B, lenB, cgB, out, T, [&](const int (&v)[2], bool (&in)[2]) {
-        bsearch4<PAGED>(A, lenA, v, in, cgA);
+        bsearch_n<PAGED>(A, lenA, v, in, cgA);
         labelled(v, in);
       });
     } else if ((long long)lenA * 16 < lenB && !(idB && idB == S.sb_id && lenB == S.sb_len)) {
       cnt = compact<PAGED>(A, lenA, cgA, out, T, [&](const int (&v)[2], bool (&in)[2]) {
-        bsearch4<PAGED>(B, lenB, v, in, cgB);
+        bsearch_n<PAGED>(B, lenB, v, in, cgB);
         labelled(v, in);
       });
     } else {
@@ -916,7 +916,7 @@ __device__ int run_slot(const MatchArgs& a, const DPlan& P, WarpState& S, int L,
 #pragma unroll
             for (int q = 0; q < 2; q++) in[q] = in[q] && leaf_maybe<MEMB_FILTER>(m, v[q]);
           }
-          if (__any_sync(FULL, in[0] || in[1])) bsearch4<PAGED>(B, lenB, v, in, cgB);
+          if (__any_sync(FULL, in[0] || in[1])) bsearch_n<PAGED>(B, lenB, v, in, cgB);
         }
         labelled(v, in);
       });
@@ -2430,7 +2430,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
         } else {
 #pragma unroll
           for (int k = 0; k < U; k++) in[k] = in[k] && leaf_maybe<MEMB_FILTER>(set, x[k]);
-          if (__any_sync(FULL, any_of(in))) bsearch4<false>(set.g, set.lenB, x, in, false);
+          if (__any_sync(FULL, any_of(in))) bsearch_n<false>(set.g, set.lenB, x, in, false);
         }
       } else if (!LABELED) {
         for (int i = 0; i <= L; i++) {
@@ -2471,7 +2471,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
             hit[k] = in[k] && x[k] != vo;
           }
         }
-        if (!LABELED) bsearch4<false>(H0, len0, x, hit, false);
+        if (!LABELED) bsearch_n<false>(H0, len0, x, hit, false);
 #pragma unroll
         for (int k = 0; k < U; k++) {
           if (!in[k]) continue;
@@ -2508,7 +2508,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
               for (int k = 0; k < U; k++) hit[k] = in[k] && ((__ldg(row + (x[k] >> 5)) >> (x[k] & 31)) & 1u);
             } else {
               const uint64_t pb = a.rowptr[p];
-              bsearch4<false>(a.colidx + pb, (int)(a.rowptr[p + 1] - pb), x, hit, false);
+              bsearch_n<false>(a.colidx + pb, (int)(a.rowptr[p + 1] - pb), x, hit, false);
             }
 #pragma unroll
             for (int k = 0; k < U; k++) f[k] -= hit[k] ? 1 : 0;

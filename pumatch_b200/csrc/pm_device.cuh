@@ -48,8 +48,8 @@ struct DPlan {
   int8_t pair_h0;                 // the slot its copy or meeting reads
   uint8_t copy_next;              // labeled: bit L: level L+1 is all copies (one candidate searched for all)
   int8_t chain_from;              // labeled: first of the fresh levels the plan ends in, 0: none (chain_kernel)
-  uint8_t hole_ok[16];
-  const ulonglong4* chain;        // its table, by vertex (null: not used)            // 1: the slot may be read in place, path vertices skipped by its walker
+  uint8_t hole_ok[16];            // 1: the slot may be read in place, path vertices skipped by its walker
+  const ulonglong4* chain;        // the chain's first table, by vertex (null: not used)
   const int2* roots;              // (v0, v1) root edges, reference order (the whole list)
   int64_t nroots;                 // positions this launch processes
   int64_t rbase;                  // first position: root_begin (0 = all)
