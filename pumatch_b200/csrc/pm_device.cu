@@ -2162,9 +2162,10 @@ __device__ __forceinline__ bool pair_ready(const MatchArgs& a, const DPlan& P, c
 // warps and at the deadline between passes; with no such bound one over 32
 // hubs' lists took 19 ms (a 5-path on an R-MAT graph of 262,144 vertices), or
 // 136 ms where each element's list is walked in turn (the 5-cycle with 4
-// labels); with it 3 and 25 ms.  Half as many cost the 6-cycle shard 8% (38.1
-// -> 41 ms), a look from inside the walks the 20-pattern batch 5%; this costs
-// the batch 3.5% (19.0 -> 19.7 ms).
+// labels); with it 3 and 15 ms.  Labeled, those take half as many (4,096: 27
+// ms); unlabeled, half as many cost the 6-cycle shard 8% (38.1 -> 41 ms).  A
+// look from inside the walks instead cost the 20-pattern batch 5%; this costs
+// it 3% (19.2 -> 19.7 ms).
 constexpr int kPairRow = 4096;
 
 template <int N>
@@ -2356,6 +2357,7 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
     mine = false;
   }
   // walk
+  constexpr int row_max = LABELED && KIND == PAIR_MEET ? kPairRow / 2 : kPairRow;
   int queued = 0;
   int total = len, next = e, next_off = 0, pair_take = 32;
   if (!PAGED) {
@@ -2365,8 +2367,8 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       if (lane >= d) incl += t;
     }
     total = __shfl_sync(FULL, incl, 31);
-    if (total > kPairRow) {
-      const int whole = __popc(__ballot_sync(FULL, incl <= kPairRow));  // candidates whose lists fit
+    if (total > row_max) {
+      const int whole = __popc(__ballot_sync(FULL, incl <= row_max));  // candidates whose lists fit
       const int take = max(1, whole);
       if (lane >= take) {
         mine = false;
@@ -2375,10 +2377,10 @@ __device__ __noinline__ unsigned long long pair_pass(const MatchArgs& a, const D
       }
       if (lane >= whole) len = incl = 0;
       next = b + whole;
-      next_off = whole ? 0 : off + kPairRow;
+      next_off = whole ? 0 : off + row_max;
       pair_take = take;
-      if (whole == 0 && lane == 0) len = kPairRow;
-      total = __shfl_sync(FULL, whole ? incl : kPairRow, take - 1);
+      if (whole == 0 && lane == 0) len = row_max;
+      total = __shfl_sync(FULL, whole ? incl : row_max, take - 1);
       incl = lane < whole ? incl : total;
     }
     S.prb[lane] = rb;
